@@ -1,0 +1,226 @@
+// Particle-to-grid scatters by warps: runs of particles that share a stencil base are summed over
+// the warp and the sums go straight to the L2 atomics.
+//
+// A warp splits its 32 particles into runs of equal stencil base. Each particle's own thread stores
+// its 27 node weights (w_x w_y) w_z, as the reference rounds them, and its values in the warp's
+// record in shared memory; the run is then summed over its particles and every node receives one
+// atomic per run (one 16-byte vector atomic for momentum and mass). Nothing is shared between
+// warps, so a block has no barrier.
+//
+// What bounds it, and why there is no block tile: a shared-memory tile over the block's node box
+// (summing the block's runs before one global atomic per node) needs three block barriers, the
+// zeroing and flushing of the tile, and shared float atomics, which are compare-and-swap loops with
+// bank conflicts; it held the LSU data pipe at 73% (momentum) and 71% (transport) of its peak. A run
+// of ~18 particles already divides the atomics by 18, and L2 takes the rest without waiting. 1M
+// particles, 128^3 grid, 40 particles a cell, fused P2G kernel: 102 us with the tile, 87 us with the
+// same kernel writing straight to L2; transport scatter 68.5 against 62.1 us, 55 with the float64
+// tensor cores; in tet order P2G of 41k particles 37 against 16 us.
+#pragma once
+
+#include <climits>
+
+#include "bk_device.cuh"
+
+namespace bk {
+
+constexpr unsigned kWarp = 0xffffffffu;
+
+// Stencil node j in 0..26 -> offsets (j / 9, (j / 3) % 3, j % 3), the reference's loop order.
+BK_DEV void node_offset(int j, int& ox, int& oy, int& oz) {
+    ox = j / 9;
+    oy = (j / 3) % 3;
+    oz = j - 9 * ox - 3 * oy;
+}
+
+// The columns of the warp's record (one per lane) that start a run: bit k is set when lane k holds a
+// valid particle whose stencil base differs from lane k - 1's.
+BK_DEV unsigned run_starts(bool valid, const int* b) {
+    const int lane = threadIdx.x & 31;
+    const int p0 = __shfl_up_sync(kWarp, b[0], 1), p1 = __shfl_up_sync(kWarp, b[1], 1),
+              p2 = __shfl_up_sync(kWarp, b[2], 1);
+    const bool before = __shfl_up_sync(kWarp, (int)valid, 1) != 0;
+    return __ballot_sync(kWarp, valid && (lane == 0 || !before || p0 != b[0] || p1 != b[1] || p2 != b[2]));
+}
+
+// Column one past the run before the next start. (A run may include columns of invalid particles,
+// whose stored weights are zero.)
+BK_DEV int run_end(unsigned later_starts) { return later_starts ? __ffs(later_starts) - 1 : 32; }
+
+// The 27 weights of this thread's particle into its lane's column of the record's node-major rows.
+template <int kPitch>
+BK_DEV void put_weights(float (&w)[27][kPitch], bool valid, const Stencil& st) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int ox = 0; ox < 3; ++ox)
+#pragma unroll
+        for (int oy = 0; oy < 3; ++oy) {
+            const float wxy = valid ? st.w[0][ox] * st.w[1][oy] : 0.f;
+#pragma unroll
+            for (int oz = 0; oz < 3; ++oz) w[9 * ox + 3 * oy + oz][lane] = valid ? wxy * st.w[2][oz] : 0.f;
+        }
+}
+
+// Widens the node box `bounds` ([0..2] lowest, [3..5] highest node) over the block's valid stencils.
+// Every thread of the block calls it, early, while the warps are still together: one test per warp
+// in place of two barriers cost 4 us of 39 on a 41k-particle body, whose warps all start on an empty
+// box and queue on its six addresses.
+BK_DEV void widen_box(int* bounds, bool valid, const int* b) {
+    __shared__ int s_box[6];
+    if (threadIdx.x < 6) s_box[threadIdx.x] = threadIdx.x < 3 ? INT_MAX : INT_MIN;
+    __syncthreads();
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const int lo = __reduce_min_sync(kWarp, valid ? b[a] : INT_MAX);
+        const int hi = __reduce_max_sync(kWarp, valid ? b[a] + 2 : INT_MIN);
+        if ((threadIdx.x & 31) == 0 && lo != INT_MAX) {
+            atomicMin(&s_box[a], lo);
+            atomicMax(&s_box[3 + a], hi);
+        }
+    }
+    __syncthreads();
+    // The box only widens, so a value read through L2 that is older than the current one is never
+    // narrower: a block whose box lies inside it skips the atomics.
+    if (threadIdx.x < 6) {
+        const int t = threadIdx.x, now = __ldcg(bounds + t);
+        if (t < 3 && s_box[t] < now) atomicMin(bounds + t, s_box[t]);
+        if (t >= 3 && s_box[t] > now) atomicMax(bounds + t, s_box[t]);
+    }
+}
+
+// ------------------------------------------------------------- momentum form
+// Node j of particle k receives w_jk (q + A o_j) in x, y, z and w_jk m in w, o_j the node's offsets
+// in cells: the run's sums of w m, w q and w A (paired accumulators, one packed multiply-add per
+// pair), with o_j applied once per run. Lane j < 27 owns node j; a lane reads its weight row at the
+// particle's column (conflict-free) and the values as 128-bit broadcasts.
+struct MomentumRecord {
+    float4 val[32][3];  // {m q0 q1 q2} {A0 A1 A2 A3} {A4 A5 A6 A7}
+    float a8[32];
+    float w[27][33];
+};
+
+BK_DEV void scatter_momentum(MomentumRecord& rec, bool valid, const Stencil& st, float m, const float* q,
+                             const float* A, float4* __restrict__ nodes, int R) {
+    const int lane = threadIdx.x & 31;
+    put_weights(rec.w, valid, st);
+    rec.val[lane][0] = make_float4(m, q[0], q[1], q[2]);
+    rec.val[lane][1] = make_float4(A[0], A[1], A[2], A[3]);
+    rec.val[lane][2] = make_float4(A[4], A[5], A[6], A[7]);
+    rec.a8[lane] = A[8];
+    __syncwarp();
+    int ox, oy, oz;
+    node_offset(lane < 27 ? lane : 0, ox, oy, oz);
+    const float fo[3] = {(float)ox, (float)oy, (float)oz};
+    const float* wj = rec.w[lane < 27 ? lane : 0];
+    unsigned starts = run_starts(valid, st.b);
+    while (starts) {
+        const int s = __ffs(starts) - 1;
+        starts &= starts - 1;
+        const int e = run_end(starts);
+        const int base[3] = {__shfl_sync(kWarp, st.b[0], s), __shfl_sync(kWarp, st.b[1], s), __shfl_sync(kWarp, st.b[2], s)};
+        if (lane < 27) {
+            float2 mq0 = {0.f, 0.f}, q12 = {0.f, 0.f}, A01 = {0.f, 0.f}, A23 = {0.f, 0.f};
+            float2 A45 = {0.f, 0.f}, A67 = {0.f, 0.f};
+            float A8 = 0.f;
+#pragma unroll 2
+            for (int k = s; k < e; ++k) {
+                const float w = wj[k];
+                const float2 ww = make_float2(w, w);
+                const float4 v0 = rec.val[k][0], v1 = rec.val[k][1], v2 = rec.val[k][2];
+                mq0 = ffma2(ww, make_float2(v0.x, v0.y), mq0);
+                q12 = ffma2(ww, make_float2(v0.z, v0.w), q12);
+                A01 = ffma2(ww, make_float2(v1.x, v1.y), A01);
+                A23 = ffma2(ww, make_float2(v1.z, v1.w), A23);
+                A45 = ffma2(ww, make_float2(v2.x, v2.y), A45);
+                A67 = ffma2(ww, make_float2(v2.z, v2.w), A67);
+                A8 = fmaf(w, rec.a8[k], A8);
+            }
+            const float aq[3] = {mq0.y, q12.x, q12.y};
+            const float aA[9] = {A01.x, A01.y, A23.x, A23.y, A45.x, A45.y, A67.x, A67.y, A8};
+            float ap[3];
+#pragma unroll
+            for (int r = 0; r < 3; ++r)
+                ap[r] = aq[r] + (aA[3 * r] * fo[0] + aA[3 * r + 1] * fo[1] + aA[3 * r + 2] * fo[2]);
+            atomicAdd(nodes + node_index(base[0] + ox, base[1] + oy, base[2] + oz, R), make_float4(ap[0], ap[1], ap[2], mq0.x));
+        }
+    }
+}
+
+// ------------------------------------------------------------- float64 form
+// kF float64 values per particle (the transport fields, the surface rates), node j receiving
+// w_jk value_k: the contraction (27 nodes x particles) (particles x kF) on the float64 tensor cores,
+// mma.m8n8k4 with four 8-node row tiles and the values in the columns, four particles a step. The
+// products and sums are float64, as the reference's float64 atomics: float32 partial sums moved the
+// node temperature E / C by ~3e-5 K, harmless to the trajectory but enough to make finite differences
+// of the loss in the initial temperatures disagree with the adjoint by several percent.
+// A scalar loop (lane j owns node j) reads five shared words and issues four float64 multiply-adds
+// per particle; the mma form reads five words and issues four mma per FOUR particles. The row pitch
+// of 36 puts the 32 words of a fragment (8 rows x 4 particles) in 32 banks.
+template <int kF>
+struct ScalarRecord {
+    double val[kF][36];
+    float w[27][36];
+};
+
+BK_DEV void dmma(double& d0, double& d1, double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+        : "+d"(d0), "+d"(d1)
+        : "d"(a), "d"(b));
+}
+
+// Adds values val[0..kF) of the warp's particles to the node fields f[0..kF) (R^3 float64 each).
+template <int kF>
+BK_DEV void scatter_scalars(ScalarRecord<kF>& rec, bool valid, const Stencil& st, const double* val,
+                            double* const (&f)[kF], int R) {
+    static_assert(kF >= 1 && kF <= 4, "the values share one 8-column tile");
+    const int lane = threadIdx.x & 31;
+    const int row = lane >> 2, quad = lane & 3;  // fragment coordinates
+    put_weights(rec.w, valid, st);
+#pragma unroll
+    for (int k = 0; k < kF; ++k) rec.val[k][lane] = valid ? val[k] : 0.0;
+    __syncwarp();
+    // Accumulator fragment: row 8 t + row, columns 2 quad and 2 quad + 1 (fields; quads 0 and 1).
+    int offset[4];
+    bool node[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        const int j = 8 * t + row;
+        int ox, oy, oz;
+        node_offset(j < 27 ? j : 0, ox, oy, oz);
+        offset[t] = (ox * R + oy) * R + oz;
+        node[t] = j < 27;
+    }
+    // (selects, not f[2 * quad]: a run-time index would copy the pointers to local memory)
+    double* const f0 = kF > 2 && quad == 1 ? f[2] : f[0];
+    double* const f1 = kF > 3 && quad == 1 ? f[3] : f[kF > 1 ? 1 : 0];
+    unsigned starts = run_starts(valid, st.b);
+    while (starts) {
+        const int s = __ffs(starts) - 1;
+        starts &= starts - 1;
+        const int e = run_end(starts);
+        const int base[3] = {__shfl_sync(kWarp, st.b[0], s), __shfl_sync(kWarp, st.b[1], s), __shfl_sync(kWarp, st.b[2], s)};
+        double d[4][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+        for (int k0 = s; k0 < e; k0 += 4) {
+            // Fragments: weight of node 8 t + row and value `row` of particle k0 + quad; particles past
+            // the run are zero on both sides (their weights may belong to another run, or be NaN).
+            const int k = k0 + quad;
+            const bool in = k < e;
+            double b = 0.0;
+            if (in && row < kF) b = rec.val[row][k];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                float w = 0.f;
+                if (in && node[t]) w = rec.w[8 * t + row][k];
+                dmma(d[t][0], d[t][1], (double)w, b);
+            }
+        }
+        const int64_t corner = node_index(base[0], base[1], base[2], R);
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+            if (node[t]) {
+                if (2 * quad < kF) atomicAdd(f0 + corner + offset[t], d[t][0]);
+                if (2 * quad + 1 < kF) atomicAdd(f1 + corner + offset[t], d[t][1]);
+            }
+    }
+}
+
+}  // namespace bk

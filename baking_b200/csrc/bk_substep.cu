@@ -14,12 +14,9 @@
 //   grid_update        momentum -> velocity with walls over the active box; zeroes the scatter fields
 //   g2p_return         G2P (v, C, x, F) fused with the Ding return map (float64 SVD in registers)
 //
-// Scatter scheme ("warp-cooperative stencil runs"): a warp loads 32 consecutive
-// particles; consecutive lanes whose particles share a stencil base form a run;
-// for each run, lane j < 27 owns stencil node j, sums the run's contributions in
-// registers (particle data broadcast from shared memory) and issues one atomic
-// per field. With particles ordered by cell this turns 27 atomics per particle
-// into 27 per run of ~tens of particles, and any order stays correct.
+// Scatter scheme (bk_scatter.cuh): a warp groups its 32 particles into runs of equal stencil base,
+// sums each run and issues one atomic per run, node and field. With particles ordered by cell this
+// turns 27 atomics per particle into 27 per run of ~tens of particles, and any order stays correct.
 //
 // The active node box (min/max stencil node of the current particles) bounds
 // every dense grid pass; the grid passes leave the scatter fields zeroed behind
@@ -36,6 +33,7 @@
 #include "bk_common.h"
 #include "bk_device.cuh"
 #include "bk_mlp.cuh"
+#include "bk_scatter.cuh"
 #include "bk_profile.h"
 
 using namespace bk;
@@ -43,7 +41,6 @@ using namespace bk;
 namespace {
 
 constexpr int kThreads = 256;
-constexpr unsigned kFull = 0xffffffffu;
 
 inline cudaStream_t S(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
@@ -151,6 +148,12 @@ __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// The 128-byte lines of plane arrays that a warp's 32 particles read, requested into L2 by one
+// instruction per 32 lines (lane c takes plane c) before the values are needed: the loads of a
+// particle kernel fall into phases (position, node gather, state) and each phase otherwise waits for
+// DRAM again.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // The status of a launch_chained call, as check_launch reports a launch's.
 int check_chained(cudaError_t e, const char* name) {
     if (e == cudaSuccess) return check_launch(name);
@@ -182,80 +185,6 @@ cudaError_t launch_chained(void (*kernel)(KArgs...), unsigned grid, unsigned blo
 // registers).
 template <class T, bool kRef>
 using Arg = typename std::conditional<kRef, const T&, const T>::type;
-
-// Stencil node j in 0..26 -> offsets (j / 9, (j / 3) % 3, j % 3), the reference's loop order.
-__device__ __forceinline__ void node_offset(int j, int& ox, int& oy, int& oz) {
-    ox = j / 9;
-    oy = (j / 3) % 3;
-    oz = j - 9 * ox - 3 * oy;
-}
-
-
-__device__ __forceinline__ long long pack_base(const int* b) {
-    return ((long long)b[0] << 42) | ((long long)b[1] << 21) | (long long)b[2];
-}
-
-// Nodes a block may stage in shared memory before flushing them to the grid.
-constexpr int kTileNodes = 512;
-
-// Node box touched by one block's particles.
-struct BlockBox {
-    int lo[3], ext[3], count;  // count = 0: no valid particle in the block
-    bool tiled;                // the box fits a shared-memory tile of kTileNodes
-};
-
-// Block-level min/max of valid stencil nodes; also widens the node box `bounds` ([0..2] lo, [3..5]
-// hi) unless it is null. The box is tiled when it holds at most `tile_nodes` nodes. Every thread of the block must
-// call this (it synchronises the block).
-__device__ BlockBox block_box(int* bounds, bool valid, const int* b, int tile_nodes = kTileNodes) {
-    __shared__ int s_box[6];
-    if (threadIdx.x < 6) s_box[threadIdx.x] = threadIdx.x < 3 ? INT_MAX : INT_MIN;
-    __syncthreads();
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        int lo = __reduce_min_sync(kFull, valid ? b[a] : INT_MAX);
-        int hi = __reduce_max_sync(kFull, valid ? b[a] + 2 : INT_MIN);
-        if ((threadIdx.x & 31) == 0 && lo != INT_MAX) {
-            atomicMin(&s_box[a], lo);
-            atomicMax(&s_box[3 + a], hi);
-        }
-    }
-    __syncthreads();
-    BlockBox bb;
-    bb.count = 0;
-    bb.tiled = true;
-    if (s_box[0] != INT_MAX) {
-        long long count = 1;
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            bb.lo[a] = s_box[a];
-            bb.ext[a] = s_box[3 + a] - s_box[a] + 1;
-            count *= bb.ext[a];
-        }
-        bb.tiled = count <= tile_nodes;
-        bb.count = bb.tiled ? (int)count : 0;
-        if (bounds != nullptr && threadIdx.x < 3) {
-            // The shared box only widens (min of lo, max of hi), so a value read through L2 that is
-            // older than the current one is never narrower: a block whose box lies inside it
-            // skips the atomics, and thousands of blocks stop contending for six addresses.
-            const int t = threadIdx.x;
-            if (s_box[t] < __ldcg(bounds + t)) atomicMin(bounds + t, s_box[t]);
-            if (s_box[3 + t] > __ldcg(bounds + 3 + t)) atomicMax(bounds + 3 + t, s_box[3 + t]);
-        }
-    }
-    return bb;
-}
-
-__device__ __forceinline__ int tile_index(const BlockBox& bb, int x, int y, int z) {
-    return ((x - bb.lo[0]) * bb.ext[1] + (y - bb.lo[1])) * bb.ext[2] + (z - bb.lo[2]);
-}
-
-__device__ __forceinline__ int64_t tile_node(const BlockBox& bb, int t, int R) {
-    int z = t % bb.ext[2];
-    int y = (t / bb.ext[2]) % bb.ext[1];
-    int x = t / (bb.ext[2] * bb.ext[1]);
-    return node_index(bb.lo[0] + x, bb.lo[1] + y, bb.lo[2] + z, R);
-}
 
 // ------------------------------------------------------------------ surface
 // geometry/mesh_tracking.py:13-38 restricted to the vertices of boundary faces. A vertex of a
@@ -305,8 +234,7 @@ __global__ void __launch_bounds__(kBlock == 32 ? 32 * kVertexWarps : kBlock) k_s
 //   loaf): one warp per owner; lane 0 sums the owner's faces in order, every lane forms the rates,
 //   lane j < 27 adds stencil node j's share (27 atomics in parallel);
 // * many owners (a fine tetrahedral mesh: about a third of a dough ball's particles own faces): one
-//   thread per owner, the node shares summed per stencil run and per block tile like the transport
-//   scatter, so the 81 float64 atomics per owner become a few per node and block.
+//   thread per owner, the node shares summed per stencil run like the transport scatter.
 // With accumulators set in `sf`, the owner's water-loss and heat-exchange accumulators also advance
 // by one substep (thermal_water.py:225-226), which bk_surface_accumulate does otherwise.
 constexpr int kOwnerThreads = 128;
@@ -377,8 +305,8 @@ __device__ __forceinline__ void surface_owners_warp_body(Arg<Params, kRef> P, Ar
     const int p = sf.owners[o];
     double exposed = 0.0, contact = 0.0;
     if (lane == 0) owner_areas(sf, o, exposed, contact);
-    exposed = __shfl_sync(kFull, exposed, 0);
-    contact = __shfl_sync(kFull, contact, 0);
+    exposed = __shfl_sync(kWarp, exposed, 0);
+    contact = __shfl_sync(kWarp, contact, 0);
     double rate[3];
     owner_rates(P, in, cst, p, exposed, contact, rate);
     if (lane == 0) owner_store(sf, o, p, rate);
@@ -398,138 +326,11 @@ __device__ __forceinline__ void surface_owners_warp_body(Arg<Params, kRef> P, Ar
     }
 }
 
-// ---------------------------------------------------------- transport P2G
-// physics/thermal_water.py:108-137 (volume, capacity, energy, water), warp-cooperative per stencil run.
-// The block routine scatters its threads' particles; each thread passes its stencil, whether it is
-// valid, and its four values (V0 det F, capacity, capacity T, W). Every thread of the block calls it.
-// The run sums are float64, as the reference's float64 atomics: float32 partial sums moved the
-// node temperature E/C by ~3e-5 K, harmless to the trajectory but enough to make finite
-// differences of the loss in the initial temperatures disagree with the adjoint by several percent.
-// The routine is shared with the surface terms (heat, loss and exchange of the face owners into
-// node fields 4..6): kF fields starting at node field kFirst, values of invalid threads ignored.
-// Stencil weights of the block's particles, in one of two forms:
-// * kNodeWeights: each particle's 27 weights (w_x w_y) w_z, formed once by its own thread as the
-//   reference rounds them, in node-major rows of kT + 1 floats; lane j of a run reads row j at the
-//   particle's column, one conflict-free load in place of three loads and two multiplies per node;
-// * otherwise the nine axis weights per particle (3 loads and 2 multiplies per node), a third of
-//   the space: the form of the scatter inside the G2P kernel, whose eight blocks per SM leave the
-//   rest of the SM's shared memory to L1 for its spilled registers (the 27-weight rows there made
-//   that kernel 4 us slower at 1M particles while the standalone scatter gained 4 us).
-template <int kT, bool kNodeWeights>
-struct ScatterWeights;
-template <int kT>
-struct ScatterWeights<kT, true> {
-    float w[27][kT + 1];
-    __device__ __forceinline__ void put(int tid, bool valid, const Stencil& st) {
-#pragma unroll
-        for (int ox = 0; ox < 3; ++ox)
-#pragma unroll
-            for (int oy = 0; oy < 3; ++oy) {
-                const float wxy = st.w[0][ox] * st.w[1][oy];
-#pragma unroll
-                for (int oz = 0; oz < 3; ++oz) w[9 * ox + 3 * oy + oz][tid] = valid ? wxy * st.w[2][oz] : 0.f;
-            }
-    }
-    // weight of node (ox, oy, oz) = lane j for particle k
-    __device__ __forceinline__ float get(int k, int j, int, int, int) const { return w[j][k]; }
-};
-template <int kT>
-struct ScatterWeights<kT, false> {
-    float w[kT][9];
-    __device__ __forceinline__ void put(int tid, bool valid, const Stencil& st) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int o = 0; o < 3; ++o) w[tid][3 * a + o] = valid ? st.w[a][o] : 0.f;
-    }
-    __device__ __forceinline__ float get(int k, int, int ox, int oy, int oz) const {
-        return w[k][ox] * w[k][3 + oy] * w[k][6 + oz];
-    }
-};
-
-template <int kT, int kTile, int kF = 4, bool kNodeWeights = true>
-struct TransportTile {
-    ScatterWeights<kT, kNodeWeights> w;
-    double val[kT][kF];
-    double tile[kF][kTile];
-};
-
-template <int kT, int kTile, int kF = 4, int kFirst = 0, bool kNodeWeights = true>
-__device__ void transport_scatter_block(TransportTile<kT, kTile, kF, kNodeWeights>& sm, const Params& P, const GridPtrs& g, int* box,
-                                        bool valid, const Stencil& st, const double* val) {
-    static_assert(kF >= 1 && kF <= 4 && kFirst + kF <= 7, "node fields 0..6, at most four at a time");
-    const int tid = threadIdx.x, lane = tid & 31;
-#pragma unroll
-    for (int f = 0; f < kF; ++f) sm.val[tid][f] = valid ? val[f] : 0.0;
-    sm.w.put(tid, valid, st);
-    const BlockBox bb = block_box(box, valid, st.b, kTile);  // synchronises the block
-    for (int t = tid; t < bb.count; t += kT)
-#pragma unroll
-        for (int f = 0; f < kF; ++f) sm.tile[f][t] = 0.0;
-    __syncthreads();
-    long long key = valid ? pack_base(st.b) : -1;
-    long long prev = __shfl_up_sync(kFull, key, 1);
-    unsigned starts = __ballot_sync(kFull, valid && (lane == 0 || prev != key));
-    const int warp_base = tid & ~31;
-    int ox, oy, oz;
-    node_offset(lane < 27 ? lane : 0, ox, oy, oz);
-    while (starts) {
-        int s = __ffs(starts) - 1;
-        starts &= starts - 1;
-        int e = starts ? __ffs(starts) - 1 : 32;
-        int b0 = __shfl_sync(kFull, st.b[0], s), b1 = __shfl_sync(kFull, st.b[1], s), b2 = __shfl_sync(kFull, st.b[2], s);
-        if (lane < 27) {
-            // Even and odd particles of the run into separate sums: two independent chains of
-            // float64 multiply-adds per field, so consecutive particles' loads and conversions overlap.
-            double acc[kF], acc_odd[kF];
-#pragma unroll
-            for (int f = 0; f < kF; ++f) acc[f] = acc_odd[f] = 0.0;
-            int k = warp_base + s;
-            const int k_end = warp_base + e;
-            for (; k + 1 < k_end; k += 2) {
-                const double w0 = (double)sm.w.get(k, lane, ox, oy, oz);
-                const double w1 = (double)sm.w.get(k + 1, lane, ox, oy, oz);
-#pragma unroll
-                for (int f = 0; f < kF; ++f) {
-                    acc[f] = fma(w0, sm.val[k][f], acc[f]);
-                    acc_odd[f] = fma(w1, sm.val[k + 1][f], acc_odd[f]);
-                }
-            }
-            if (k < k_end) {
-                const double w0 = (double)sm.w.get(k, lane, ox, oy, oz);
-#pragma unroll
-                for (int f = 0; f < kF; ++f) acc[f] = fma(w0, sm.val[k][f], acc[f]);
-            }
-#pragma unroll
-            for (int f = 0; f < kF; ++f) acc[f] += acc_odd[f];
-            if (bb.tiled) {
-                int t = tile_index(bb, b0 + ox, b1 + oy, b2 + oz);
-#pragma unroll
-                for (int f = 0; f < kF; ++f) atomicAdd(&sm.tile[f][t], acc[f]);
-            } else {
-                int64_t node = node_index(b0 + ox, b1 + oy, b2 + oz, P.R);
-#pragma unroll
-                for (int f = 0; f < kF; ++f) atomicAdd(g.f[kFirst + f] + node, acc[f]);
-            }
-        }
-    }
-    __syncthreads();
-    for (int t = tid; t < bb.count; t += kT) {
-        bool empty = true;
-#pragma unroll
-        for (int f = 0; f < kF; ++f) empty = empty && sm.tile[f][t] == 0.0;
-        if (empty) continue;
-        int64_t node = tile_node(bb, t, P.R);
-#pragma unroll
-        for (int f = 0; f < kF; ++f) atomicAdd(g.f[kFirst + f] + node, sm.tile[f][t]);
-    }
-}
-
 template <bool kRef = false>
-__device__ __forceinline__ void surface_owners_tile_body(Arg<Params, kRef> P, Arg<BkState, kRef> in,
+__device__ __forceinline__ void surface_owners_run_body(Arg<Params, kRef> P, Arg<BkState, kRef> in,
                                                          Arg<BkConstants, kRef> cst, Arg<BkSurface, kRef> sf,
                                                          Arg<GridPtrs, kRef> g, int32_t* sim_flags, Slot sl) {
-    __shared__ TransportTile<kOwnerThreads, kTileNodes, 3> sm;
+    __shared__ ScalarRecord<3> sm[kOwnerThreads / 32];
     const int64_t o = sl.block * (int64_t)kOwnerThreads + threadIdx.x;
     bool valid = false;
     Stencil st;
@@ -546,33 +347,35 @@ __device__ __forceinline__ void surface_owners_tile_body(Arg<Params, kRef> P, Ar
         if (!valid) set_flag(sim_flags, 1);
     }
     // the owners' nodes lie inside the particles' transport box: no box to widen
-    transport_scatter_block<kOwnerThreads, kTileNodes, 3, 4>(sm, P, g, nullptr, valid, st, rate);
+    scatter_scalars<3>(sm[threadIdx.x >> 5], valid, st, rate, {g.f[4], g.f[5], g.f[6]}, P.R);
 }
 
-// Many owners take the tiled form (one thread each), few the warp form (one warp each).
+// Many owners take the run form (one thread each), few the warp form (one warp each).
 template <bool kRef = false>
 __device__ __forceinline__ void surface_owners_body(Arg<Params, kRef> P, Arg<BkState, kRef> in, Arg<BkConstants, kRef> cst,
                                                     Arg<BkSurface, kRef> sf, Arg<GridPtrs, kRef> g, int32_t* sim_flags,
-                                                    bool tiled, Slot sl) {
-    if (tiled) surface_owners_tile_body<kRef>(P, in, cst, sf, g, sim_flags, sl);
+                                                    bool in_runs, Slot sl) {
+    if (in_runs) surface_owners_run_body<kRef>(P, in, cst, sf, g, sim_flags, sl);
     else surface_owners_warp_body<kRef>(P, in, cst, sf, g, sim_flags, sl);
 }
 
-// Whether a body with `owners` face owners among `n` particles takes the tiled form, and its blocks.
-inline bool owners_tiled(int64_t owners, int64_t n) { return owners * 16 >= n; }
+// Whether a body with `owners` face owners among `n` particles takes the run form, and its blocks.
+inline bool owners_in_runs(int64_t owners, int64_t n) { return owners * 16 >= n; }
 inline unsigned owner_blocks(int64_t owners, int64_t n) {
-    const int64_t threads = owners_tiled(owners, n) ? owners : owners * 32;
+    const int64_t threads = owners_in_runs(owners, n) ? owners : owners * 32;
     return (unsigned)((threads + kOwnerThreads - 1) / kOwnerThreads);
 }
 
 __global__ void __launch_bounds__(kOwnerThreads) k_surface_owners(Params P, BkState in, BkConstants cst, BkSurface sf,
-                                                                 GridPtrs g, int32_t* sim_flags, int tiled) {
+                                                                 GridPtrs g, int32_t* sim_flags, int in_runs) {
     pdl_enter();
-    surface_owners_body(P, in, cst, sf, g, sim_flags, tiled != 0, grid_slot());
+    surface_owners_body(P, in, cst, sf, g, sim_flags, in_runs != 0, grid_slot());
 }
 
-// 256 nodes: the 27 weight rows of 256 particles leave room for no larger tile in 48 KB of static shared memory.
-using ScatterTile = TransportTile<kThreads, 256>;
+// ---------------------------------------------------------- transport P2G
+// physics/thermal_water.py:108-137 (volume, capacity, energy, water) by warp runs (bk_scatter.cuh),
+// with the node box of the substep.
+using ScatterRecord = ScalarRecord<4>;
 
 template <bool kRef = false>
 __device__ __forceinline__ void transport_scatter_body(Arg<Params, kRef> P, Arg<BkState, kRef> in,
@@ -580,7 +383,7 @@ __device__ __forceinline__ void transport_scatter_body(Arg<Params, kRef> P, Arg<
                                                        Slot sl) {
     // Shared memory is declared in the bodies, not passed in: through a reference the compiler may
     // not see that it is shared memory and issue generic loads, stores and atomics.
-    __shared__ ScatterTile sm;
+    __shared__ ScatterRecord sm[kThreads / 32];
     const int64_t i = sl.block * (int64_t)kThreads + threadIdx.x;
     const int64_t pitch = P.pitch;
     bool valid = false;
@@ -599,10 +402,11 @@ __device__ __forceinline__ void transport_scatter_body(Arg<Params, kRef> P, Arg<
         val[2] = cap * in.temperature[i];
         val[3] = in.water[i];
     }
-    transport_scatter_block<kThreads, 256>(sm, P, g, g.bounds, valid, st, val);
+    widen_box(g.bounds, valid, st.b);
+    scatter_scalars<4>(sm[threadIdx.x >> 5], valid, st, val, {g.f[0], g.f[1], g.f[2], g.f[3]}, P.R);
 }
 
-__global__ void __launch_bounds__(kThreads) k_transport_scatter(Params P, BkState in, BkConstants cst, GridPtrs g,
+__global__ void __launch_bounds__(kThreads, 4) k_transport_scatter(Params P, BkState in, BkConstants cst, GridPtrs g,
                                                                int32_t* sim_flags) {
     pdl_enter();
     transport_scatter_body(P, in, cst, g, sim_flags, grid_slot());
@@ -828,203 +632,87 @@ __global__ void k_grid_update(Params P, GridPtrs g) {
 // ------------------------------------------------------------- fused P2G
 // Scalar G2P (thermal_water.py:206-229), local gas source (:238-245), gas stress (gas.py:16-35),
 // water stress (thermal_water.py:248-253) and momentum P2G (transfer.py:47-70) for one particle
-// per thread, then the warp-cooperative momentum scatter.
-// One particle's scatter record: its 27 stencil weights (w_x w_y) w_z, formed once by its own
-// thread, in node-major rows of kThreads + 1 floats (lane j of a run reads row j at the particle's
-// column: one conflict-free load per node in place of three loads and two multiplies), and
-// {m q0 q1 q2} {A0 A1 A2 A3} {A4 A5 A6 A7} read as 128-bit broadcasts plus A8.
-// The staged form first copies the block's particle planes (x, v, C, F and, for Ding, tau: 33
-// planes of 256 floats) into shared memory with bulk copies (cp.async.bulk, the TMA engine's 1-D
-// copy) issued by one thread and counted on an mbarrier, so the loads of a block are in flight
-// together and each thread then reads its particle's 33 values from shared memory; the scatter
-// records reuse that space once every thread has read it.
-// A full block (256 particles) also stages its per-particle scalars: temperature, water, dry mass
-// and gas content (float64), reference volume, gas source rate and porosity (float32), those the
-// substep reads; the last, partial block loads them directly (the arrays need not extend past n).
-constexpr int kP2GPlanes = 33;
-struct P2GSmem {
-    union {
-        struct {
-            float planes[kP2GPlanes][kThreads];  // x 0-2 (unused: x is read directly), v 3-5, C 6-14, F 15-23, tau 24-32
-            double d[4][kThreads];               // temperature, water, dry mass, gas moles
-            float f[3][kThreads];                // reference volume, gas source rate, porosity
-        } in;
-        struct {
-            float4 val[kThreads][3];
-            float a8[kThreads];
-            float w[27][kThreads + 1];
-        } rec;
-    };
-    float4 tile[kTileNodes];
-    unsigned long long mbar;
-};
-// Above the 48 KB of static shared memory: the kernels take it as dynamic shared memory, opted in
-// per device before their first launch there.
-constexpr size_t kP2GSmemBytes = sizeof(P2GSmem);
+// per thread, then the momentum scatter by warp runs (bk_scatter.cuh). Bound by the LSU data pipe
+// (69% of its peak at 1M particles: the run loop's broadcasts and the node gather) and by the loads'
+// latency behind it. Loads are plain: staging the block's planes by bulk copies (33 KB and two
+// barriers a block) took 87.0 us where this form, with its L2 prefetch and no barrier, takes 82.
+// Blocks of 128 against 256: 81.8 and 84.2 us at 1M particles (no barrier spans a block, so the size
+// only sets how early a finished block's slot is refilled).
+constexpr int kP2GThreads = 128;
 
-// Which per-particle scalars a full P2G block stages (bit k of d[k], bit 4 + k of f[k]).
-__host__ __device__ inline unsigned p2g_staged_scalars(int transport, int gas, int material, int rate_per_particle) {
-    unsigned m = 0;
-    if (transport) m |= 1u | 2u | 4u | 16u;
-    if (transport && gas) m |= 8u | (rate_per_particle ? 32u : 0u);
-    if (material == 1 && gas) m |= 64u;
-    return m;
-}
-
-// OR of the base addresses the bulk-staged P2G copies from (each must be 16-byte aligned).
-inline uintptr_t p2g_stage_bases(const BkSubstepParams& p, const BkState& in, const BkConstants& c) {
-    uintptr_t b = (uintptr_t)in.x | (uintptr_t)in.v | (uintptr_t)in.C | (uintptr_t)in.F |
-                  (p.material == 1 ? (uintptr_t)in.tau : 0);
-    const unsigned m = p2g_staged_scalars(p.transport, p.gas, p.material, c.gas_rate_per_particle);
-    if (m & 1u) b |= (uintptr_t)in.temperature;
-    if (m & 2u) b |= (uintptr_t)in.water;
-    if (m & 4u) b |= (uintptr_t)c.dry_mass;
-    if (m & 8u) b |= (uintptr_t)in.gas_moles;
-    if (m & 16u) b |= (uintptr_t)c.volume;
-    if (m & 32u) b |= (uintptr_t)c.gas_rate;
-    if (m & 64u) b |= (uintptr_t)in.porosity;
-    return b;
-}
-
-// Opts `kernel` into `bytes` of dynamic shared memory on the current device. Set on every launch:
-// a host call without device work, and correct after a device reset or in another context.
-int allow_smem(const void* kernel, size_t bytes, const char* what) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
-        return check_launch(what);
-    return 0;
-}
-
-namespace stage {
-// Polls of a bulk copy's mbarrier before a block gives up (far beyond any copy's latency).
-constexpr uint32_t kWaitPolls = 1u << 22;
-
-__device__ __forceinline__ void arrive_expect_tx(uint32_t mbar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
-}
-
-// 1-D bulk copy global -> this CTA's shared memory, completing `bytes` on the mbarrier. Both
-// addresses 16-byte aligned, bytes a multiple of 16.
-__device__ __forceinline__ void copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t mbar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(dst), "l"(src), "r"(bytes), "r"(mbar)
-                 : "memory");
-}
-}  // namespace stage
-
-// Four 256-thread blocks per SM (64 registers) measured faster than three at 77 registers.
-template <bool kStaged, bool kRef = false>
+template <bool kRef = false>
 __device__ __forceinline__ void p2g_body(Arg<Params, kRef> P, Arg<BkState, kRef> in, Arg<BkState, kRef> out,
                                          Arg<BkConstants, kRef> cst, Arg<GridPtrs, kRef> g, Arg<BkFlags, kRef> flags,
                                          float* max_residuals, Slot sl) {
-    extern __shared__ __align__(16) unsigned char p2g_smem[];
-    P2GSmem& sm = *reinterpret_cast<P2GSmem*>(p2g_smem);
+    __shared__ MomentumRecord sm[kP2GThreads / 32];
     if (sl.block == 0 && threadIdx.x < 2) max_residuals[threadIdx.x] = 0.0f;
-    const int tid = threadIdx.x, lane = tid & 31;
-    const int64_t i = sl.block * (int64_t)kThreads + tid;
+    const int64_t i = sl.block * (int64_t)kP2GThreads + threadIdx.x;
     const int64_t pitch = P.pitch;
-    // Scalars this block reads from shared memory (full blocks of the staged form), by bit as in
-    // p2g_staged_scalars; the others are loaded directly.
-    const unsigned staged_scalars =
-        kStaged && P.n - (int64_t)sl.block * kThreads >= kThreads
-            ? p2g_staged_scalars(P.transport, P.gas, P.material, cst.gas_rate_per_particle) : 0u;
-    // The particle's stencil and its scalar G2P of the diffused node fields (thermal_water.py:206-215)
-    // read only x and the grid: the staged form runs them while its bulk copies are in flight.
+    {
+        // v, C, F and tau planes by lane, then the scalars' lines (two per float64 array)
+        const int lane = threadIdx.x & 31;
+        const int64_t w0 = i - lane;
+        if (w0 < P.n) {
+            if (lane < (P.material == 1 ? 30 : 21)) {
+                const float* a = lane < 3 ? in.v + lane * pitch : lane < 12 ? in.C + (lane - 3) * pitch
+                                 : lane < 21 ? in.F + (lane - 12) * pitch : in.tau + (lane - 21) * pitch;
+                prefetch_l2(a + w0);
+            }
+            if (P.transport && lane < 8) {
+                const double* a = lane < 2 ? in.temperature : lane < 4 ? in.water : lane < 6 ? cst.dry_mass : in.gas_moles;
+                if (lane < 6 || P.gas) prefetch_l2(a + (w0 + 16 * (lane & 1) < P.n ? w0 + 16 * (lane & 1) : w0));
+            }
+            if (lane == 8) prefetch_l2(cst.volume + w0);
+            if (lane == 9 && P.material == 1 && P.gas) prefetch_l2(in.porosity + w0);
+            if (lane == 10 && P.gas && cst.gas_rate_per_particle) prefetch_l2(cst.gas_rate + w0);
+        }
+    }
     bool valid = false;
     Stencil st;
     st.b[0] = st.b[1] = st.b[2] = 0;
-    double dTp = 0.0, ratio = 0.0;
-    auto stencil_and_gather = [&]() {
-        if (i < P.n) {
-            st = make_stencil(load_v3(in.x, i, pitch), P.origin, P.dx, P.R);
-            valid = st.valid;
-            if (!valid) set_flag(flags.simulation, 1);
-        }
-        if (valid && P.transport) {
-#pragma unroll
-            for (int ox = 0; ox < 3; ++ox)
-#pragma unroll
-                for (int oy = 0; oy < 3; ++oy)
-#pragma unroll
-                    for (int oz = 0; oz < 3; ++oz) {
-                        double w = (double)(st.w[0][ox] * st.w[1][oy] * st.w[2][oz]);
-                        double2 d = __ldg(g.dTr + node_index(st.b[0] + ox, st.b[1] + oy, st.b[2] + oz, P.R));
-                        dTp += w * d.x;
-                        ratio += w * d.y;
-                    }
-        }
-    };
-    if constexpr (kStaged) {
-        // Planes are pitch-long with a pitch that is a multiple of 4 and 16-byte aligned bases (the
-        // host checks), so the block's range rounded up to 16 bytes stays inside each plane. The x
-        // planes are not copied: x is read directly, before the wait.
-        const uint32_t mbar = mlp::smem_addr(&sm.mbar);
-        if (tid == 0) mlp::mbar_init(mbar, 1);
-        __syncthreads();
-        const int64_t start = (int64_t)sl.block * kThreads;
-        if (tid == 0) {
-            const int64_t count = P.n - start < kThreads ? P.n - start : kThreads;
-            const uint32_t bytes = (uint32_t)((count * 4 + 15) & ~15ll);
-            const int arrays = P.material == 1 ? 5 : 4;
-            const float* src[5] = {in.x, in.v, in.C, in.F, in.tau};
-            const int planes[5] = {3, 3, 9, 9, 9};
-            const unsigned m = count == kThreads ? staged_scalars : 0u;
-            uint32_t total = bytes * (uint32_t)(P.material == 1 ? kP2GPlanes - 3 : kP2GPlanes - 12);
-#pragma unroll
-            for (int k = 0; k < 7; ++k)
-                if (m & (1u << k)) total += k < 4 ? kThreads * 8 : kThreads * 4;
-            stage::arrive_expect_tx(mbar, total);
-            int k = 3;
-            for (int a = 1; a < arrays; ++a)
-                for (int c = 0; c < planes[a]; ++c, ++k)
-                    stage::copy(mlp::smem_addr(&sm.in.planes[k][0]), src[a] + c * pitch + start, bytes, mbar);
-            const double* dsrc[4] = {in.temperature, in.water, cst.dry_mass, in.gas_moles};
-            const float* fsrc[3] = {cst.volume, cst.gas_rate, in.porosity};
-            for (int k = 0; k < 4; ++k)
-                if (m & (1u << k)) stage::copy(mlp::smem_addr(&sm.in.d[k][0]), dsrc[k] + start, kThreads * 8, mbar);
-            for (int k = 0; k < 3; ++k)
-                if (m & (16u << k)) stage::copy(mlp::smem_addr(&sm.in.f[k][0]), fsrc[k] + start, kThreads * 4, mbar);
-        }
-        stencil_and_gather();
-        const bool arrived = __syncthreads_and(mlp::mbar_wait(mbar, 0, stage::kWaitPolls)) != 0;
-        if (!arrived) {
-            // Leave this block's particles unprocessed and report it; wait (bounded) for the copies
-            // still in flight into this block's shared memory before leaving.
-            if (tid == 0 && P.status) atomicExch(P.status, 1);
-            mlp::mbar_wait(mbar, 0, stage::kWaitPolls);
-            return;
-        }
-    } else {
-        stencil_and_gather();
+    if (i < P.n) {
+        st = make_stencil(load_v3(in.x, i, pitch), P.origin, P.dx, P.R);
+        valid = st.valid;
+        if (!valid) set_flag(flags.simulation, 1);
     }
-    // This particle's plane arrays: from the staged copies or from global memory.
-    auto ld_v3 = [&](const float* src, int plane0) {
-        if constexpr (kStaged) return V3{{sm.in.planes[plane0][tid], sm.in.planes[plane0 + 1][tid], sm.in.planes[plane0 + 2][tid]}};
-        else return load_v3(src, i, pitch);
-    };
-    auto ld_m3 = [&](const float* src, int plane0) {
-        if constexpr (kStaged) {
-            M3 r;
-#pragma unroll
-            for (int c = 0; c < 9; ++c) r.m[c] = sm.in.planes[plane0 + c][tid];
-            return r;
-        } else {
-            return load_m3(src, i, pitch);
-        }
-    };
+    // The transport scatter of this substep has widened the box over the same positions already.
+    if (!P.transport || P.prescattered) widen_box(g.bounds, valid, st.b);
     float mass = 0.f, q[3] = {0.f, 0.f, 0.f}, A[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (valid) {
-        M3 F = ld_m3(in.F, 15);
+        M3 F = load_m3(in.F, i, pitch);
         float J = det3(F);
         M3 tau;
         float T_mat = 0.f;
         float rho_ref = P.density;
-        double sat = 0.0;
+        double sat = 0.0, N = 0.0;
         if (P.transport) {
-            double T_old = (staged_scalars & 1u) ? sm.in.d[0][tid] : in.temperature[i];
+            // The scalar G2P of the diffused node fields (thermal_water.py:206-215), axis by axis.
+            double dTp = 0.0, ratio = 0.0;
+            const double2* nodes = g.dTr + node_index(st.b[0], st.b[1], st.b[2], P.R);
+            const int64_t R = P.R;
+#pragma unroll
+            for (int ox = 0; ox < 3; ++ox) {
+                double tx = 0.0, rx = 0.0;
+#pragma unroll
+                for (int oy = 0; oy < 3; ++oy) {
+                    double ty = 0.0, ry = 0.0;
+#pragma unroll
+                    for (int oz = 0; oz < 3; ++oz) {
+                        const double2 d = __ldg(nodes + (ox * R + oy) * R + oz);
+                        ty = fma((double)st.w[2][oz], d.x, ty);
+                        ry = fma((double)st.w[2][oz], d.y, ry);
+                    }
+                    tx = fma((double)st.w[1][oy], ty, tx);
+                    rx = fma((double)st.w[1][oy], ry, rx);
+                }
+                dTp = fma((double)st.w[0][ox], tx, dTp);
+                ratio = fma((double)st.w[0][ox], rx, ratio);
+            }
+            double T_old = in.temperature[i];
             double Tn = T_old + dTp;
-            double Wn = ((staged_scalars & 2u) ? sm.in.d[1][tid] : in.water[i]) * (1.0 + ratio);
-            double dry = (staged_scalars & 4u) ? sm.in.d[2][tid] : cst.dry_mass[i];
-            float V0 = (staged_scalars & 16u) ? sm.in.f[0][tid] : cst.volume[i];
+            double Wn = in.water[i] * (1.0 + ratio);
+            double dry = cst.dry_mass[i];
+            float V0 = cst.volume[i];
             out.temperature[i] = Tn;
             out.water[i] = Wn;
             mass = (float)(dry + Wn);
@@ -1032,13 +720,11 @@ __device__ __forceinline__ void p2g_body(Arg<Params, kRef> P, Arg<BkState, kRef>
             sat = Wn / ((double)P.water_density * (double)V0 * (double)J);
             T_mat = (float)Tn;
             if (P.gas) {
-                double N = (staged_scalars & 8u) ? sm.in.d[3][tid] : in.gas_moles[i];
+                N = in.gas_moles[i];
                 if (!P.settling) {
                     double Tm = 0.5 * (T_old + Tn);
                     double z = (Tm - (double)P.peak) / (double)P.width;
-                    const float rate = (staged_scalars & 32u) ? sm.in.f[1][tid]
-                                                              : cst.gas_rate[cst.gas_rate_per_particle ? i : 0];
-                    N += (double)(P.dt * P.density) * (double)rate * exp(-(z * z));
+                    N += (double)(P.dt * P.density) * (double)cst.gas_rate[cst.gas_rate_per_particle ? i : 0] * exp(-(z * z));
                 }
                 out.gas_moles[i] = N;
             }
@@ -1047,13 +733,13 @@ __device__ __forceinline__ void p2g_body(Arg<Params, kRef> P, Arg<BkState, kRef>
             if (P.material == 1) T_mat = in.material_temperature[i];
         }
         if (P.material == 1) {
-            tau = ld_m3(in.tau, 24);
+            tau = load_m3(in.tau, i, pitch);
             if (P.gas) {
-                float n = (staged_scalars & 64u) ? sm.in.f[2][tid] : in.porosity[i];
+                float n = in.porosity[i];
                 if (n <= 0.0f || n >= 1.0f || !isfinite(n) || J <= 0.0f) {
                     set_flag(flags.ding, 0);
                 } else {
-                    float p = (float)gas_pressure(out.gas_moles[i], T_mat, J, n);
+                    float p = (float)gas_pressure(N, T_mat, J, n);
                     float iso = J * (P.ambient - p);
 #pragma unroll
                     for (int e = 0; e < 9; ++e) tau.m[e] += (e % 4) == 0 ? iso : iso * 0.0f;
@@ -1084,9 +770,9 @@ __device__ __forceinline__ void p2g_body(Arg<Params, kRef> P, Arg<BkState, kRef>
 #pragma unroll
             for (int e = 0; e < 9; ++e) tau.m[e] -= (e % 4) == 0 ? iso : iso * 0.0f;
         }
-        float scale = P.dt * ((staged_scalars & 16u) ? sm.in.f[0][tid] : cst.volume[i]) * 4.0f / (P.dx * P.dx);
-        M3 Cm = ld_m3(in.C, 6);
-        V3 vel = ld_v3(in.v, 3);
+        float scale = P.dt * cst.volume[i] * 4.0f / (P.dx * P.dx);
+        M3 Cm = load_m3(in.C, i, pitch);
+        V3 vel = load_v3(in.v, i, pitch);
 #pragma unroll
         for (int e = 0; e < 9; ++e) A[e] = mass * Cm.m[e] - scale * tau.m[e];
         // w (m v + A (o - l) dx) = w (q + A dx o) with q = m v - A l dx.
@@ -1096,89 +782,15 @@ __device__ __forceinline__ void p2g_body(Arg<Params, kRef> P, Arg<BkState, kRef>
 #pragma unroll
         for (int e = 0; e < 9; ++e) A[e] *= P.dx;
     }
-    if constexpr (kStaged) __syncthreads();  // every thread has read its planes: the records reuse them
-    {
-#pragma unroll
-        for (int ox = 0; ox < 3; ++ox)
-#pragma unroll
-            for (int oy = 0; oy < 3; ++oy) {
-                const float wxy = st.w[0][ox] * st.w[1][oy];
-#pragma unroll
-                for (int oz = 0; oz < 3; ++oz) sm.rec.w[9 * ox + 3 * oy + oz][tid] = valid ? wxy * st.w[2][oz] : 0.f;
-            }
-        sm.rec.val[tid][0] = make_float4(mass, q[0], q[1], q[2]);
-        sm.rec.val[tid][1] = make_float4(A[0], A[1], A[2], A[3]);
-        sm.rec.val[tid][2] = make_float4(A[4], A[5], A[6], A[7]);
-        sm.rec.a8[tid] = A[8];
-    }
-    const BlockBox bb = block_box(g.bounds, valid, st.b);  // synchronises the block
-    for (int t = tid; t < bb.count; t += kThreads) sm.tile[t] = make_float4(0.f, 0.f, 0.f, 0.f);
-    __syncthreads();
-    long long key = valid ? pack_base(st.b) : -1;
-    long long prev = __shfl_up_sync(kFull, key, 1);
-    unsigned starts = __ballot_sync(kFull, valid && (lane == 0 || prev != key));
-    const int warp_base = tid & ~31;
-    int ox, oy, oz;
-    node_offset(lane < 27 ? lane : 0, ox, oy, oz);
-    const float fo[3] = {(float)ox, (float)oy, (float)oz};
-    while (starts) {
-        int s = __ffs(starts) - 1;
-        starts &= starts - 1;
-        int e = starts ? __ffs(starts) - 1 : 32;
-        int b0 = __shfl_sync(kFull, st.b[0], s), b1 = __shfl_sync(kFull, st.b[1], s), b2 = __shfl_sync(kFull, st.b[2], s);
-        if (lane < 27) {
-            // Node j receives sum_k w_jk (m_k, q_k + A_k o_j): accumulate sum w m, sum w q, sum w A
-            // (paired accumulators, one packed multiply-add per pair) and apply the node's offset
-            // o_j once per run.
-            float2 mq0 = {0.f, 0.f}, q12 = {0.f, 0.f}, A01 = {0.f, 0.f}, A23 = {0.f, 0.f};
-            float2 A45 = {0.f, 0.f}, A67 = {0.f, 0.f};
-            float A8 = 0.f;
-            const float* wj = sm.rec.w[lane];
-#pragma unroll 2
-            for (int k = warp_base + s; k < warp_base + e; ++k) {
-                const float w = wj[k];
-                const float2 ww = make_float2(w, w);
-                const float4 v0 = sm.rec.val[k][0], v1 = sm.rec.val[k][1], v2 = sm.rec.val[k][2];
-                mq0 = ffma2(ww, make_float2(v0.x, v0.y), mq0);
-                q12 = ffma2(ww, make_float2(v0.z, v0.w), q12);
-                A01 = ffma2(ww, make_float2(v1.x, v1.y), A01);
-                A23 = ffma2(ww, make_float2(v1.z, v1.w), A23);
-                A45 = ffma2(ww, make_float2(v2.x, v2.y), A45);
-                A67 = ffma2(ww, make_float2(v2.z, v2.w), A67);
-                A8 = fmaf(w, sm.rec.a8[k], A8);
-            }
-            const float am = mq0.x;
-            const float aq[3] = {mq0.y, q12.x, q12.y};
-            const float aA[9] = {A01.x, A01.y, A23.x, A23.y, A45.x, A45.y, A67.x, A67.y, A8};
-            float ap[3];
-#pragma unroll
-            for (int r = 0; r < 3; ++r)
-                ap[r] = aq[r] + (aA[3 * r] * fo[0] + aA[3 * r + 1] * fo[1] + aA[3 * r + 2] * fo[2]);
-            if (bb.tiled) {
-                float* cell = reinterpret_cast<float*>(&sm.tile[tile_index(bb, b0 + ox, b1 + oy, b2 + oz)]);
-                atomicAdd(cell + 0, ap[0]);
-                atomicAdd(cell + 1, ap[1]);
-                atomicAdd(cell + 2, ap[2]);
-                atomicAdd(cell + 3, am);
-            } else {
-                atomicAdd(g.pm + node_index(b0 + ox, b1 + oy, b2 + oz, P.R), make_float4(ap[0], ap[1], ap[2], am));
-            }
-        }
-    }
-    __syncthreads();
-    for (int t = tid; t < bb.count; t += kThreads) {
-        float4 v = sm.tile[t];
-        if (v.w == 0.0f && v.x == 0.0f && v.y == 0.0f && v.z == 0.0f) continue;
-        atomicAdd(g.pm + tile_node(bb, t, P.R), v);
-    }
+    scatter_momentum(sm[threadIdx.x >> 5], valid, st, mass, q, A, g.pm, P.R);
 }
 
-template <bool kStaged, bool kLoaf = false>
-__global__ void __launch_bounds__(kThreads, 4) k_p2g(Params P, BkState in, BkState out, BkConstants cst, GridPtrs g,
+template <bool kLoaf = false>
+__global__ void __launch_bounds__(kP2GThreads, 8) k_p2g(Params P, BkState in, BkState out, BkConstants cst, GridPtrs g,
                                                  BkFlags flags, float* max_residuals) {
     pdl_enter();
     if constexpr (kLoaf) fix_loaf_mode(P);
-    p2g_body<kStaged>(P, in, out, cst, g, flags, max_residuals, grid_slot());
+    p2g_body(P, in, out, cst, g, flags, max_residuals, grid_slot());
 }
 
 // ------------------------------------------------------ fused G2P + return
@@ -1431,9 +1043,8 @@ __device__ __forceinline__ void g2p_return_particle(const Params& P, const BkSta
     }
 }
 
-// Shared-memory node tile of the transport prescatter in k_g2p_return (128 particles per block).
-constexpr int kG2PTile = 256;
-using G2PTransportTile = TransportTile<128, kG2PTile, 4, false>;
+// Dynamic shared memory of the transport prescatter in k_g2p_return (128 particles per block).
+constexpr size_t kG2PScatterBytes = 4 * sizeof(ScatterRecord);
 
 template <bool kRef = false>
 __device__ __forceinline__ void g2p_return_body(Arg<Params, kRef> P, Arg<BkState, kRef> in,
@@ -1453,7 +1064,7 @@ __device__ __forceinline__ void g2p_return_body(Arg<Params, kRef> P, Arg<BkState
         // x' and F' by this thread (read back with plain loads), T' and W' by this substep's P2G.
         // The grid update has zeroed the transport fields over this substep's box and restarted
         // the prescatter box bounds[12..17]. Uniform branch: every thread of the block scatters.
-        G2PTransportTile& sm = *reinterpret_cast<G2PTransportTile*>(g2p_smem);
+        ScatterRecord* sm = reinterpret_cast<ScatterRecord*>(g2p_smem);
         const int64_t pitch = P.pitch;
         bool valid = false;
         Stencil st;
@@ -1472,7 +1083,8 @@ __device__ __forceinline__ void g2p_return_body(Arg<Params, kRef> P, Arg<BkState
                 val[3] = out.water[i];
             }
         }
-        transport_scatter_block<128, kG2PTile, 4, 0, false>(sm, P, g, g.bounds + 12, valid, st, val);
+        widen_box(g.bounds + 12, valid, st.b);
+        scatter_scalars<4>(sm[threadIdx.x >> 5], valid, st, val, {g.f[0], g.f[1], g.f[2], g.f[3]}, P.R);
     }
 }
 
@@ -1727,7 +1339,7 @@ int bk_substep(const BkSubstepParams* params, const BkState* in, BkState* out, c
                 int rec = profile_begin("surface_owners", s);
                 e = launch_chained(k_surface_owners, owner_blocks(surface->owner_count, p.n), kOwnerThreads, 0, s, P,
                                    *in, *constants, *surface, g, flags->simulation,
-                                   (int)owners_tiled(surface->owner_count, p.n));
+                                   (int)owners_in_runs(surface->owner_count, p.n));
                 profile_end(rec, s);
             }
             if (int rc = check_chained(e, "bk_substep/surface_owners")) return rc;
@@ -1761,17 +1373,9 @@ int bk_substep(const BkSubstepParams* params, const BkState* in, BkState* out, c
         if (int rc = check_chained(e, "bk_substep/clear_previous")) return rc;
         {
             int rec = profile_begin("p2g", s);
-            // Bulk staging needs 16-byte aligned plane starts: a pitch that is a multiple of 4 floats
-            // and 16-byte aligned array bases.
-            const bool staged = p.pitch % 4 == 0 && (p2g_stage_bases(p, *in, *constants) & 15) == 0;
-            if (int rc = allow_smem(staged ? (loaf_mode(p, *diagnostics) ? (const void*)k_p2g<true, true> : (const void*)k_p2g<true>)
-                                           : (loaf_mode(p, *diagnostics) ? (const void*)k_p2g<false, true> : (const void*)k_p2g<false>),
-                                    kP2GSmemBytes, "bk_substep/p2g"))
-                return rc;
-            const bool loaf = loaf_mode(p, *diagnostics);
-            auto* kernel = staged ? (loaf ? k_p2g<true, true> : k_p2g<true>) : (loaf ? k_p2g<false, true> : k_p2g<false>);
-            e = launch_chained(kernel, particle_blocks, kThreads, kP2GSmemBytes, s, P, *in, *out, *constants, g, *flags,
-                               diagnostics->max_residuals);
+            e = launch_chained(loaf_mode(p, *diagnostics) ? k_p2g<true> : k_p2g<false>, blocks_for(p.n, kP2GThreads),
+                               kP2GThreads, 0, s, P,
+                               *in, *out, *constants, g, *flags, diagnostics->max_residuals);
             profile_end(rec, s);
         }
         if (int rc = check_chained(e, "bk_substep/p2g")) return rc;
@@ -1792,7 +1396,7 @@ int bk_substep(const BkSubstepParams* params, const BkState* in, BkState* out, c
             profile_end(rec, s);
         } else {
             int rec = profile_begin("g2p_return", s);
-            const size_t smem = p.transport_prescatter_next ? sizeof(G2PTransportTile) : 0;
+            const size_t smem = p.transport_prescatter_next ? kG2PScatterBytes : 0;
             auto* kernel = !loaf_mode(p, *diagnostics)       ? k_g2p_return<false>
                            : p.transport_prescatter_next ? k_g2p_return<true, true>
                                                          : k_g2p_return<true, false>;
@@ -1862,7 +1466,7 @@ struct BatchEntry {
     BkFlags flags;
     SurrogateDev sg;   // sf carries the surface accumulators of `out`
     int prescatter_ok;  // takes part in the transport prescatter
-    int owners_tiled;   // the surface terms take the tiled form (owners_tiled)
+    int owners_in_runs;   // the surface terms take the run form (owners_in_runs)
 };
 static_assert(sizeof(BatchEntry) % 4 == 0, "entries are copied as 4-byte words");
 
@@ -1911,7 +1515,7 @@ __global__ void __launch_bounds__(kBlock == 32 ? 32 * kVertexWarps : kBlock) kb_
 __global__ void __launch_bounds__(kOwnerThreads) kb_surface_owners(BatchArgs b) {
     __shared__ BatchEntry e;
     const Slot sl = batch_load(b, kStOwners, e);
-    surface_owners_body<true>(e.P, e.in, e.cst, e.sf, e.g, e.flags.simulation, e.owners_tiled != 0, sl);
+    surface_owners_body<true>(e.P, e.in, e.cst, e.sf, e.g, e.flags.simulation, e.owners_in_runs != 0, sl);
 }
 
 __global__ void __launch_bounds__(kThreads) kb_transport_scatter(BatchArgs b) {
@@ -1933,11 +1537,10 @@ __global__ void __launch_bounds__(kThreads) kb_clear_previous(BatchArgs b) {
     clear_previous_body<true>(e.P, e.g, sl);
 }
 
-template <bool kStaged>
-__global__ void __launch_bounds__(kThreads, 4) kb_p2g(BatchArgs b) {
+__global__ void __launch_bounds__(kP2GThreads, 8) kb_p2g(BatchArgs b) {
     __shared__ BatchEntry e;
     const Slot sl = batch_load(b, kStP2G, e);
-    p2g_body<kStaged, true>(e.P, e.in, e.out, e.cst, e.g, e.flags, e.diag.max_residuals, sl);
+    p2g_body<true>(e.P, e.in, e.out, e.cst, e.g, e.flags, e.diag.max_residuals, sl);
 }
 
 __global__ void __launch_bounds__(kThreads) kb_grid_update(BatchArgs b) {
@@ -1968,7 +1571,6 @@ struct BkBatch {
     uint32_t owner_offset[kBatchStages] = {};
     uint32_t total[kBatchStages] = {};
     int vertex_block = 32;
-    bool staged = true;             // every instance allows the bulk-staged P2G
     bool all_prescatter = true;     // every transport instance takes part in the prescatter
     bool any_transport = false;
 };
@@ -2023,8 +1625,7 @@ int bk_batch_create(const BkBatchInstance* instances, int32_t count, BkBatch** b
             e.flags = in.flags;
             e.sg = surrogate_dev(surrogate ? p.surrogate : nullptr);
             e.prescatter_ok = p.transport && !p.keep_transport_fields && !surrogate;
-            e.owners_tiled = owners_tiled(in.surface.owner_count, p.n);
-            host.staged = host.staged && p.pitch % 4 == 0 && (p2g_stage_bases(p, a, in.constants) & 15) == 0;
+            e.owners_in_runs = owners_in_runs(in.surface.owner_count, p.n);
         }
         host.any_transport = host.any_transport || p.transport;
         if (p.transport && (p.keep_transport_fields || surrogate)) host.all_prescatter = false;
@@ -2036,11 +1637,13 @@ int bk_batch_create(const BkBatchInstance* instances, int32_t count, BkBatch** b
                 blocks[kStOwners] = owner_blocks(in.surface.owner_count, n);
                 blocks[kStScatter] = blocks_for(n, kThreads);
             }
-            // node-box passes: about one block per 2048 particles (256 nodes at 8 particles a cell)
-            const uint32_t box = (uint32_t)std::min<int64_t>(std::max<int64_t>(1, (n + 2047) / 2048), 4 * sms);
-            if (p.transport) blocks[kStDiffuse] = box;
+            // Node-box passes: the diffusion takes a block per 256 particles (a tile of 256 nodes costs it
+            // ~3 us, and a ball's box holds about one node per particle: with a block per 2048 particles
+            // 12 balls of 4.8-11.2k particles took 54 us, now 15), the clears one per 1024.
+            const uint32_t box = (uint32_t)std::min<int64_t>((n + 1023) / 1024, 4 * sms);
+            if (p.transport) blocks[kStDiffuse] = (uint32_t)std::min<int64_t>((n + 255) / 256, 4 * sms);
             blocks[kStClear] = box;
-            blocks[kStP2G] = blocks_for(n, kThreads);
+            blocks[kStP2G] = blocks_for(n, kP2GThreads);
             blocks[kStGrid] = box;
             if (surrogate) {
                 // a persistent share of 4 CTAs per SM in proportion to the particles
@@ -2143,11 +1746,7 @@ int bk_batch_substep(BkBatch* batch, int32_t parity, int32_t phases, int32_t pre
         }
         if (T[kStP2G]) {
             int rec = profile_begin("batch_p2g", s);
-            if (int rc = allow_smem(B.staged ? (const void*)kb_p2g<true> : (const void*)kb_p2g<false>,
-                                    kP2GSmemBytes, "bk_batch_substep/p2g"))
-                return rc;
-            if (B.staged) kb_p2g<true><<<T[kStP2G], kThreads, kP2GSmemBytes, s>>>(a);
-            else kb_p2g<false><<<T[kStP2G], kThreads, kP2GSmemBytes, s>>>(a);
+            kb_p2g<<<T[kStP2G], kP2GThreads, 0, s>>>(a);
             profile_end(rec, s);
             if (int rc = check_launch("bk_batch_substep/p2g")) return rc;
         }
@@ -2159,7 +1758,7 @@ int bk_batch_substep(BkBatch* batch, int32_t parity, int32_t phases, int32_t pre
         }
         if (T[kStG2P]) {
             int rec = profile_begin("batch_g2p_return", s);
-            const size_t smem = prescatter_next ? sizeof(G2PTransportTile) : 0;
+            const size_t smem = prescatter_next ? kG2PScatterBytes : 0;
             kb_g2p_return<<<T[kStG2P], 128, smem, s>>>(a);
             profile_end(rec, s);
             if (int rc = check_launch("bk_batch_substep/g2p_return")) return rc;
