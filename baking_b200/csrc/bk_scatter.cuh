@@ -14,7 +14,7 @@
 // of ~18 particles already divides the atomics by 18, and L2 takes the rest without waiting. 1M
 // particles, 128^3 grid, 40 particles a cell, fused P2G kernel: 102 us with the tile, 87 us with the
 // same kernel writing straight to L2; transport scatter 68.5 against 62.1 us, 55 with the float64
-// tensor cores; in tet order P2G of 41k particles 37 against 16 us.
+// tensor cores; in tet order P2G of 41k particles 37 against 16 us, 8.6 with grouped lanes.
 #pragma once
 
 #include <climits>
@@ -32,31 +32,72 @@ BK_DEV void node_offset(int j, int& ox, int& oy, int& oz) {
     oz = j - 9 * ox - 3 * oy;
 }
 
-// The columns of the warp's record (one per lane) that start a run: bit k is set when lane k holds a
-// valid particle whose stencil base differs from lane k - 1's.
-BK_DEV unsigned run_starts(bool valid, const int* b) {
+// How a warp's particles are laid out in its record: this lane's column, and the columns that start a
+// run (bit k: column k holds a valid particle whose stencil base differs from column k - 1's).
+struct Runs {
+    int column;
+    unsigned starts;
+};
+
+// A warp with this many runs first groups its lanes by stencil base, in bodies of this many particles
+// (grids up to 1024^3, whose bases fit 3 x 10 bits). Particles ordered by cell have 2 (40 a cell) to 5
+// (8 a cell) runs a warp and gain nothing; particles in another order, as sampled tet by tet (up to 32
+// runs a warp, about 10 bases), get a third of the atomics, and node sums of fewer and larger parts.
+// P2G in tet order: 41k particles 16 -> 8.6 us, 5k 9.7 -> 8.3. Smaller bodies keep the order of their
+// samples (192 particles: 9.4 us, grouped 8.6): their float32 sums, and with them every rounding of a
+// position, stay those that finite differences over a few hundred particles were resolved with.
+constexpr int kGroupRuns = 8;
+constexpr int64_t kGroupParticles = 1024;
+
+BK_DEV bool group_lanes(int64_t n, int R) { return n >= kGroupParticles && R <= 1024; }
+
+BK_DEV Runs find_runs(bool valid, const int* b, bool group) {
     const int lane = threadIdx.x & 31;
     const int p0 = __shfl_up_sync(kWarp, b[0], 1), p1 = __shfl_up_sync(kWarp, b[1], 1),
               p2 = __shfl_up_sync(kWarp, b[2], 1);
     const bool before = __shfl_up_sync(kWarp, (int)valid, 1) != 0;
-    return __ballot_sync(kWarp, valid && (lane == 0 || !before || p0 != b[0] || p1 != b[1] || p2 != b[2]));
+    Runs r;
+    r.column = lane;
+    r.starts = __ballot_sync(kWarp, valid && (lane == 0 || !before || p0 != b[0] || p1 != b[1] || p2 != b[2]));
+    if (group && __popc(r.starts) >= kGroupRuns) {
+        // An invalid particle is a group of its own (its stored weights are zero).
+        const unsigned key = valid ? (unsigned)(b[0] << 20 | b[1] << 10 | b[2]) : 0x80000000u | (unsigned)lane;
+        const unsigned peers = __match_any_sync(kWarp, key);
+        const int rank = __popc(peers & ((1u << lane) - 1u)), first = __ffs(peers) - 1;
+        const int size = rank == 0 ? __popc(peers) : 0;
+        int sum = size;  // columns up to and including this lane's group, groups in the order of their first lanes
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(kWarp, sum, o);
+            if (lane >= o) sum += v;
+        }
+        r.column = __shfl_sync(kWarp, sum - size, first) + rank;
+        r.starts = __reduce_or_sync(kWarp, valid && rank == 0 ? 1u << r.column : 0u);
+    }
+    return r;
 }
 
 // Column one past the run before the next start. (A run may include columns of invalid particles,
 // whose stored weights are zero.)
 BK_DEV int run_end(unsigned later_starts) { return later_starts ? __ffs(later_starts) - 1 : 32; }
 
-// The 27 weights of this thread's particle into its lane's column of the record's node-major rows.
+// The stencil base of the run that starts at column s.
+BK_DEV void run_base(const Runs& r, int s, const int* b, int* base) {
+    const int lane = __ffs(__ballot_sync(kWarp, r.column == s)) - 1;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) base[a] = __shfl_sync(kWarp, b[a], lane);
+}
+
+// The 27 weights of this thread's particle into its column of the record's node-major rows.
 template <int kPitch>
-BK_DEV void put_weights(float (&w)[27][kPitch], bool valid, const Stencil& st) {
-    const int lane = threadIdx.x & 31;
+BK_DEV void put_weights(float (&w)[27][kPitch], int column, bool valid, const Stencil& st) {
 #pragma unroll
     for (int ox = 0; ox < 3; ++ox)
 #pragma unroll
         for (int oy = 0; oy < 3; ++oy) {
             const float wxy = valid ? st.w[0][ox] * st.w[1][oy] : 0.f;
 #pragma unroll
-            for (int oz = 0; oz < 3; ++oz) w[9 * ox + 3 * oy + oz][lane] = valid ? wxy * st.w[2][oz] : 0.f;
+            for (int oz = 0; oz < 3; ++oz) w[9 * ox + 3 * oy + oz][column] = valid ? wxy * st.w[2][oz] : 0.f;
         }
 }
 
@@ -99,24 +140,26 @@ struct MomentumRecord {
 };
 
 BK_DEV void scatter_momentum(MomentumRecord& rec, bool valid, const Stencil& st, float m, const float* q,
-                             const float* A, float4* __restrict__ nodes, int R) {
+                             const float* A, float4* __restrict__ nodes, int R, bool group) {
     const int lane = threadIdx.x & 31;
-    put_weights(rec.w, valid, st);
-    rec.val[lane][0] = make_float4(m, q[0], q[1], q[2]);
-    rec.val[lane][1] = make_float4(A[0], A[1], A[2], A[3]);
-    rec.val[lane][2] = make_float4(A[4], A[5], A[6], A[7]);
-    rec.a8[lane] = A[8];
+    const Runs runs = find_runs(valid, st.b, group);
+    put_weights(rec.w, runs.column, valid, st);
+    rec.val[runs.column][0] = make_float4(m, q[0], q[1], q[2]);
+    rec.val[runs.column][1] = make_float4(A[0], A[1], A[2], A[3]);
+    rec.val[runs.column][2] = make_float4(A[4], A[5], A[6], A[7]);
+    rec.a8[runs.column] = A[8];
     __syncwarp();
     int ox, oy, oz;
     node_offset(lane < 27 ? lane : 0, ox, oy, oz);
     const float fo[3] = {(float)ox, (float)oy, (float)oz};
     const float* wj = rec.w[lane < 27 ? lane : 0];
-    unsigned starts = run_starts(valid, st.b);
+    unsigned starts = runs.starts;
     while (starts) {
         const int s = __ffs(starts) - 1;
         starts &= starts - 1;
         const int e = run_end(starts);
-        const int base[3] = {__shfl_sync(kWarp, st.b[0], s), __shfl_sync(kWarp, st.b[1], s), __shfl_sync(kWarp, st.b[2], s)};
+        int base[3];
+        run_base(runs, s, st.b, base);
         if (lane < 27) {
             float2 mq0 = {0.f, 0.f}, q12 = {0.f, 0.f}, A01 = {0.f, 0.f}, A23 = {0.f, 0.f};
             float2 A45 = {0.f, 0.f}, A67 = {0.f, 0.f};
@@ -170,13 +213,14 @@ BK_DEV void dmma(double& d0, double& d1, double a, double b) {
 // Adds values val[0..kF) of the warp's particles to the node fields f[0..kF) (R^3 float64 each).
 template <int kF>
 BK_DEV void scatter_scalars(ScalarRecord<kF>& rec, bool valid, const Stencil& st, const double* val,
-                            double* const (&f)[kF], int R) {
+                            double* const (&f)[kF], int R, bool group) {
     static_assert(kF >= 1 && kF <= 4, "the values share one 8-column tile");
     const int lane = threadIdx.x & 31;
     const int row = lane >> 2, quad = lane & 3;  // fragment coordinates
-    put_weights(rec.w, valid, st);
+    const Runs runs = find_runs(valid, st.b, group);
+    put_weights(rec.w, runs.column, valid, st);
 #pragma unroll
-    for (int k = 0; k < kF; ++k) rec.val[k][lane] = valid ? val[k] : 0.0;
+    for (int k = 0; k < kF; ++k) rec.val[k][runs.column] = valid ? val[k] : 0.0;
     __syncwarp();
     // Accumulator fragment: row 8 t + row, columns 2 quad and 2 quad + 1 (fields; quads 0 and 1).
     int offset[4];
@@ -192,12 +236,13 @@ BK_DEV void scatter_scalars(ScalarRecord<kF>& rec, bool valid, const Stencil& st
     // (selects, not f[2 * quad]: a run-time index would copy the pointers to local memory)
     double* const f0 = kF > 2 && quad == 1 ? f[2] : f[0];
     double* const f1 = kF > 3 && quad == 1 ? f[3] : f[kF > 1 ? 1 : 0];
-    unsigned starts = run_starts(valid, st.b);
+    unsigned starts = runs.starts;
     while (starts) {
         const int s = __ffs(starts) - 1;
         starts &= starts - 1;
         const int e = run_end(starts);
-        const int base[3] = {__shfl_sync(kWarp, st.b[0], s), __shfl_sync(kWarp, st.b[1], s), __shfl_sync(kWarp, st.b[2], s)};
+        int base[3];
+        run_base(runs, s, st.b, base);
         double d[4][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
         for (int k0 = s; k0 < e; k0 += 4) {
             // Fragments: weight of node 8 t + row and value `row` of particle k0 + quad; particles past

@@ -347,7 +347,8 @@ __device__ __forceinline__ void surface_owners_run_body(Arg<Params, kRef> P, Arg
         if (!valid) set_flag(sim_flags, 1);
     }
     // the owners' nodes lie inside the particles' transport box: no box to widen
-    scatter_scalars<3>(sm[threadIdx.x >> 5], valid, st, rate, {g.f[4], g.f[5], g.f[6]}, P.R);
+    scatter_scalars<3>(sm[threadIdx.x >> 5], valid, st, rate, {g.f[4], g.f[5], g.f[6]}, P.R,
+                       group_lanes(P.n, P.R));
 }
 
 // Many owners take the run form (one thread each), few the warp form (one warp each).
@@ -403,7 +404,8 @@ __device__ __forceinline__ void transport_scatter_body(Arg<Params, kRef> P, Arg<
         val[3] = in.water[i];
     }
     widen_box(g.bounds, valid, st.b);
-    scatter_scalars<4>(sm[threadIdx.x >> 5], valid, st, val, {g.f[0], g.f[1], g.f[2], g.f[3]}, P.R);
+    scatter_scalars<4>(sm[threadIdx.x >> 5], valid, st, val, {g.f[0], g.f[1], g.f[2], g.f[3]}, P.R,
+                       group_lanes(P.n, P.R));
 }
 
 __global__ void __launch_bounds__(kThreads, 4) k_transport_scatter(Params P, BkState in, BkConstants cst, GridPtrs g,
@@ -782,7 +784,7 @@ __device__ __forceinline__ void p2g_body(Arg<Params, kRef> P, Arg<BkState, kRef>
 #pragma unroll
         for (int e = 0; e < 9; ++e) A[e] *= P.dx;
     }
-    scatter_momentum(sm[threadIdx.x >> 5], valid, st, mass, q, A, g.pm, P.R);
+    scatter_momentum(sm[threadIdx.x >> 5], valid, st, mass, q, A, g.pm, P.R, group_lanes(P.n, P.R));
 }
 
 template <bool kLoaf = false>
@@ -1084,7 +1086,8 @@ __device__ __forceinline__ void g2p_return_body(Arg<Params, kRef> P, Arg<BkState
             }
         }
         widen_box(g.bounds + 12, valid, st.b);
-        scatter_scalars<4>(sm[threadIdx.x >> 5], valid, st, val, {g.f[0], g.f[1], g.f[2], g.f[3]}, P.R);
+        scatter_scalars<4>(sm[threadIdx.x >> 5], valid, st, val, {g.f[0], g.f[1], g.f[2], g.f[3]}, P.R,
+                       group_lanes(P.n, P.R));
     }
 }
 
