@@ -440,8 +440,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_adj_g2p_return(AdjParams P, BkS
                 if (D.temperature_enabled) {
                     if (T >= D.knots[3]) gel = 1;
                     if (gel) Teff = D.knots[3];
-                    float fy = temperature_factor(Teff, D.knots, D.yield_factors);
-                    float fv = temperature_factor(Teff, D.knots, D.viscosity_factors);
+                    float fy = temperature_factor(Teff, D, D.yield_factors);
+                    float fv = temperature_factor(Teff, D, D.viscosity_factors);
                     ty = D.yield_stress * fy;
                     eta_factor = fv;
                     eta = eta * fv;
@@ -480,7 +480,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_adj_g2p_return(AdjParams P, BkS
                 float cg = 1.f, target = 1.f;
                 if (coupled) {
                     target = (float)(1.0 - (double)D.initial_porosity + (double)n_ret);
-                    cg = cbrt_near_one((double)detFn / ((double)target * ((double)pr.g[0] * pr.g[1] * pr.g[2])));
+                    cg = cbrt_near_one((double)detFn, (double)target * ((double)pr.g[0] * pr.g[1] * pr.g[2]));
 #pragma unroll
                     for (int k = 0; k < 3; ++k) gv[k] *= cg;
                     if (porosity_free) nret_b += por_b;  // porosity' = n_ret
@@ -1042,15 +1042,7 @@ AdjParams adj_params(const BkSubstepParams& p) {
     a.dx = p.spacing; a.dt = p.time_step;
     a.material = p.material;
     a.transport = p.transport;
-    const BkDingParams& d = p.ding;
-    a.ding.coupled_porosity = d.coupled_porosity; a.ding.temperature_enabled = d.temperature_enabled;
-    a.ding.mu = d.shear_modulus; a.ding.lam = d.lame_lambda; a.ding.yield_stress = d.yield_stress;
-    a.ding.initial_porosity = d.initial_porosity; a.ding.dt = d.time_step;
-    for (int k = 0; k < 4; ++k) {
-        a.ding.knots[k] = d.temperature_knots[k];
-        a.ding.yield_factors[k] = d.yield_factors[k];
-        a.ding.viscosity_factors[k] = d.viscosity_factors[k];
-    }
+    a.ding = ding_params_dev(p.ding);
     return a;
 }
 

@@ -30,6 +30,36 @@ BK_DEV float2 ffma2(float2 a, float2 b, float2 c) {
     return d;
 }
 
+// a / d for a divisor known before the launch, with rec = 1 / d rounded to nearest: the product a rec
+// corrected once by its exact remainder (Markstein, IBM J. Res. Dev. 34 (1990) 111), three dependent
+// operations instead of the general division's sequence with its range test. Equal to the IEEE
+// quotient (tests/test_uniform_division.py); an infinite product is returned uncorrected.
+BK_DEV float div_uniform(float a, float d, float rec) {
+    const float q = a * rec;
+    const float r = fmaf(-q, d, a);
+    return fabsf(q) <= 3.4028235e38f ? fmaf(r, rec, q) : q;
+}
+
+// 1 / sqrt(x) and 1 / x in float64 by Newton's iteration from the float32 value: relative error below
+// 1e-15, for the intermediate results of the singular value decomposition and the volume correction,
+// which are rounded to float32 afterwards. x positive; arguments outside the float32 range (reached
+// only by degenerate gradients) take the library's functions.
+BK_DEV double rsqrt_newton(double x) {
+    if (!(x > 1e-36 && x < 1e36)) return rsqrt(x);
+    double y = (double)rsqrtf((float)x);
+    const double h = 0.5 * x;
+    y = fma(y, fma(-h * y, y, 0.5), y);
+    y = fma(y, fma(-h * y, y, 0.5), y);
+    return y;
+}
+BK_DEV double reciprocal_newton(double x) {
+    if (!(fabs(x) > 1e-36 && fabs(x) < 1e36)) return 1.0 / x;
+    double y = (double)__fdividef(1.0f, (float)x);
+    y = fma(y, fma(-x, y, 1.0), y);
+    y = fma(y, fma(-x, y, 1.0), y);
+    return y;
+}
+
 // ------------------------------------------------------------- SoA access
 BK_DEV V3 load_v3(const float* __restrict__ p, int64_t i, int64_t pitch) {
     V3 r;
@@ -365,13 +395,13 @@ BK_DEV void svd3f(const M3& A, M3& U, float s[3], M3& V, float e[3]) {
     double vv[9], bb[9];
     {
         double c0[3] = {v[0], v[3], v[6]}, c1[3] = {v[1], v[4], v[7]};
-        double n0 = rsqrt(c0[0] * c0[0] + c0[1] * c0[1] + c0[2] * c0[2]);
+        double n0 = rsqrt_newton(c0[0] * c0[0] + c0[1] * c0[1] + c0[2] * c0[2]);
 #pragma unroll
         for (int i = 0; i < 3; ++i) c0[i] *= n0;
         double d01 = c0[0] * c1[0] + c0[1] * c1[1] + c0[2] * c1[2];
 #pragma unroll
         for (int i = 0; i < 3; ++i) c1[i] -= d01 * c0[i];
-        double n1 = rsqrt(c1[0] * c1[0] + c1[1] * c1[1] + c1[2] * c1[2]);
+        double n1 = rsqrt_newton(c1[0] * c1[0] + c1[1] * c1[1] + c1[2] * c1[2]);
 #pragma unroll
         for (int i = 0; i < 3; ++i) c1[i] *= n1;
 #pragma unroll
@@ -403,8 +433,10 @@ BK_DEV void svd3f(const M3& A, M3& U, float s[3], M3& V, float e[3]) {
         if (gamma * gamma <= 1e-30 * alpha * beta) continue;
         // tan of the rotation angle, t = 2 gamma sign(d) / (|d| + sqrt(d^2 + 4 gamma^2)), d = beta - alpha.
         double d = beta - alpha;
-        double t = 2.0 * gamma / (d >= 0.0 ? d + sqrt(d * d + 4.0 * gamma * gamma) : d - sqrt(d * d + 4.0 * gamma * gamma));
-        double c = rsqrt(1.0 + t * t);
+        const double h2 = d * d + 4.0 * gamma * gamma;
+        const double h = h2 * rsqrt_newton(h2);
+        double t = 2.0 * gamma * reciprocal_newton(d >= 0.0 ? d + h : d - h);
+        double c = rsqrt_newton(1.0 + t * t);
         double sn = c * t;
 #pragma unroll
         for (int r = 0; r < 3; ++r) {
@@ -421,7 +453,7 @@ BK_DEV void svd3f(const M3& A, M3& U, float s[3], M3& V, float e[3]) {
     for (int c = 0; c < 3; ++c) {
         double n2 = bb[c] * bb[c] + bb[3 + c] * bb[3 + c] + bb[6 + c] * bb[6 + c];
         degenerate |= !(n2 > 1e-30);
-        double inv = rsqrt(n2);
+        double inv = rsqrt_newton(n2);
         s[c] = (float)(n2 * inv);
 #pragma unroll
         for (int r = 0; r < 3; ++r) U.m[3 * r + c] = (float)(bb[3 * r + c] * inv);
@@ -457,11 +489,11 @@ struct Stencil {
     bool valid;
 };
 
-BK_DEV Stencil make_stencil(const V3& x, const float* origin, float dx, int R) {
+BK_DEV Stencil stencil_of(const float* g3, int R) {
     Stencil s;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        float g = (x.v[a] - origin[a]) / dx;
+        const float g = g3[a];
         s.b[a] = (int)floorf(g - 0.5f);
         s.l[a] = g - (float)s.b[a];
     }
@@ -473,6 +505,17 @@ BK_DEV Stencil make_stencil(const V3& x, const float* origin, float dx, int R) {
     return s;
 }
 
+BK_DEV Stencil make_stencil(const V3& x, const float* origin, float dx, int R) {
+    const float g[3] = {(x.v[0] - origin[0]) / dx, (x.v[1] - origin[1]) / dx, (x.v[2] - origin[2]) / dx};
+    return stencil_of(g, R);
+}
+// The same with rec_dx = 1 / dx rounded on the host.
+BK_DEV Stencil make_stencil(const V3& x, const float* origin, float dx, int R, float rec_dx) {
+    const float g[3] = {div_uniform(x.v[0] - origin[0], dx, rec_dx), div_uniform(x.v[1] - origin[1], dx, rec_dx),
+                        div_uniform(x.v[2] - origin[2], dx, rec_dx)};
+    return stencil_of(g, R);
+}
+
 BK_DEV int64_t node_index(int i, int j, int k, int R) { return ((int64_t)i * R + j) * R + k; }
 
 // flags may be NULL (a re-evaluation whose flags are not reported).
@@ -481,12 +524,42 @@ BK_DEV void set_flag(int32_t* flags, int index) {
 }
 
 // ------------------------------------------------------- ding.py:56-100
-BK_DEV float temperature_factor(float T, const float* knots, const float* factors) {
+struct DingParamsDev {
+    int coupled_porosity, temperature_enabled;
+    float mu, lam, yield_stress, initial_porosity, dt;
+    float knots[4], yield_factors[4], viscosity_factors[4];
+    float rec_2mu, rec_bulk, rec_knots[3];  // reciprocals of 2 mu, 2 mu + 3 lam and the knot distances
+};
+
+// From the C ABI's parameters (BkDingParams).
+template <class HostParams>
+inline DingParamsDev ding_params_dev(const HostParams& p) {
+    DingParamsDev d;
+    d.coupled_porosity = p.coupled_porosity;
+    d.temperature_enabled = p.temperature_enabled;
+    d.mu = p.shear_modulus;
+    d.lam = p.lame_lambda;
+    d.yield_stress = p.yield_stress;
+    d.initial_porosity = p.initial_porosity;
+    d.dt = p.time_step;
+    for (int k = 0; k < 4; ++k) {
+        d.knots[k] = p.temperature_knots[k];
+        d.yield_factors[k] = p.yield_factors[k];
+        d.viscosity_factors[k] = p.viscosity_factors[k];
+    }
+    d.rec_2mu = 1.0f / (2.0f * d.mu);
+    d.rec_bulk = 1.0f / (2.0f * d.mu + 3.0f * d.lam);
+    for (int k = 0; k < 3; ++k) d.rec_knots[k] = 1.0f / (d.knots[k + 1] - d.knots[k]);
+    return d;
+}
+
+BK_DEV float temperature_factor(float T, const DingParamsDev& P, const float* factors) {
+    const float* knots = P.knots;
     float f = factors[0];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         if (T >= knots[k]) {
-            float frac = fminf((T - knots[k]) / (knots[k + 1] - knots[k]), 1.0f);
+            float frac = fminf(div_uniform(T - knots[k], knots[k + 1] - knots[k], P.rec_knots[k]), 1.0f);
             f = (1.0f - frac) * factors[k] + frac * factors[k + 1];
         }
     }
@@ -529,8 +602,8 @@ BK_DEV float solve_overstress(float q2, float p2, float d, float h, float r0 = 0
 BK_DEV double pressure_coefficient64(double n) {
     double c = 0.0;
     if (n > 0.0) {
-        double lg = log(1.0 / n);
-        c = 9.0 / (4.0 * (lg * lg) * (3.5 * n + 1.0));
+        const double lg = log(n);
+        c = 2.25 * reciprocal_newton(lg * lg * (3.5 * n + 1.0));
     }
     return c;
 }
@@ -543,11 +616,12 @@ BK_DEV double overstress64(double q, double p, double d, double h, double* warm 
     if (!(q + p > 1.0)) r = 0.0;
     if (q + p > 1.0) {
         for (int it = 0; it < 48; ++it) {
-            double u = 1.0 + d * r, v = 1.0 + h * r;
-            double u2 = u * u, v2 = v * v;
-            double res = r + 1.0 - q / u2 - p / v2;
-            double der = 1.0 + 2.0 * d * q / (u2 * u) + 2.0 * h * p / (v2 * v);
-            r -= res / der;
+            // 1 / u and 1 / v from one reciprocal; the derivative's only steers the step
+            const double u = 1.0 + d * r, v = 1.0 + h * r;
+            const double uv = reciprocal_newton(u * v), iu = v * uv, iv = u * uv;
+            const double A = q * iu * iu, B = p * iv * iv;
+            const double res = r + 1.0 - A - B;
+            r -= res * reciprocal_newton(1.0 + 2.0 * (d * A * iu + h * B * iv));
             // From a warm start above the root a step can pass zero; restart from r = 0 (the
             // iterates from 0 increase monotonically and never get here).
             if (r < 0.0) { r = 0.0; continue; }
@@ -563,8 +637,7 @@ BK_DEV double porosity_prediction(double n, float q, float p, float d, float h, 
     double a = pressure_coefficient64(n);
     double r = overstress64((double)q, a * (double)p, (double)d, (double)h * a, warm);
     if (r == 0.0) return Vp - 1.0 + (double)n0;  // no overstress: exp(e (1 - 1/1)) = exp(0) = 1 exactly
-    double den = 1.0 + (double)h * a * r;
-    return Vp * exp((double)e * (1.0 - 1.0 / den)) - 1.0 + (double)n0;
+    return Vp * exp((double)e * (1.0 - reciprocal_newton(1.0 + (double)h * a * r))) - 1.0 + (double)n0;
 }
 
 // prediction(n) and its derivative in n. The overstress root r(n) is the reference's 48-step Newton
@@ -574,22 +647,22 @@ BK_DEV double porosity_prediction(double n, float q, float p, float d, float h, 
 BK_DEV double porosity_prediction_slope(double n, float qf, float pf, float df, float hf, float ef, double Vp,
                                         float n0, double& slope, double* warm = nullptr) {
     const double q = qf, p = pf, d = df, h = hf, e = ef;
-    double a = pressure_coefficient64(n);
-    double r = overstress64(q, a * p, d, h * a, warm);
-    double v = 1.0 + h * a * r;
-    double core = Vp * exp(e * (1.0 - 1.0 / v));
-    double da = 0.0;
+    double a = 0.0, da = 0.0;
     if (n > 0.0) {
-        double lg = log(1.0 / n);
-        da = a * (2.0 / (n * lg) - 3.5 / (3.5 * n + 1.0));
+        const double lg = log(n), m = 3.5 * n + 1.0;  // lg = -log(1 / n)
+        a = 2.25 * reciprocal_newton(lg * lg * m);
+        da = -a * (2.0 * m + 3.5 * n * lg) * reciprocal_newton(n * lg * m);
     }
+    double r = overstress64(q, a * p, d, h * a, warm);
+    const double u = 1.0 + d * r, v = 1.0 + h * a * r;
+    const double uv = reciprocal_newton(u * v), iu = v * uv, iv = u * uv;
+    double core = Vp * exp(e * (1.0 - iv));
     double dr = 0.0;
     if (q + a * p > 1.0) {
-        double u = 1.0 + d * r;
-        double Rr = 1.0 + 2.0 * d * q / (u * u * u) + 2.0 * h * a * a * p / (v * v * v);
-        dr = p * (1.0 - h * a * r) / (Rr * v * v * v) * da;
+        const double Rr = 1.0 + 2.0 * (d * q * iu * iu * iu + h * a * a * p * iv * iv * iv);
+        dr = p * (1.0 - h * a * r) * iv * iv * iv * reciprocal_newton(Rr) * da;
     }
-    slope = core * e * h * (da * r + a * dr) / (v * v);
+    slope = core * e * h * (da * r + a * dr) * iv * iv;
     return core - 1.0 + (double)n0;
 }
 
@@ -651,7 +724,7 @@ BK_DEV float solve_porosity(float q, float p, float d, float h, float e, double 
         if (g == 0.0) break;  // n is the root
         if (n < pred) lo = n; else hi = n;
         double dg = 1.0 - slope;
-        double next = n - g / dg;
+        double next = n - g * reciprocal_newton(dg);
         // A converged Newton step ends the solve before the bracket test: when the root sits on
         // the end of the bracket that n just became (g at the float64 rounding level, as when the
         // mean stress vanishes), the step falls on that end, and treating it as a bracket escape
@@ -667,72 +740,39 @@ BK_DEV float solve_porosity(float q, float p, float d, float h, float e, double 
     return (float)n;
 }
 
-struct DingOut {
-    M3 Fe, tau;
-    float residual;
-    float e[3];     // returned log principal strains before the isochoric correction (exponents of Fe)
-    bool yielded;   // q^2 + p^2 > 1: the overstress solve ran
+// Gas mode's end-state porosity (ding.py:181-197) with its consistency residual and the overstress root
+// it ended with. Out of line: particles that are certainly elastic (certain_elastic) never come here,
+// and the float64 solve would otherwise stand between the instructions that every particle runs (the
+// kernel's top stall was instruction fetch). Scalars by value: a reference to the kernel's parameters
+// would copy them to local memory.
+struct DingPorosity {
+    float ret_por, consistency, r;
 };
-
-// Ding return map (ding.py:103-137) given the SVD of the trial gradient (float32 factors) and its
-// principal log stretches log_s (svd3f).
-BK_DEV DingOut ding_return(float det_trial, const M3& Um, const float* log_s, const M3& Vm, float mu, float lam,
-                           float ty, float eta, float a, float dt, float r0 = 0.0f) {
-    const float* U = Um.m;
-    const float* V = Vm.m;
-    float eps[3] = {log_s[0], log_s[1], log_s[2]};
-    float tr = eps[0] + eps[1] + eps[2];
-    float ts[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) ts[k] = 2.0f * mu * eps[k] + lam * tr;
-    float mean = (ts[0] + ts[1] + ts[2]) / 3.0f;
-    float dev[3] = {ts[0] - mean, ts[1] - mean, ts[2] - mean};
-    float ty2 = ty * ty;
-    float q2 = 1.5f * (dev[0] * dev[0] + dev[1] * dev[1] + dev[2] * dev[2]) / ty2;
-    float p2 = a * mean * mean / ty2;
-    float df = 6.0f * mu * dt * ty * ty / eta;
-    float mf = 2.0f * a / 3.0f * (2.0f * mu + 3.0f * lam) * dt * ty * ty / eta;
-    float r = solve_overstress(q2, p2, df, mf, r0);
-    float cs[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) cs[k] = dev[k] / (1.0f + df * r) + mean / (1.0f + mf * r);
-    float cm = (cs[0] + cs[1] + cs[2]) / 3.0f;
-    float ex[3];
-    DingOut o;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        o.e[k] = (cs[k] - cm) / (2.0f * mu) + cm / (2.0f * mu + 3.0f * lam);
-        ex[k] = expf(o.e[k]);
-    }
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            o.Fe.m[3 * i + k] = (U[3 * i] * ex[0]) * V[3 * k] + (U[3 * i + 1] * ex[1]) * V[3 * k + 1]
-                              + (U[3 * i + 2] * ex[2]) * V[3 * k + 2];
-            o.tau.m[3 * i + k] = (U[3 * i] * cs[0]) * U[3 * k] + (U[3 * i + 1] * cs[1]) * U[3 * k + 1]
-                               + (U[3 * i + 2] * cs[2]) * U[3 * k + 2];
-        }
-    if (a == 0.0f) {
-        // pow(x, 1/3) of the reference; cube root of the same argument.
-        float scale = cbrtf(det_trial / det3(o.Fe));
-#pragma unroll
-        for (int e = 0; e < 9; ++e) o.Fe.m[e] *= scale;
-    }
-    o.residual = 0.0f;
-    o.yielded = q2 + p2 > 1.0f;
-    if (o.yielded) {
-        float u = 1.0f + df * r, w = 1.0f + mf * r;
-        o.residual = fabsf(r + 1.0f - q2 / (u * u) - p2 / (w * w));
-    }
+static __device__ __noinline__ DingPorosity ding_porosity(float q2, float p2, float df, float ms, float ex, float por,
+                                                          float n0) {
+    DingPorosity o;
+    double r_warm = 0.0;  // overstress root carried from one solve to the next
+    const double Vp = 1.0 - (double)n0 + (double)por;
+    bool elastic_exit;
+    o.ret_por = solve_porosity(q2, p2, df, ms, ex, Vp, n0, &r_warm, &elastic_exit);
+    // Certain elastic exit: prediction(ret_por) has r = 0 and returns Vp - 1 + n0 exactly.
+    const double pred = elastic_exit ? Vp - 1.0 + (double)n0
+                                     : porosity_prediction((double)o.ret_por, q2, p2, df, ms, ex, Vp, n0, &r_warm);
+    o.consistency = (float)fabs((double)o.ret_por - pred);
+    o.r = (float)r_warm;
     return o;
 }
 
-struct DingParamsDev {
-    int coupled_porosity, temperature_enabled;
-    float mu, lam, yield_stress, initial_porosity, dt;
-    float knots[4], yield_factors[4], viscosity_factors[4];
-};
+// Gas mode: true only where the elastic exit of the porosity solve (q + a(trial) p <= 1) is certain.
+// a(n) from the hardware logarithm is within 1e-5 of its value for n <= 0.9, and q + a p is tested
+// against 1 - 1e-4; other particles take the full branch, which decides exactly.
+BK_DEV bool certain_elastic(float dev2, float mean, float ty, double trial) {
+    const float n = (float)trial;
+    if (!(n >= 1.0e-30f && n <= 0.9f)) return false;
+    const float lg = __logf(n);
+    const float a = __fdividef(9.0f, 4.0f * (lg * lg) * (3.5f * n + 1.0f));
+    return dev2 + a * mean * mean <= (1.0f - 1.0e-4f) * (ty * ty);
+}
 
 struct DingParticleOut {
     M3 Fe, Fp, tau;
@@ -763,8 +803,8 @@ BK_DEV bool ding_prelude(const DingParamsDev& P, const M3& Fe_old, float por, in
     if (P.temperature_enabled) {
         if (reached) gel = 1;
         if (gel) Teff = P.knots[3];
-        ty = P.yield_stress * temperature_factor(Teff, P.knots, P.yield_factors);
-        eta = eta_base * temperature_factor(Teff, P.knots, P.viscosity_factors);
+        ty = P.yield_stress * temperature_factor(Teff, P, P.yield_factors);
+        eta = eta_base * temperature_factor(Teff, P, P.viscosity_factors);
     }
     M3 G;
 #pragma unroll
@@ -779,16 +819,27 @@ BK_DEV bool ding_prelude(const DingParamsDev& P, const M3& Fe_old, float por, in
     return true;
 }
 
-// Where ding_close reads the total gradient F' from: a matrix the caller holds (FInRegs), or the F'
-// this thread stored earlier in the same kernel (FStored), read back with plain loads only where
-// the close needs it, so that it is not held in registers through the return map.
+BK_DEV double det3_64(const M3& a) {
+    M3d d;
+#pragma unroll
+    for (int e = 0; e < 9; ++e) d.m[e] = (double)a.m[e];
+    return det3(d);
+}
+
+// Where ding_close takes the total gradient F' and its float64 determinant from: a matrix the caller
+// holds (FInRegs), or the F' this thread stored earlier in the same kernel (FStored), whose
+// determinant the caller formed while it held F' and whose entries are read back with plain loads
+// only where the close needs them, so that they are not held in registers through the return map.
 struct FInRegs {
     const M3& m;
     BK_DEV M3 get() const { return m; }
+    BK_DEV double det() const { return det3_64(m); }
 };
 struct FStored {
     const float* p;  // not the read-only path: the data were written during this kernel
     int64_t i, pitch;
+    double determinant;
+    BK_DEV double det() const { return determinant; }
     BK_DEV M3 get() const {
         M3 r;
 #pragma unroll
@@ -802,10 +853,11 @@ struct FStored {
 // (1 + d)^(1/3) = 1 + d/3 - d^2/9 + 5 d^3/81 - 10 d^4/243 + ...; for |d| < 2^-10 the omitted terms
 // are below 3e-17, so the rounded result is that of the float64 cube root unless the root lies
 // within ~2e-16 (relative) of a float32 rounding boundary. Elsewhere it calls cbrt.
-BK_DEV float cbrt_near_one(double v) {
-    const double d = v - 1.0;
+// The ratio comes as num / den.
+BK_DEV float cbrt_near_one(double num, double den) {
+    const double d = (num - den) * reciprocal_newton(den);
     if (fabs(d) < 0x1p-10) return (float)(1.0 + d * (1.0 / 3.0 + d * (-1.0 / 9.0 + d * (5.0 / 81.0 - d * (10.0 / 243.0)))));
-    return (float)cbrt(v);
+    return (float)cbrt(num / den);
 }
 
 // Volume correction (gas mode), plastic gradient and porosity update shared by the exact and the
@@ -814,14 +866,9 @@ template <class FSrc>
 BK_DEV void ding_close(const DingParamsDev& P, float por, const FSrc& F_src, float ret_por, M3 Fe, int32_t* flags,
                        DingParticleOut& out, bool need_fp) {
     const float n0 = P.initial_porosity;
-    const M3 F_tot = F_src.get();
     if (P.coupled_porosity) {
         double target = 1.0 - (double)n0 + (double)ret_por;
-        M3d Fd, Fed;
-#pragma unroll
-        for (int e = 0; e < 9; ++e) { Fd.m[e] = (double)F_tot.m[e]; Fed.m[e] = (double)Fe.m[e]; }
-        double vs = det3(Fd) / (target * det3(Fed));
-        float scale = cbrt_near_one(vs);  // pow(vs, 1/3) in the reference
+        float scale = cbrt_near_one(F_src.det(), target * det3_64(Fe));  // pow(ratio, 1/3) in the reference
 #pragma unroll
         for (int e = 0; e < 9; ++e) Fe.m[e] *= scale;
     }
@@ -829,9 +876,9 @@ BK_DEV void ding_close(const DingParamsDev& P, float por, const FSrc& F_src, flo
     float npor;
     if (P.coupled_porosity) {
         npor = ret_por;
-        if (need_fp) Fp = matmul(inverse3(Fe), F_tot);
+        if (need_fp) Fp = matmul(inverse3(Fe), F_src.get());
     } else {
-        Fp = matmul(inverse3(Fe), F_tot);
+        Fp = matmul(inverse3(Fe), F_src.get());
         npor = det3(Fp) - 1.0f + n0;
     }
     if (n0 == 0.0f && por == 0.0f) npor = 0.0f;
@@ -841,49 +888,87 @@ BK_DEV void ding_close(const DingParamsDev& P, float por, const FSrc& F_src, flo
     out.porosity = npor;
 }
 
-// The exact return of UpdateDing after the prelude (ding.py:181-221).
+// The exact return of UpdateDing after the prelude (ding.py:103-137, 181-221): principal stresses of the
+// trial state, the plastic branch where it is not certainly elastic (there u = w = 1 and the end-state
+// porosity is the trial's), Fe = U exp(e) V^T, tau = U c U^T, and the close.
 template <class FSrc>
 BK_DEV void ding_exact(const DingParamsDev& P, const DingPrelude& d, float por, const FSrc& F_tot, int32_t* flags,
                        DingParticleOut& out, bool need_fp) {
-    const float dt = P.dt, mu = P.mu, lam = P.lam, n0 = P.initial_porosity;
-    const float ty = d.ty, eta = d.eta;
-    float ret_por = por, consistency = 0.0f;
-    double r_warm = 0.0;  // overstress root carried from one solve to the next
-    if (P.coupled_porosity) {
-        const float* st = d.e;
-        float tr = st[0] + st[1] + st[2];
-        float ts[3];
+    const float mu = P.mu, lam = P.lam, n0 = P.initial_porosity;
+    const float third = 1.0f / 3.0f;
+    const float* eps = d.e;
+    const float tr = eps[0] + eps[1] + eps[2];
+    float ts[3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) ts[k] = 2.0f * mu * st[k] + lam * tr;
-        float mean = (ts[0] + ts[1] + ts[2]) / 3.0f;
-        float dev[3] = {ts[0] - mean, ts[1] - mean, ts[2] - mean};
-        float ty2 = ty * ty;
-        float qv = 1.5f * (dev[0] * dev[0] + dev[1] * dev[1] + dev[2] * dev[2]) / ty2;
-        float pv = mean * mean / ty2;
-        float df = 6.0f * mu * dt * ty * ty / eta;
-        float ms = 2.0f / 3.0f * (2.0f * mu + 3.0f * lam) * dt * ty * ty / eta;
-        float ex = 3.0f * mean / (2.0f * mu + 3.0f * lam);
-        double Vp = 1.0 - (double)n0 + (double)por;
-        bool elastic_exit;
-        ret_por = solve_porosity(qv, pv, df, ms, ex, Vp, n0, &r_warm, &elastic_exit);
-        // Certain elastic exit: prediction(ret_por) has r = 0 and returns Vp - 1 + n0 exactly.
-        double pred = elastic_exit ? Vp - 1.0 + (double)n0
-                                   : porosity_prediction((double)ret_por, qv, pv, df, ms, ex, Vp, n0, &r_warm);
-        consistency = (float)fabs((double)ret_por - pred);
-        if (consistency > 1.0e-6f || ret_por <= 0.0f || ret_por >= 1.0f) set_flag(flags, 1);
+    for (int k = 0; k < 3; ++k) ts[k] = 2.0f * mu * eps[k] + lam * tr;
+    const float mean = div_uniform(ts[0] + ts[1] + ts[2], 3.0f, third);
+    const float dev[3] = {ts[0] - mean, ts[1] - mean, ts[2] - mean};
+    const float dev2 = 1.5f * (dev[0] * dev[0] + dev[1] * dev[1] + dev[2] * dev[2]);
+    const double trial = 1.0 - (double)n0 + (double)por - 1.0 + (double)n0;
+    float cs[3], ret_por = por;
+    out.residual = 0.0f;
+    out.porosity_residual = 0.0f;
+    out.yielded = false;
+    bool von_mises = false;  // a(n) = 0
+    if (P.coupled_porosity && certain_elastic(dev2, mean, d.ty, trial)) {
+        ret_por = (float)trial;
+        out.porosity_residual = (float)fabs((double)ret_por - trial);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) cs[k] = dev[k] + mean;
+    } else {
+        const float ty = d.ty, eta = d.eta, dt = P.dt, ty2 = ty * ty;
+        const float q2 = dev2 / ty2;
+        const float df = 6.0f * mu * dt * ty * ty / eta;
+        float r_warm = 0.0f;
+        if (P.coupled_porosity) {
+            const float ms = 2.0f / 3.0f * (2.0f * mu + 3.0f * lam) * dt * ty * ty / eta;
+            const DingPorosity o = ding_porosity(q2, mean * mean / ty2, df, ms, 3.0f * mean / (2.0f * mu + 3.0f * lam), por, n0);
+            ret_por = o.ret_por;
+            out.porosity_residual = o.consistency;
+            r_warm = o.r;
+        }
+        const float a = porosity_coefficient(ret_por);
+        const float p2 = a * mean * mean / ty2;
+        const float mf = 2.0f * a / 3.0f * (2.0f * mu + 3.0f * lam) * dt * ty * ty / eta;
+        const float r = solve_overstress(q2, p2, df, mf, r_warm);
+        const float u = 1.0f + df * r, w = 1.0f + mf * r;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) cs[k] = dev[k] / u + mean / w;
+        von_mises = a == 0.0f;
+        out.yielded = q2 + p2 > 1.0f;
+        if (out.yielded) out.residual = fabsf(r + 1.0f - q2 / (u * u) - p2 / (w * w));
     }
-    DingOut r = ding_return(d.det_trial, d.U, d.e, d.V, mu, lam, ty, eta, porosity_coefficient(ret_por), dt,
-                            (float)r_warm);
-    ding_close(P, por, F_tot, ret_por, r.Fe, flags, out, need_fp);
-    out.tau = r.tau;
-    out.residual = r.residual;
-    out.porosity_residual = consistency;
-    out.yield_stress = ty;
-    out.viscosity = eta;
-    out.gelled = d.gel;
+    if (P.coupled_porosity && (out.porosity_residual > 1.0e-6f || ret_por <= 0.0f || ret_por >= 1.0f)) set_flag(flags, 1);
+    const float cm = div_uniform(cs[0] + cs[1] + cs[2], 3.0f, third);
+    const float cm_bulk = div_uniform(cm, 2.0f * mu + 3.0f * lam, P.rec_bulk);
+    float ex[3];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) out.e[k] = r.e[k];
-    out.yielded = r.yielded;
+    for (int k = 0; k < 3; ++k) {
+        out.e[k] = div_uniform(cs[k] - cm, 2.0f * mu, P.rec_2mu) + cm_bulk;
+        ex[k] = expf(out.e[k]);
+    }
+    const float* U = d.U.m;
+    const float* V = d.V.m;
+    M3 Fe;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            Fe.m[3 * i + k] = (U[3 * i] * ex[0]) * V[3 * k] + (U[3 * i + 1] * ex[1]) * V[3 * k + 1]
+                            + (U[3 * i + 2] * ex[2]) * V[3 * k + 2];
+            out.tau.m[3 * i + k] = (U[3 * i] * cs[0]) * U[3 * k] + (U[3 * i + 1] * cs[1]) * U[3 * k + 1]
+                                 + (U[3 * i + 2] * cs[2]) * U[3 * k + 2];
+        }
+    if (von_mises) {
+        // pow(x, 1/3) of the reference; cube root of the same argument.
+        float scale = cbrtf(d.det_trial / det3(Fe));
+#pragma unroll
+        for (int e = 0; e < 9; ++e) Fe.m[e] *= scale;
+    }
+    ding_close(P, por, F_tot, ret_por, Fe, flags, out, need_fp);
+    out.yield_stress = d.ty;
+    out.viscosity = d.eta;
+    out.gelled = d.gel;
 }
 
 // UpdateDing for one particle (ding.py:154-221). Returns false when the old porosity is

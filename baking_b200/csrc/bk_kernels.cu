@@ -513,20 +513,6 @@ __global__ void k_porosity_coefficient(int64_t n, const float* __restrict__ por,
     out[i] = porosity_coefficient(por[i]);
 }
 
-DingParamsDev to_dev(const BkDingParams& p) {
-    DingParamsDev d;
-    d.coupled_porosity = p.coupled_porosity;
-    d.temperature_enabled = p.temperature_enabled;
-    d.mu = p.shear_modulus; d.lam = p.lame_lambda; d.yield_stress = p.yield_stress;
-    d.initial_porosity = p.initial_porosity; d.dt = p.time_step;
-    for (int k = 0; k < 4; ++k) {
-        d.knots[k] = p.temperature_knots[k];
-        d.yield_factors[k] = p.yield_factors[k];
-        d.viscosity_factors[k] = p.viscosity_factors[k];
-    }
-    return d;
-}
-
 bool bad_counts(int64_t n, int64_t pitch) { return n < 0 || pitch < n || n > (int64_t)INT32_MAX * 64; }
 
 }  // namespace
@@ -606,7 +592,7 @@ int bk_update_ding(int64_t n, int64_t pitch, const float* Fe_old, const float* p
     k_update_ding<<<blocks_for(n, 128), 128, 0, S(stream)>>>(
         n, pitch, Fe_old, porosity_old, gelled_old, F_total, C_new, Fe_new, Fp_new, tau_new, residuals, porosity_new,
         temperature_out, gelled_new, yield_out, viscosity_out, viscosity_parameter, flags, porosity_residuals,
-        to_dev(*params), temperature_local);
+        ding_params_dev(*params), temperature_local);
     return check_launch("bk_update_ding");
 }
 

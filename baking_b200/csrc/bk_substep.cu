@@ -48,7 +48,7 @@ inline cudaStream_t S(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 struct Params {
     int64_t n, pitch;
     int R, bc;
-    float origin[3], dx, dt, gravity[3];
+    float origin[3], dx, rec_dx, dt, gravity[3];
     int material;
     DingParamsDev ding;
     int transport, gas, settling;
@@ -65,17 +65,9 @@ Params to_params(const BkSubstepParams& p) {
     Params k;
     k.n = p.n; k.pitch = p.pitch; k.R = p.resolution; k.bc = p.boundary_cells;
     for (int a = 0; a < 3; ++a) { k.origin[a] = p.origin[a]; k.gravity[a] = p.gravity[a]; }
-    k.dx = p.spacing; k.dt = p.time_step;
+    k.dx = p.spacing; k.rec_dx = 1.0f / p.spacing; k.dt = p.time_step;
     k.material = p.material;
-    const BkDingParams& d = p.ding;
-    k.ding.coupled_porosity = d.coupled_porosity; k.ding.temperature_enabled = d.temperature_enabled;
-    k.ding.mu = d.shear_modulus; k.ding.lam = d.lame_lambda; k.ding.yield_stress = d.yield_stress;
-    k.ding.initial_porosity = d.initial_porosity; k.ding.dt = d.time_step;
-    for (int i = 0; i < 4; ++i) {
-        k.ding.knots[i] = d.temperature_knots[i];
-        k.ding.yield_factors[i] = d.yield_factors[i];
-        k.ding.viscosity_factors[i] = d.viscosity_factors[i];
-    }
+    k.ding = ding_params_dev(p.ding);
     k.transport = p.transport; k.gas = p.gas; k.settling = p.settling;
     k.oven = p.scalar.oven_temperature; k.tray = p.scalar.tray_temperature;
     k.tray_transfer = p.scalar.tray_transfer; k.surface_loss = p.scalar.surface_loss;
@@ -310,7 +302,7 @@ __device__ __forceinline__ void surface_owners_warp_body(Arg<Params, kRef> P, Ar
     double rate[3];
     owner_rates(P, in, cst, p, exposed, contact, rate);
     if (lane == 0) owner_store(sf, o, p, rate);
-    Stencil st = make_stencil(load_v3(in.x, p, P.pitch), P.origin, P.dx, P.R);
+    Stencil st = make_stencil(load_v3(in.x, p, P.pitch), P.origin, P.dx, P.R, P.rec_dx);
     if (!st.valid) {
         if (lane == 0) set_flag(sim_flags, 1);
         return;
@@ -342,7 +334,7 @@ __device__ __forceinline__ void surface_owners_run_body(Arg<Params, kRef> P, Arg
         owner_areas(sf, o, exposed, contact);
         owner_rates(P, in, cst, p, exposed, contact, rate);
         owner_store(sf, o, p, rate);
-        st = make_stencil(load_v3(in.x, p, P.pitch), P.origin, P.dx, P.R);
+        st = make_stencil(load_v3(in.x, p, P.pitch), P.origin, P.dx, P.R, P.rec_dx);
         valid = st.valid;
         if (!valid) set_flag(sim_flags, 1);
     }
@@ -392,7 +384,7 @@ __device__ __forceinline__ void transport_scatter_body(Arg<Params, kRef> P, Arg<
     st.b[0] = st.b[1] = st.b[2] = 0;
     double val[4] = {0.0, 0.0, 0.0, 0.0};
     if (i < P.n) {
-        st = make_stencil(load_v3(in.x, i, pitch), P.origin, P.dx, P.R);
+        st = make_stencil(load_v3(in.x, i, pitch), P.origin, P.dx, P.R, P.rec_dx);
         valid = st.valid;
         if (!valid) set_flag(sim_flags, 1);
     }
@@ -673,7 +665,7 @@ __device__ __forceinline__ void p2g_body(Arg<Params, kRef> P, Arg<BkState, kRef>
     Stencil st;
     st.b[0] = st.b[1] = st.b[2] = 0;
     if (i < P.n) {
-        st = make_stencil(load_v3(in.x, i, pitch), P.origin, P.dx, P.R);
+        st = make_stencil(load_v3(in.x, i, pitch), P.origin, P.dx, P.R, P.rec_dx);
         valid = st.valid;
         if (!valid) set_flag(flags.simulation, 1);
     }
@@ -813,7 +805,7 @@ __device__ __forceinline__ bool g2p_gather(const Params& P, const BkState& in, c
                                            const BkFlags& flags, int64_t i, M3& Fn, M3& Cn) {
     const int64_t pitch = P.pitch;
     V3 xi = load_v3(in.x, i, pitch);
-    Stencil st = make_stencil(xi, P.origin, P.dx, P.R);
+    Stencil st = make_stencil(xi, P.origin, P.dx, P.R, P.rec_dx);
     if (!st.valid) { set_flag(flags.simulation, 1); return false; }
     float nv[3] = {0.f, 0.f, 0.f}, mo[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     const float4* vbase = g.v + node_index(st.b[0], st.b[1], st.b[2], P.R);
@@ -1007,6 +999,12 @@ __device__ bool ding_surrogate(const DingParamsDev& D, const DingPrelude& d, flo
     return true;
 }
 
+// Bound by instruction issue and fetch (1M elastic particles: 3,090 instructions a warp at 67% issue,
+// the top stall no_instruction), so it is the instructions that every particle runs which count:
+// divisions by launch constants are corrected products (div_uniform), an elastic particle is certified
+// without the exact invariants, the plastic branch's float64 solve stands out of line, det F' is
+// formed while F' is in registers, and the float64 special functions of the decomposition and the
+// solves are Newton steps from float32 seeds. 1M elastic loaf 142 -> 120.5 us, 4M yielding 1037 -> 903.
 // 8 blocks of 128 threads per SM (64 registers): the return map's dependent float64 chains are
 // latency bound, so resident warps outweigh the spilled registers (measured at 3 to 12 blocks per
 // SM: 8 is fastest for both elastic and yielding particles). With `sg.samples` set (harvest),
@@ -1018,6 +1016,7 @@ __device__ __forceinline__ void g2p_return_particle(const Params& P, const BkSta
     if (!g2p_gather(P, in, out, g, flags, i, Fn, Cn)) return;
     if (P.material != 1) return;
     const int64_t pitch = P.pitch;
+    const double det_F = P.ding.coupled_porosity ? det3_64(Fn) : 0.0;
     float T = P.transport ? (float)out.temperature[i] : in.material_temperature[i];
     const float por = in.porosity[i];
     DingPrelude d;
@@ -1025,7 +1024,7 @@ __device__ __forceinline__ void g2p_return_particle(const Params& P, const BkSta
                       flags.ding, d))
         return;
     DingParticleOut o;
-    ding_exact(P.ding, d, por, FStored{out.F, i, pitch}, flags.ding, o, diag.plastic_gradients != nullptr);
+    ding_exact(P.ding, d, por, FStored{out.F, i, pitch, det_F}, flags.ding, o, diag.plastic_gradients != nullptr);
     ding_store(P, out, diag, i, T, o);
     if (sg.samples && o.yielded && i % sg.sample_stride == sg.sample_offset) {
         int slot = atomicAdd(sg.sample_count, 1);
@@ -1033,7 +1032,7 @@ __device__ __forceinline__ void g2p_return_particle(const Params& P, const BkSta
             int perm[3];
             order3(d.e, perm);
             float f[7];
-            surrogate_features(P, out, cst, i, d, por, det3(FStored{out.F, i, pitch}.get()), perm, f);
+            surrogate_features(P, out, cst, i, d, por, det3(FStored{out.F, i, pitch, 0.0}.get()), perm, f);
             float* row = sg.samples + (int64_t)slot * 12;
 #pragma unroll
             for (int k = 0; k < 7; ++k) row[k] = f[k];
@@ -1055,6 +1054,17 @@ __device__ __forceinline__ void g2p_return_body(Arg<Params, kRef> P, Arg<BkState
                                                 Slot sl) {
     extern __shared__ __align__(16) unsigned char g2p_smem[];
     const int64_t i = sl.block * (int64_t)blockDim.x + threadIdx.x;
+    {
+        // F and Fe planes by lane, then the scalars' lines
+        const int lane = threadIdx.x & 31;
+        const int64_t w0 = i - lane;
+        if (w0 < P.n) {
+            if (lane < (P.material == 1 ? 18 : 9))
+                prefetch_l2((lane < 9 ? in.F + lane * P.pitch : in.Fe + (lane - 9) * P.pitch) + w0);
+            if (lane == 18 && P.material == 1) prefetch_l2(in.porosity + w0);
+            if (lane == 19 && P.material == 1) prefetch_l2(in.gelled + w0);
+        }
+    }
     if (sl.block == 0 && threadIdx.x < 6) {
         // This substep's box becomes the box the next substep clears; the active box restarts empty.
         g.bounds[6 + threadIdx.x] = g.bounds[threadIdx.x];
@@ -1075,11 +1085,11 @@ __device__ __forceinline__ void g2p_return_body(Arg<Params, kRef> P, Arg<BkState
         if (i < P.n) {
             const float* xs = out.x;
             const V3 x{{xs[i], xs[pitch + i], xs[2 * pitch + i]}};
-            st = make_stencil(x, P.origin, P.dx, P.R);
+            st = make_stencil(x, P.origin, P.dx, P.R, P.rec_dx);
             valid = st.valid;
             if (valid) {
                 const double cap = cst.capacity[i];
-                val[0] = (double)cst.volume[i] * (double)det3(FStored{out.F, i, pitch}.get());
+                val[0] = (double)cst.volume[i] * (double)det3(FStored{out.F, i, pitch, 0.0}.get());
                 val[1] = cap;
                 val[2] = cap * out.temperature[i];
                 val[3] = out.water[i];
@@ -1235,8 +1245,8 @@ __global__ void k_materialize(Params P, BkState s, BkConstants cst, float* Fp, f
     float ty = D.yield_stress, eta = __ldg(cst.viscosity_parameter);
     if (D.temperature_enabled) {
         float Teff = s.gelled[i] ? D.knots[3] : T;
-        ty = D.yield_stress * temperature_factor(Teff, D.knots, D.yield_factors);
-        eta = eta * temperature_factor(Teff, D.knots, D.viscosity_factors);
+        ty = D.yield_stress * temperature_factor(Teff, D, D.yield_factors);
+        eta = eta * temperature_factor(Teff, D, D.viscosity_factors);
     }
     if (yield) yield[i] = ty;
     if (visc) visc[i] = eta;
