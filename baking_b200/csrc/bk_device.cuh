@@ -684,7 +684,7 @@ static __device__ __noinline__ float solve_porosity_bisection(float q, float p, 
 // bisection steps: a step that leaves the current bracket becomes a bisection step, so the
 // iteration cannot escape the bracket and converges in a few evaluations. When the bracket's
 // lower end is not below the root (g(0+) >= 0) the reference's bisection runs unchanged. The root
-// is resolved to ~1e-14 relative, far below the float32 rounding of the returned porosity.
+// is resolved to ~1e-13 relative, far below the float32 rounding of the returned porosity.
 // Each evaluation's overstress root starts from the previous one (`warm`, which also returns the
 // last root to the caller); the roots are the reference's to its |residual| < 1e-12 test.
 //
@@ -694,11 +694,17 @@ static __device__ __noinline__ float solve_porosity_bisection(float q, float p, 
 // trial and at its float32 rounding (which moves ln n by at most 2^-24). `elastic_exit` (may be
 // NULL) reports that certain case; there prediction(float(trial)) has no overstress and equals
 // trial, so the caller can skip that evaluation. Every other case takes the float64 test.
+//
+// A Newton step below 1e-7 n^2 (or 1e-14 n) ends the solve without another evaluation: the error left
+// is of the order of its square over n (a(n) varies with ln n). `consistency` (may be NULL) then returns |float(n) - prediction(float(n))| from the
+// root and the slope there (the terms left out are of the order of ulp^2), or -1 where the caller has
+// to evaluate it.
 BK_DEV float solve_porosity(float q, float p, float d, float h, float e, double Vp, float n0,
-                            double* warm = nullptr, bool* elastic_exit = nullptr) {
+                            double* warm = nullptr, bool* elastic_exit = nullptr, double* consistency = nullptr) {
     double r_local = 0.0;
     if (!warm) warm = &r_local;
     if (elastic_exit) *elastic_exit = false;
+    if (consistency) *consistency = -1.0;
     double trial = Vp - 1.0 + (double)n0;
     if (trial > 0.0 && trial < 1.0) {
         const float nf = (float)trial;
@@ -721,7 +727,10 @@ BK_DEV float solve_porosity(float q, float p, float d, float h, float e, double 
         double slope;
         double pred = porosity_prediction_slope(n, q, p, d, h, e, Vp, n0, slope, warm);
         double g = n - pred;
-        if (g == 0.0) break;  // n is the root
+        if (g == 0.0) {  // n is the root
+            if (consistency) *consistency = fabs(((double)(float)n - n) * (1.0 - slope));
+            break;
+        }
         if (n < pred) lo = n; else hi = n;
         double dg = 1.0 - slope;
         double next = n - g * reciprocal_newton(dg);
@@ -729,8 +738,9 @@ BK_DEV float solve_porosity(float q, float p, float d, float h, float e, double 
         // the end of the bracket that n just became (g at the float64 rounding level, as when the
         // mean stress vanishes), the step falls on that end, and treating it as a bracket escape
         // would bisect all the way back to it.
-        if (fabs(next - n) <= 1e-14 * fabs(n)) {
+        if (fabs(next - n) <= fmax(1e-14 * fabs(n), 1e-7 * n * n)) {
             if (next > lo && next < hi) n = next;
+            if (consistency) *consistency = fabs(((double)(float)n - n) * dg);
             break;
         }
         if (!(next > lo && next < hi)) next = 0.5 * (lo + hi);
@@ -754,11 +764,15 @@ static __device__ __noinline__ DingPorosity ding_porosity(float q2, float p2, fl
     double r_warm = 0.0;  // overstress root carried from one solve to the next
     const double Vp = 1.0 - (double)n0 + (double)por;
     bool elastic_exit;
-    o.ret_por = solve_porosity(q2, p2, df, ms, ex, Vp, n0, &r_warm, &elastic_exit);
-    // Certain elastic exit: prediction(ret_por) has r = 0 and returns Vp - 1 + n0 exactly.
-    const double pred = elastic_exit ? Vp - 1.0 + (double)n0
-                                     : porosity_prediction((double)o.ret_por, q2, p2, df, ms, ex, Vp, n0, &r_warm);
-    o.consistency = (float)fabs((double)o.ret_por - pred);
+    double consistency;
+    o.ret_por = solve_porosity(q2, p2, df, ms, ex, Vp, n0, &r_warm, &elastic_exit, &consistency);
+    if (consistency < 0.0) {
+        // Certain elastic exit: prediction(ret_por) has r = 0 and returns Vp - 1 + n0 exactly.
+        const double pred = elastic_exit ? Vp - 1.0 + (double)n0
+                                         : porosity_prediction((double)o.ret_por, q2, p2, df, ms, ex, Vp, n0, &r_warm);
+        consistency = fabs((double)o.ret_por - pred);
+    }
+    o.consistency = (float)consistency;
     o.r = (float)r_warm;
     return o;
 }

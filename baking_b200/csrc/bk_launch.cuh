@@ -1,0 +1,47 @@
+// Programmatic dependent launch between the kernels of a substep and of its reverse: each is launched
+// with programmatic stream serialisation (launch_chained), so the launch of the next kernel and the
+// placement of its blocks overlap the tail of the one before it. Every such kernel first waits until
+// the kernel before it in the stream has completed and its memory is visible (which makes the chain
+// transitive), then lets the next kernel launch; its blocks only take SM slots left free by blocks
+// already running. A kernel without a programmatic predecessor returns from the wait at once.
+#pragma once
+
+#include <cstdio>
+#include <utility>
+
+#include "baking_b200.h"
+#include "bk_common.h"
+
+namespace bk {
+
+__device__ __forceinline__ void pdl_enter() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// The status of a launch_chained call, as check_launch reports a launch's.
+inline int check_chained(cudaError_t e, const char* name) {
+    if (e == cudaSuccess) return check_launch(name);
+    cudaGetLastError();
+    char msg[256];
+    snprintf(msg, sizeof msg, "%s: %s", name, cudaGetErrorString(e));
+    return fail(BK_ERR_LAUNCH, msg);
+}
+
+template <class... KArgs, class... Args>
+cudaError_t launch_chained(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
+                           Args&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+}  // namespace bk

@@ -25,6 +25,70 @@ namespace bk {
 
 constexpr unsigned kWarp = 0xffffffffu;
 
+// ------------------------------------------------------------- node gathers
+// sum_j w_j v_j and the moments sum_j w_j v_j o_jc over the stencil's nodes, with the offsets o_j in
+// {0, 1, 2} known at compile time: what G2P forms v and C of (C_rc = 4/dx (M_rc - l_c S_r)).
+BK_DEV void gather_velocity(const Stencil& st, const float4* __restrict__ node_v, int R32, float* nv, float* mo) {
+#pragma unroll
+    for (int r = 0; r < 3; ++r) nv[r] = 0.f;
+#pragma unroll
+    for (int e = 0; e < 9; ++e) mo[e] = 0.f;
+    const float4* vbase = node_v + node_index(st.b[0], st.b[1], st.b[2], R32);
+    const int64_t R = R32;
+#pragma unroll
+    for (int ox = 0; ox < 3; ++ox)
+#pragma unroll
+        for (int oy = 0; oy < 3; ++oy) {
+            const float wxy = st.w[0][ox] * st.w[1][oy];
+#pragma unroll
+            for (int oz = 0; oz < 3; ++oz) {
+                float w = wxy * st.w[2][oz];
+                float4 u = __ldg(vbase + (ox * R + oy) * R + oz);
+                float wu[3] = {w * u.x, w * u.y, w * u.z};
+#pragma unroll
+                for (int r = 0; r < 3; ++r) {
+                    nv[r] += wu[r];
+                    if (ox) mo[3 * r + 0] += (float)ox * wu[r];
+                    if (oy) mo[3 * r + 1] += (float)oy * wu[r];
+                    if (oz) mo[3 * r + 2] += (float)oz * wu[r];
+                }
+            }
+        }
+}
+
+// sum_j w_j (dT, dW/W)_j of the diffused node fields in float64, axis by axis (two multiply-adds a
+// node instead of a weight product, its conversion and two multiply-adds).
+BK_DEV void gather_scalars(const Stencil& st, const double2* __restrict__ dTr, int R32, double& dT, double& ratio) {
+    const double2* nodes = dTr + node_index(st.b[0], st.b[1], st.b[2], R32);
+    const int64_t R = R32;
+    dT = ratio = 0.0;
+#pragma unroll
+    for (int ox = 0; ox < 3; ++ox) {
+        double tx = 0.0, rx = 0.0;
+#pragma unroll
+        for (int oy = 0; oy < 3; ++oy) {
+            double ty = 0.0, ry = 0.0;
+#pragma unroll
+            for (int oz = 0; oz < 3; ++oz) {
+                const double2 d = __ldg(nodes + (ox * R + oy) * R + oz);
+                ty = fma((double)st.w[2][oz], d.x, ty);
+                ry = fma((double)st.w[2][oz], d.y, ry);
+            }
+            tx = fma((double)st.w[1][oy], ty, tx);
+            rx = fma((double)st.w[1][oy], ry, rx);
+        }
+        dT = fma((double)st.w[0][ox], tx, dT);
+        ratio = fma((double)st.w[0][ox], rx, ratio);
+    }
+}
+
+// Derivative of the quadratic weight of offset o by l (transfer.py:4-13).
+BK_DEV float qweight_grad(float l, int o) {
+    if (o == 0) return -(1.5f - l);
+    if (o == 1) return -2.f * (l - 1.f);
+    return l - 0.5f;
+}
+
 // Stencil node j in 0..26 -> offsets (j / 9, (j / 3) % 3, j % 3), the reference's loop order.
 BK_DEV void node_offset(int j, int& ox, int& oy, int& oz) {
     ox = j / 9;
@@ -47,7 +111,7 @@ struct Runs {
 // samples (192 particles: 9.4 us, grouped 8.6): their float32 sums, and with them every rounding of a
 // position, stay those that finite differences over a few hundred particles were resolved with.
 constexpr int kGroupRuns = 8;
-constexpr int64_t kGroupParticles = 1024;
+constexpr int64_t kGroupParticles = 256;
 
 BK_DEV bool group_lanes(int64_t n, int R) { return n >= kGroupParticles && R <= 1024; }
 
@@ -80,13 +144,6 @@ BK_DEV Runs find_runs(bool valid, const int* b, bool group) {
 // Column one past the run before the next start. (A run may include columns of invalid particles,
 // whose stored weights are zero.)
 BK_DEV int run_end(unsigned later_starts) { return later_starts ? __ffs(later_starts) - 1 : 32; }
-
-// The stencil base of the run that starts at column s.
-BK_DEV void run_base(const Runs& r, int s, const int* b, int* base) {
-    const int lane = __ffs(__ballot_sync(kWarp, r.column == s)) - 1;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) base[a] = __shfl_sync(kWarp, b[a], lane);
-}
 
 // The 27 weights of this thread's particle into its column of the record's node-major rows.
 template <int kPitch>
@@ -135,10 +192,12 @@ BK_DEV void widen_box(int* bounds, bool valid, const int* b) {
 // particle's column (conflict-free) and the values as 128-bit broadcasts.
 struct MomentumRecord {
     float4 val[32][3];  // {m q0 q1 q2} {A0 A1 A2 A3} {A4 A5 A6 A7}
+    int64_t corner[32];  // the stencil's first node (a run reads its start's: one broadcast, no shuffles)
     float a8[32];
     float w[27][33];
 };
 
+// (The adjoint of G2P has the same form with m = 0.)
 BK_DEV void scatter_momentum(MomentumRecord& rec, bool valid, const Stencil& st, float m, const float* q,
                              const float* A, float4* __restrict__ nodes, int R, bool group) {
     const int lane = threadIdx.x & 31;
@@ -148,18 +207,18 @@ BK_DEV void scatter_momentum(MomentumRecord& rec, bool valid, const Stencil& st,
     rec.val[runs.column][1] = make_float4(A[0], A[1], A[2], A[3]);
     rec.val[runs.column][2] = make_float4(A[4], A[5], A[6], A[7]);
     rec.a8[runs.column] = A[8];
+    rec.corner[runs.column] = node_index(st.b[0], st.b[1], st.b[2], R);
     __syncwarp();
     int ox, oy, oz;
     node_offset(lane < 27 ? lane : 0, ox, oy, oz);
     const float fo[3] = {(float)ox, (float)oy, (float)oz};
     const float* wj = rec.w[lane < 27 ? lane : 0];
+    float4* const mine = nodes + ((int64_t)ox * R + oy) * R + oz;
     unsigned starts = runs.starts;
     while (starts) {
         const int s = __ffs(starts) - 1;
         starts &= starts - 1;
         const int e = run_end(starts);
-        int base[3];
-        run_base(runs, s, st.b, base);
         if (lane < 27) {
             float2 mq0 = {0.f, 0.f}, q12 = {0.f, 0.f}, A01 = {0.f, 0.f}, A23 = {0.f, 0.f};
             float2 A45 = {0.f, 0.f}, A67 = {0.f, 0.f};
@@ -183,7 +242,7 @@ BK_DEV void scatter_momentum(MomentumRecord& rec, bool valid, const Stencil& st,
 #pragma unroll
             for (int r = 0; r < 3; ++r)
                 ap[r] = aq[r] + (aA[3 * r] * fo[0] + aA[3 * r + 1] * fo[1] + aA[3 * r + 2] * fo[2]);
-            atomicAdd(nodes + node_index(base[0] + ox, base[1] + oy, base[2] + oz, R), make_float4(ap[0], ap[1], ap[2], mq0.x));
+            atomicAdd(mine + rec.corner[s], make_float4(ap[0], ap[1], ap[2], mq0.x));
         }
     }
 }
@@ -201,6 +260,7 @@ BK_DEV void scatter_momentum(MomentumRecord& rec, bool valid, const Stencil& st,
 template <int kF>
 struct ScalarRecord {
     double val[kF][36];
+    int64_t corner[32];  // the stencil's first node
     float w[27][36];
 };
 
@@ -210,8 +270,9 @@ BK_DEV void dmma(double& d0, double& d1, double a, double b) {
         : "d"(a), "d"(b));
 }
 
-// Adds values val[0..kF) of the warp's particles to the node fields f[0..kF) (R^3 float64 each).
-template <int kF>
+// Adds values val[0..kF) of the warp's particles to the node fields f[0..kF) (R^3 float64 each, kStride
+// apart: 2 for the halves of a double2 field).
+template <int kF, int kStride = 1>
 BK_DEV void scatter_scalars(ScalarRecord<kF>& rec, bool valid, const Stencil& st, const double* val,
                             double* const (&f)[kF], int R, bool group) {
     static_assert(kF >= 1 && kF <= 4, "the values share one 8-column tile");
@@ -221,6 +282,7 @@ BK_DEV void scatter_scalars(ScalarRecord<kF>& rec, bool valid, const Stencil& st
     put_weights(rec.w, runs.column, valid, st);
 #pragma unroll
     for (int k = 0; k < kF; ++k) rec.val[k][runs.column] = valid ? val[k] : 0.0;
+    rec.corner[runs.column] = node_index(st.b[0], st.b[1], st.b[2], R);
     __syncwarp();
     // Accumulator fragment: row 8 t + row, columns 2 quad and 2 quad + 1 (fields; quads 0 and 1).
     int offset[4];
@@ -241,8 +303,6 @@ BK_DEV void scatter_scalars(ScalarRecord<kF>& rec, bool valid, const Stencil& st
         const int s = __ffs(starts) - 1;
         starts &= starts - 1;
         const int e = run_end(starts);
-        int base[3];
-        run_base(runs, s, st.b, base);
         double d[4][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
         for (int k0 = s; k0 < e; k0 += 4) {
             // Fragments: weight of node 8 t + row and value `row` of particle k0 + quad; particles past
@@ -258,12 +318,12 @@ BK_DEV void scatter_scalars(ScalarRecord<kF>& rec, bool valid, const Stencil& st
                 dmma(d[t][0], d[t][1], (double)w, b);
             }
         }
-        const int64_t corner = node_index(base[0], base[1], base[2], R);
+        const int64_t corner = rec.corner[s];
 #pragma unroll
         for (int t = 0; t < 4; ++t)
             if (node[t]) {
-                if (2 * quad < kF) atomicAdd(f0 + corner + offset[t], d[t][0]);
-                if (2 * quad + 1 < kF) atomicAdd(f1 + corner + offset[t], d[t][1]);
+                if (2 * quad < kF) atomicAdd(f0 + kStride * (corner + offset[t]), d[t][0]);
+                if (2 * quad + 1 < kF) atomicAdd(f1 + kStride * (corner + offset[t]), d[t][1]);
             }
     }
 }

@@ -36,7 +36,7 @@ import torch
 
 from .. import _lib, arrays
 from .materials.ding import DingMaterial
-from .substep import PHASE_MECHANICS, PHASE_TRANSPORT, BkConstants, BkSurface, state_struct
+from .substep import PHASE_MECHANICS, PHASE_TRANSPORT, BkConstants, BkState, BkSurface, state_struct
 
 P = C.c_void_p
 
@@ -216,10 +216,10 @@ class _Runner:
         if inputs.get("young_modulus") is not None:
             self._set_young_modulus(inputs["young_modulus"].detach().reshape(()).item())
         self.checkpoints = [self._snapshot(state)]
-        for k in range(self.steps):
-            sim._substep(check=False)
-            if (k + 1) % self.every == 0 and k + 1 < self.steps:
+        for first in range(0, self.steps, self.every):
+            if first:
                 self.checkpoints.append(self._snapshot(sim._current))
+            sim._unchecked_substeps(min(self.every, self.steps - first))
         messages = sim._device_flag_messages()
         flags = sim.error_flags.tolist()
         if flags[0]:
@@ -330,20 +330,22 @@ class _Runner:
             # P2G of a transport substep uses T', dry + W' and the water-stressed stress.
             cst_mech = BkConstants.from_buffer_copy(cst)
             cst_mech.mass = _p(tb["mass"])
+        prepared = eng.prepare(False)
+        structs = [state_struct(w, self.is_ding, self.transport, self.gas) for w in work]
         for seg in range(len(self.checkpoints) - 1, -1, -1):
             first = seg * self.every
             length = min(self.every, self.steps - first)
             _copy_state(work[0], self.checkpoints[seg], self.is_ding, self.transport, self.gas)
             for t in range(length):
-                self._run(work[t], work[t + 1], phases, grids[t][0], surface)
+                self._run(work[t], work[t + 1], phases, grids[t][0], surface, prepared)
             for t in range(length - 1, -1, -1):
                 grid, g = grids[t]
-                sin = state_struct(work[t], self.is_ding, self.transport, self.gas)
+                sin = structs[t]
                 if self.transport:
                     self._check(self.lib.bk_transport_adjoint_prepare(
                         C.byref(p), C.byref(sin), C.byref(cst), _p(g["node_dT_ratio"]), _p(tb["T_mat"]),
                         _p(tb["mass"]), _p(tb["tau"]), stream), "bk_transport_adjoint_prepare")
-                    smech = state_struct(work[t], self.is_ding, self.transport, self.gas)
+                    smech = BkState.from_buffer_copy(sin)
                     smech.tau, smech.material_temperature = _p(tb["tau"]), _p(tb["T_mat"])
                     self._check(self.fn(C.byref(p), C.byref(smech), C.byref(cst_mech), _p(g["node_pm"]),
                                         _p(g["node_v"]), g["bounds"].data_ptr() + 6 * 4, C.byref(adj_struct),
@@ -360,15 +362,15 @@ class _Runner:
         self.checkpoints = []
         return adj, params_adj, rate_adj
 
-    def _run(self, state_in, state_out, phases, grid, surface):
+    def _run(self, state_in, state_out, phases, grid, surface, prepared):
         eng = self.engine
         if not self.transport:
-            eng.run(state_in, state_out, False, phases, False, grid=grid)
+            eng.run(state_in, state_out, False, phases, False, grid=grid, prepared=prepared)
             return
         saved = eng.surface
         eng.surface = surface
         try:
-            eng.run(state_in, state_out, False, phases, False, grid=grid, keep_fields=True)
+            eng.run(state_in, state_out, False, phases, False, grid=grid, keep_fields=True, prepared=prepared)
         finally:
             eng.surface = saved
 

@@ -430,9 +430,12 @@ class MpmSimulator:
         output = self._allocate_like_current(share_accumulators=False) if self.retain_history else self.next_state
         full = self.diagnostics == "full"
         if check and self.transport is not None:
-            self._engine.run(original, output, was_settling, PHASE_TRANSPORT, full, prescattered=prescattered)
+            prepared = self._engine.prepare(was_settling)
+            self._engine.run(original, output, was_settling, PHASE_TRANSPORT, full, prescattered=prescattered,
+                             prepared=prepared)
             self.transport.CheckState()
-            self._engine.run(original, output, was_settling, PHASE_MECHANICS, full, prescatter_next=prescatter_next)
+            self._engine.run(original, output, was_settling, PHASE_MECHANICS, full, prescatter_next=prescatter_next,
+                             prepared=prepared)
         else:
             # unchecked: the surface kernel advances the accumulators (nothing can reject the substep)
             self._engine.run(original, output, was_settling, PHASE_TRANSPORT | PHASE_MECHANICS, full,
@@ -461,6 +464,32 @@ class MpmSimulator:
         if self.sort_interval and self.step_count % self.sort_interval == 0:
             self.SortParticles()
 
+    def _unchecked_substeps(self, count, ahead=False):
+        """``count`` unchecked substeps. Past settling, and unless a state history or a recorder wants
+        to see each of them, the library launches them from one call (the host's work per substep was
+        more than a small body's substep takes on the device), in pieces that end where the particles
+        are re-sorted. ``ahead``: each substep scatters the next one's transport fields, to the last."""
+        if self.IsSettling or self.retain_history or getattr(self, "result_recorder", None) is not None:
+            for k in range(count):
+                self._substep(check=False, prescattered=ahead and k > 0, prescatter_next=ahead and k + 1 < count)
+            return
+        full = self.diagnostics == "full"
+        while count > 0:
+            piece = count
+            if self.sort_interval:
+                piece = min(count, self.sort_interval - self.step_count % self.sort_interval)
+            self._engine.run_many(self._current, self.next_state, piece, full, ahead)
+            if piece % 2:
+                self._current, self.next_state = self.next_state, self._current
+            self._stale = True
+            if full:
+                self._engine.materialize(self._current, plastic=False)
+                self._stale = False
+            self.step_count += piece
+            count -= piece
+            if self.sort_interval and self.step_count % self.sort_interval == 0:
+                self.SortParticles()
+
     def MaxReturnResiduals(self):
         """(max return residual, max porosity residual) of the last substep, on the host."""
         return tuple(self._engine.max_residuals.tolist())
@@ -485,9 +514,15 @@ class MpmSimulator:
             raise ValueError("step_count must be positive")
         start = self.step_count
         ahead = self.scatter_ahead and self._engine.prescatter_allowed()
-        for k in range(step_count):
-            self._substep(check=self.IsSettling, prescattered=ahead and k > 0,
-                          prescatter_next=ahead and k + 1 < step_count)
+        left = step_count
+        while left > 0 and self.IsSettling:
+            self._substep(check=True, prescattered=ahead and left < step_count, prescatter_next=ahead and left > 1)
+            left -= 1
+        if left == step_count:
+            self._unchecked_substeps(left, ahead)
+        else:
+            for k in range(left):
+                self._substep(check=False, prescattered=ahead, prescatter_next=ahead and k + 1 < left)
         values = self._check_values()
         messages = []
         if isinstance(self.material, DingMaterial):
@@ -507,8 +542,7 @@ class MpmSimulator:
         With ``scatter_ahead`` set, each substep's G2P within the call scatters the next substep's
         transport fields ahead."""
         ahead = self.scatter_ahead and self._engine.prescatter_allowed()
-        for k in range(step_count):
-            self._substep(check=False, prescattered=ahead and k > 0, prescatter_next=ahead and k + 1 < step_count)
+        self._unchecked_substeps(step_count, ahead)
 
     def StepSummary(self, out=None):
         """Device tensor (grid mass of the last substep, particle kinetic energy of the current

@@ -104,6 +104,7 @@ CHECK_BLOCKS = 296
 _SIGS = {
     "bk_check_state": [P, P, P, P],
     "bk_substep": [P] * 8 + [C.c_int32, P],
+    "bk_substeps": [P] * 9 + [C.c_int32, C.c_int32, P],
     "bk_materialize": [P] * 11 + [P],
     "bk_surface_accumulate": [P, C.c_float, P, P, P],
     "bk_batch_create": [P, C.c_int32, P],
@@ -331,18 +332,56 @@ class SubstepEngine:
         sur = self.surrogate
         return bool(self.transport) and not (sur is not None and sur.packed)
 
+    def prepare(self, settling):
+        """The parameter and constant structs of ``run``, for several runs of one call that nothing
+        can change in between."""
+        return self.params(settling), self.constants(settling)
+
+    def _diagnostics(self, state_out, full):
+        diag = BkDiagnostics()
+        diag.max_residuals = _p(self.max_residuals)
+        if full and self.is_ding:
+            m = state_out.material_state
+            diag.plastic_gradients = _p(m.plastic_gradients)
+            diag.return_residuals = _p(m.return_residuals)
+            diag.porosity_residuals = _p(m.porosity_residuals)
+        return diag
+
+    def run_many(self, state, other, count, full_diagnostics, scatter_ahead=False):
+        """``count`` unchecked substeps past settling, state -> other -> state ..., in one library call
+        (bk_substeps): what ``count`` runs with ``accumulate`` of the state written would launch."""
+        p, cst = self.prepare(False)
+        p.status = _p(self.status)
+        p.transport_prescatter_stale = int(self.transport and self.prescatter_pending)
+        if self.transport:
+            self.prescatter_pending = False
+        pair = (state, other)
+        states = (BkState * 2)(*(state_struct(s, self.is_ding, self.transport, self.gas) for s in pair))
+        diags = (BkDiagnostics * 2)(*(self._diagnostics(s, full_diagnostics) for s in pair))
+        losses = exchanges = None
+        if self.transport:
+            losses = (P * 2)(*(_p(s.transport_state.water_losses) for s in pair))
+            exchanges = (P * 2)(*(_p(s.transport_state.heat_exchanges) for s in pair))
+        rc = self.lib.bk_substeps(C.byref(p), states, losses, exchanges, C.byref(cst), C.byref(self.grid),
+                                  C.byref(self.surface), diags, C.byref(self.flags), int(count), int(scatter_ahead),
+                                  _lib.stream_handle())
+        if rc != 0:
+            raise RuntimeError(f"bk_substeps failed ({rc}): {self.lib.bk_last_error().decode(errors='replace')}")
+
     def run(self, state_in, state_out, settling, phases, full_diagnostics, grid=None, keep_fields=False,
-            prescattered=False, prescatter_next=False, accumulate=None):
+            prescattered=False, prescatter_next=False, accumulate=None, prepared=None):
         """One substep through bk_substep. ``prescattered``: the previous run scattered this substep's
         transport fields ahead (its ``prescatter_next``), so the scalar P2G is skipped;
         ``prescatter_next``: scatter the next substep's, which must start from ``state_out`` with
         nothing changed in between. ``accumulate``: a transport state whose water-loss and
-        heat-exchange accumulators the surface kernel advances (in place of accumulate_surface)."""
-        p = self.params(settling)
+        heat-exchange accumulators the surface kernel advances (in place of accumulate_surface).
+        ``prepared``: the structs of ``prepare``."""
+        p, cst = self.prepare(settling) if prepared is None else prepared
         p.keep_transport_fields = int(keep_fields)
         p.transport_prescattered = int(prescattered)
         p.transport_prescatter_next = int(prescatter_next)
         p.status = _p(self.status)
+        p.transport_prescatter_stale = 0
         own_grid = grid is None
         if own_grid and (phases & PHASE_TRANSPORT) and self.transport:
             if prescattered and not self.prescatter_pending:
@@ -350,16 +389,9 @@ class SubstepEngine:
             # fields scattered ahead that this substep does not use are cleared first
             p.transport_prescatter_stale = int(self.prescatter_pending and not prescattered)
             self.prescatter_pending = False
-        cst = self.constants(settling)
         sin = state_struct(state_in, self.is_ding, self.transport, self.gas)
         sout = state_struct(state_out, self.is_ding, self.transport, self.gas)
-        diag = BkDiagnostics()
-        diag.max_residuals = _p(self.max_residuals)
-        if full_diagnostics and self.is_ding:
-            m = state_out.material_state
-            diag.plastic_gradients = _p(m.plastic_gradients)
-            diag.return_residuals = _p(m.return_residuals)
-            diag.porosity_residuals = _p(m.porosity_residuals)
+        diag = self._diagnostics(state_out, full_diagnostics)
         # (under a KernelTimer the library times bk_substep's kernels one by one)
         stream = _lib.stream_handle()
         sf = self.surface

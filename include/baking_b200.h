@@ -311,8 +311,7 @@ typedef struct BkSubstepParams {
                                        scattered ahead (box in bounds[12..17]) are still on the grid
                                        and are cleared before this substep's scalar P2G */
     int32_t *status;                /* optional (device, 1 int, may be NULL): set to 1 when a kernel gave
-                                       up a bounded wait (a bulk copy into shared memory or a
-                                       tensor-core completion) and left its particles unprocessed */
+                                       up a bounded wait (a tensor-core completion) and left its particles unprocessed */
 } BkSubstepParams;
 
 #define BK_PHASE_TRANSPORT 1       /* surface terms, scalar P2G, diffusion */
@@ -322,6 +321,18 @@ typedef struct BkSubstepParams {
 BK_API int bk_substep(const BkSubstepParams *params, const BkState *in, BkState *out, const BkConstants *constants,
                       BkGrid *grid, BkSurface *surface, BkDiagnostics *diagnostics, BkFlags *flags,
                       int32_t phases, void *stream);
+
+/* `count` substeps back to back (both phases, nothing read on the host in between), stepping
+   states[0] -> states[1] -> states[0] and so on: the launches that `count` calls of bk_substep would
+   make. Index k of water_losses, heat_exchanges (surface accumulators, advanced every substep; NULL
+   without transport) and diagnostics belongs to the substeps that write states[k]. With scatter_ahead
+   every substep but the last scatters the next one's transport fields (transport_prescatter_next);
+   params' own transport_prescattered and transport_prescatter_next must be 0, its
+   transport_prescatter_stale applies to the first substep. */
+BK_API int bk_substeps(const BkSubstepParams *params, const BkState *states, double *const *water_losses,
+                       double *const *heat_exchanges, const BkConstants *constants, BkGrid *grid,
+                       const BkSurface *surface, const BkDiagnostics *diagnostics, BkFlags *flags, int32_t count,
+                       int32_t scatter_ahead, void *stream);
 
 /* bk_substep's mechanics phase with the grid held in a fixed array inside this library, for
    callers that must not allocate device memory (code inside an allocator hook, a real-time or
