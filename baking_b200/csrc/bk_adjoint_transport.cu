@@ -26,6 +26,8 @@
 #include "baking_b200.h"
 #include "bk_common.h"
 #include "bk_device.cuh"
+#include "bk_launch.cuh"
+#include "bk_scatter.cuh"
 
 using namespace bk;
 
@@ -44,7 +46,7 @@ struct BkGridFields {
 struct TParams {
     int64_t n, pitch;
     int R;
-    float origin[3], dx, dt;
+    float origin[3], dx, rec_dx, dt;
     double rho_w, s0, c_water, kc, kw, cell;
     int water_enabled;
     double oven, tray, tray_transfer, surface_loss, latent;
@@ -52,27 +54,6 @@ struct TParams {
     int gas, settling;
     double ambient, peak, width, source_scale;  // gas: ambient pressure, source peak/width, dt * density
 };
-
-__device__ __forceinline__ float qgrad(float l, int o) {
-    if (o == 0) return -(1.5f - l);
-    if (o == 1) return -2.f * (l - 1.f);
-    return l - 0.5f;
-}
-
-__device__ __forceinline__ void node_offset(int j, int& ox, int& oy, int& oz) {
-    ox = j / 9;
-    oy = (j / 3) % 3;
-    oz = j - 9 * ox - 3 * oy;
-}
-
-// Weight of stencil node j and its gradient with respect to the particle position.
-__device__ __forceinline__ float weight_and_grad(const Stencil& st, int ox, int oy, int oz, float inv_dx, float* dw) {
-    const float wx = st.w[0][ox], wy = st.w[1][oy], wz = st.w[2][oz];
-    dw[0] = qgrad(st.l[0], ox) * inv_dx * wy * wz;
-    dw[1] = qgrad(st.l[1], oy) * inv_dx * wx * wz;
-    dw[2] = qgrad(st.l[2], oz) * inv_dx * wx * wy;
-    return wx * wy * wz;
-}
 
 __device__ __forceinline__ void add_det_grad(float* Fb, int64_t i, int64_t pitch, const M3& F, float scale) {
     // d det(F) / dF = det(F) F^-T; adds scale * det(F) F^-T
@@ -103,21 +84,14 @@ __device__ __forceinline__ double source_moles(const TParams& P, const BkState& 
 // ------------------------------------------------------------------ prepare
 __global__ void k_tadj_prepare(TParams P, BkState in, BkConstants cst, const double2* __restrict__ dTr,
                                float* __restrict__ T_mat, float* __restrict__ mass, float* __restrict__ tau_eff) {
+    pdl_enter();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= P.n) return;
     const int64_t pitch = P.pitch;
-    Stencil st = make_stencil(load_v3(in.x, i, pitch), P.origin, P.dx, P.R);
+    Stencil st = make_stencil(load_v3(in.x, i, pitch), P.origin, P.dx, P.R, P.rec_dx);
     if (!st.valid) return;
-    double dTp = 0.0, ratio = 0.0;
-#pragma unroll
-    for (int j = 0; j < 27; ++j) {
-        int ox, oy, oz;
-        node_offset(j, ox, oy, oz);
-        const double w = (double)(st.w[0][ox] * st.w[1][oy] * st.w[2][oz]);
-        const double2 d = dTr[node_index(st.b[0] + ox, st.b[1] + oy, st.b[2] + oz, P.R)];
-        dTp += w * d.x;
-        ratio += w * d.y;
-    }
+    double dTp, ratio;
+    gather_scalars(st, dTr, P.R, dTp, ratio);
     const double T = in.temperature[i];
     const double Tn = T + dTp, Wn = in.water[i] * (1.0 + ratio);
     T_mat[i] = (float)Tn;
@@ -134,7 +108,7 @@ __global__ void k_tadj_prepare(TParams P, BkState in, BkConstants cst, const dou
             for (int e = 0; e < 9; ++e) tau.m[e] += (e % 4) == 0 ? iso : 0.0f;
         }
     }
-    const double sat = Wn / (P.rho_w * (double)cst.volume[i] * (double)J);
+    const double sat = Wn * reciprocal_newton(P.rho_w * (double)cst.volume[i] * (double)J);
     const float iso = J * (float)P.c_water * ((float)sat - (float)P.s0);
 #pragma unroll
     for (int e = 0; e < 9; ++e) tau.m[e] -= (e % 4) == 0 ? iso : 0.0f;
@@ -142,62 +116,68 @@ __global__ void k_tadj_prepare(TParams P, BkState in, BkConstants cst, const dou
 }
 
 // ------------------------------------------------------------- scalar chain
-// Node adjoints of (dT, dW/W) are scattered like the forward's scalar P2G: a block stages the node
-// box its particles touch in shared memory (when it fits kTileNodes), and within a warp each run
-// of particles with the same stencil base is summed by 27 lanes, one node each, before one atomic
-// per node.
-constexpr int kTileNodes = 512;
-
-struct ScalarSmem {
-    float w[kThreads][9];
-    double val[kThreads][2];
-    double tile[2][kTileNodes];
-    int box[6];
-};
-
-__device__ __forceinline__ long long pack_base(const int* b) {
-    return ((long long)b[0] << 42) | ((long long)b[1] << 21) | (long long)b[2];
-}
-
-__global__ void __launch_bounds__(kThreads) k_tadj_scalar(TParams P, BkState in, BkConstants cst,
+// Node adjoints of (dT, dW/W) are scattered like the forward's scalar P2G (bk_scatter.cuh). The gather
+// needs sum w (dT, r) for T' and W' and sum grad w (dT, r), which does not depend on the adjoints, for
+// the weight gradients of x: both in float64, axis by axis. 1M particles: 173 us with a weight product,
+// its gradients and a block tile per node and particle, now 133; it waits for memory (long_scoreboard 12
+// of 17 cycles an issue at 4 blocks per SM), so eight blocks per SM with a few spilled registers are faster.
+__global__ void __launch_bounds__(kThreads, 8) k_tadj_scalar(TParams P, BkState in, BkConstants cst,
                                                         const double2* __restrict__ dTr, BkAdjointTransport a,
                                                         const BkAdjointState adj, double2* __restrict__ dTr_bar) {
-    __shared__ ScalarSmem sm;
+    pdl_enter();
+    __shared__ ScalarRecord<2> sm[kThreads / 32];
     const int tid = threadIdx.x, lane = tid & 31;
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + tid;
     const int64_t pitch = P.pitch;
+    prefetch_planes(i, P.n, pitch, in.F, 9, adj.F, 9, adj.x, 3);
     double rate_b = 0.0;  // dL/d(gas source rate) through this particle
     double Tnb = 0.0, ratiob = 0.0;
     Stencil st;
     st.valid = false;
     st.b[0] = st.b[1] = st.b[2] = 0;
-    if (i < P.n) st = make_stencil(load_v3(in.x, i, pitch), P.origin, P.dx, P.R);
+    if (i < P.n) st = make_stencil(load_v3(in.x, i, pitch), P.origin, P.dx, P.R, P.rec_dx);
     const bool valid = i < P.n && st.valid;
     if (i < P.n && !st.valid) {
         a.temperature_in[i] = 0.0;
         a.water_in[i] = 0.0;
         if (P.gas) a.gas_moles_in[i] = 0.0;
     } else if (valid) {
-        // one pass over the stencil: T' and W' need sum w (dT, r); the weight gradients of x need
-        // sum grad w (dT, r), which do not depend on the adjoints
         double dTp = 0.0, ratio = 0.0;
-        float gT[3] = {0.f, 0.f, 0.f}, gr[3] = {0.f, 0.f, 0.f};
-        const float inv_dx = 1.f / P.dx;
+        double gT[3] = {0.0, 0.0, 0.0}, gr[3] = {0.0, 0.0, 0.0};  // times dx
+        const double2* nodes = dTr + node_index(st.b[0], st.b[1], st.b[2], P.R);
+        const int64_t R = P.R;
+#pragma unroll 1
+        for (int ox = 0; ox < 3; ++ox) {
+            const double wx = (double)pick3(st.w[0], ox), gx = (double)qweight_grad(st.l[0], ox);
+            double tx = 0.0, rx = 0.0, tgy = 0.0, rgy = 0.0, tgz = 0.0, rgz = 0.0;
 #pragma unroll
-        for (int j = 0; j < 27; ++j) {
-            int ox, oy, oz;
-            node_offset(j, ox, oy, oz);
-            float dw[3];
-            const double w = (double)weight_and_grad(st, ox, oy, oz, inv_dx, dw);
-            const double2 d = dTr[node_index(st.b[0] + ox, st.b[1] + oy, st.b[2] + oz, P.R)];
-            dTp += w * d.x;
-            ratio += w * d.y;
-            const float fx = (float)d.x, fy = (float)d.y;
+            for (int oy = 0; oy < 3; ++oy) {
+                const double wy = (double)st.w[1][oy], gy = (double)qweight_grad(st.l[1], oy);
+                double ty = 0.0, ry = 0.0, tg = 0.0, rg = 0.0;
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                gT[c] += dw[c] * fx;
-                gr[c] += dw[c] * fy;
+                for (int oz = 0; oz < 3; ++oz) {
+                    const double wz = (double)st.w[2][oz], gz = (double)qweight_grad(st.l[2], oz);
+                    const double2 d = __ldg(nodes + (ox * R + oy) * R + oz);
+                    ty = fma(wz, d.x, ty);
+                    ry = fma(wz, d.y, ry);
+                    tg = fma(gz, d.x, tg);
+                    rg = fma(gz, d.y, rg);
+                }
+                tx = fma(wy, ty, tx);
+                rx = fma(wy, ry, rx);
+                tgy = fma(gy, ty, tgy);
+                rgy = fma(gy, ry, rgy);
+                tgz = fma(wy, tg, tgz);
+                rgz = fma(wy, rg, rgz);
             }
+            dTp = fma(wx, tx, dTp);
+            ratio = fma(wx, rx, ratio);
+            gT[0] = fma(gx, tx, gT[0]);
+            gr[0] = fma(gx, rx, gr[0]);
+            gT[1] = fma(wx, tgy, gT[1]);
+            gr[1] = fma(wx, rgy, gr[1]);
+            gT[2] = fma(wx, tgz, gT[2]);
+            gr[2] = fma(wx, rgz, gr[2]);
         }
         const double T = in.temperature[i], Tn = T + dTp;
         const double W = in.water[i];
@@ -206,7 +186,8 @@ __global__ void __launch_bounds__(kThreads) k_tadj_scalar(TParams P, BkState in,
         const float Jf = det3(F);
         const double J = (double)Jf;
         const double V0 = (double)cst.volume[i];
-        const double sat = Wn / (P.rho_w * V0 * J);
+        const double i_J = reciprocal_newton(J), i_full = i_J * reciprocal_newton(P.rho_w * V0);
+        const double sat = Wn * i_full;
         // adjoints arriving at T', W', T_mat, mass and the P2G stress
         Tnb = a.temperature_out[i] + (double)adj.temperature[i];
         double Wnb = a.water_out[i] + (double)adj.mass[i];
@@ -215,8 +196,8 @@ __global__ void __launch_bounds__(kThreads) k_tadj_scalar(TParams P, BkState in,
         const double isob = -trace;
         double Jb = isob * P.c_water * (sat - P.s0);
         const double satb = isob * J * P.c_water;
-        Wnb += satb / (P.rho_w * V0 * J);
-        Jb -= satb * sat / J;
+        Wnb += satb * i_full;
+        Jb -= satb * sat * i_J;
         double Tb_direct = 0.0;  // through the source's mean temperature, besides T'
         if (P.gas) {
             double ez = 0.0, z = 0.0;
@@ -229,10 +210,11 @@ __global__ void __launch_bounds__(kThreads) k_tadj_scalar(TParams P, BkState in,
                 const double pg = (double)(float)gas_pressure(Np, Tm, Jf, n);
                 Jb += trace * (P.ambient - pg);
                 const double pb = -trace * J;
-                Npb += pb * kGasConstant * (double)Tm / (J * (double)n);
-                Tnb += pb * pg / (double)Tm;
-                Jb -= pb * pg / J;
-                adj.porosity[i] += (float)(-pb * pg / (double)n);
+                const double i_n = reciprocal_newton((double)n);
+                Npb += pb * kGasConstant * (double)Tm * (i_J * i_n);
+                Tnb += pb * pg * reciprocal_newton((double)Tm);
+                Jb -= pb * pg * i_J;
+                adj.porosity[i] += (float)(-pb * pg * i_n);
             }
             a.gas_moles_in[i] = Npb;
             if (!P.settling) {
@@ -248,85 +230,13 @@ __global__ void __launch_bounds__(kThreads) k_tadj_scalar(TParams P, BkState in,
         a.water_in[i] = Wnb * (1.0 + ratio);
         a.temperature_in[i] = Tnb + Tb_direct;
         // weight gradients: x_bar += sum_j grad w_j (dT_j T'_bar + r_j ratio_bar)
-        const float tb = (float)Tnb, rb = (float)ratiob;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) adj.x[c * pitch + i] += gT[c] * tb + gr[c] * rb;
+        for (int c = 0; c < 3; ++c) adj.x[c * pitch + i] += (float)((gT[c] * Tnb + gr[c] * ratiob) * (double)P.rec_dx);
         add_det_grad(adj.F, i, pitch, F, (float)Jb);
     }
     // ---- scatter w (T'_bar, ratio_bar) into the node adjoints
-#pragma unroll
-    for (int ax = 0; ax < 3; ++ax)
-#pragma unroll
-        for (int o = 0; o < 3; ++o) sm.w[tid][3 * ax + o] = valid ? st.w[ax][o] : 0.f;
-    sm.val[tid][0] = Tnb;
-    sm.val[tid][1] = ratiob;
-    if (tid < 6) sm.box[tid] = tid < 3 ? INT_MAX : INT_MIN;
-    __syncthreads();
-#pragma unroll
-    for (int ax = 0; ax < 3; ++ax) {
-        const int lo = __reduce_min_sync(0xffffffffu, valid ? st.b[ax] : INT_MAX);
-        const int hi = __reduce_max_sync(0xffffffffu, valid ? st.b[ax] + 2 : INT_MIN);
-        if (lane == 0 && lo != INT_MAX) {
-            atomicMin(&sm.box[ax], lo);
-            atomicMax(&sm.box[3 + ax], hi);
-        }
-    }
-    __syncthreads();
-    int lo[3] = {0, 0, 0}, ext[3] = {1, 1, 1};
-    int count = 0;
-    bool tiled = false;
-    if (sm.box[0] != INT_MAX) {
-        long long c = 1;
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax) {
-            lo[ax] = sm.box[ax];
-            ext[ax] = sm.box[3 + ax] - sm.box[ax] + 1;
-            c *= ext[ax];
-        }
-        tiled = c <= kTileNodes;
-        count = tiled ? (int)c : 0;
-    }
-    for (int t = tid; t < count; t += kThreads) sm.tile[0][t] = sm.tile[1][t] = 0.0;
-    __syncthreads();
-    const long long key = valid ? pack_base(st.b) : -1;
-    const long long prev = __shfl_up_sync(0xffffffffu, key, 1);
-    unsigned starts = __ballot_sync(0xffffffffu, valid && (lane == 0 || prev != key));
-    const int warp_base = tid & ~31;
-    int ox, oy, oz;
-    node_offset(lane < 27 ? lane : 0, ox, oy, oz);
-    while (starts) {
-        const int s0 = __ffs(starts) - 1;
-        starts &= starts - 1;
-        const int e = starts ? __ffs(starts) - 1 : 32;
-        const int b0 = __shfl_sync(0xffffffffu, st.b[0], s0), b1 = __shfl_sync(0xffffffffu, st.b[1], s0),
-                  b2 = __shfl_sync(0xffffffffu, st.b[2], s0);
-        if (lane < 27) {
-            double acc0 = 0.0, acc1 = 0.0;
-            for (int k = warp_base + s0; k < warp_base + e; ++k) {
-                const double w = (double)(sm.w[k][ox] * sm.w[k][3 + oy] * sm.w[k][6 + oz]);
-                acc0 += w * sm.val[k][0];
-                acc1 += w * sm.val[k][1];
-            }
-            if (tiled) {
-                const int t = ((b0 + ox - lo[0]) * ext[1] + (b1 + oy - lo[1])) * ext[2] + (b2 + oz - lo[2]);
-                atomicAdd(&sm.tile[0][t], acc0);
-                atomicAdd(&sm.tile[1][t], acc1);
-            } else {
-                double2* d = dTr_bar + node_index(b0 + ox, b1 + oy, b2 + oz, P.R);
-                atomicAdd(&d->x, acc0);
-                atomicAdd(&d->y, acc1);
-            }
-        }
-    }
-    __syncthreads();
-    for (int t = tid; t < count; t += kThreads) {
-        const double v0 = sm.tile[0][t], v1 = sm.tile[1][t];
-        if (v0 == 0.0 && v1 == 0.0) continue;
-        const int z = t % ext[2], y = (t / ext[2]) % ext[1], x = t / (ext[2] * ext[1]);
-        double2* d = dTr_bar + node_index(lo[0] + x, lo[1] + y, lo[2] + z, P.R);
-        atomicAdd(&d->x, v0);
-        atomicAdd(&d->y, v1);
-    }
+    const double val[2] = {Tnb, ratiob};
+    scatter_scalars<2, 2>(sm[tid >> 5], valid, st, val, {&dTr_bar->x, &dTr_bar->y}, P.R, group_lanes(P.n, P.R));
     if (P.gas && a.gas_rate) {
         if (cst.gas_rate_per_particle) {
             if (i < P.n) a.gas_rate[i] += rate_b;
@@ -362,6 +272,7 @@ __device__ __forceinline__ NodeVals node_vals(const TParams& P, double* const* f
 }
 
 __global__ void k_tadj_diffuse(TParams P, BkGridFields g, const int32_t* __restrict__ box) {
+    pdl_enter();
     int lo[3], ext[3];
     int64_t count = 1;
 #pragma unroll
@@ -446,20 +357,23 @@ __global__ void k_tadj_diffuse(TParams P, BkGridFields g, const int32_t* __restr
 // Node fields (volume V0 det F, capacity, capacity T, W) += w (...) for every particle: the
 // reverse of that scatter is a 27-node gather of the four field adjoints. The block first stages
 // the adjoints of its particles' node box in shared memory (when the box fits kScatterTile nodes),
-// so that the gathers read shared memory.
+// so that the gathers read shared memory. 1M particles: 141 us with the weight products and their
+// gradients formed per node and field, now 116 (seven blocks per SM for the same reason as above).
 constexpr int kScatterTile = 512;
 
-__global__ void __launch_bounds__(kThreads) k_tadj_scatter(TParams P, BkState in, BkConstants cst, BkGridFields g,
+__global__ void __launch_bounds__(kThreads, 7) k_tadj_scatter(TParams P, BkState in, BkConstants cst, BkGridFields g_bar,
                                                          BkAdjointTransport a, const BkAdjointState adj) {
+    pdl_enter();
     __shared__ double s_bar[4][kScatterTile];
     __shared__ int s_box[6];
     const int tid = threadIdx.x, lane = tid & 31;
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + tid;
     const int64_t pitch = P.pitch;
+    prefetch_planes(i, P.n, pitch, in.F, 9, adj.F, 9, adj.x, 3);
     Stencil st;
     st.valid = false;
     st.b[0] = st.b[1] = st.b[2] = 0;
-    if (i < P.n) st = make_stencil(load_v3(in.x, i, pitch), P.origin, P.dx, P.R);
+    if (i < P.n) st = make_stencil(load_v3(in.x, i, pitch), P.origin, P.dx, P.R, P.rec_dx);
     const bool valid = i < P.n && st.valid;
     // the block's node box
     if (tid < 6) s_box[tid] = tid < 3 ? INT_MAX : INT_MIN;
@@ -490,37 +404,63 @@ __global__ void __launch_bounds__(kThreads) k_tadj_scatter(TParams P, BkState in
         const int z = t % ext[2], y = (t / ext[2]) % ext[1], x = t / (ext[2] * ext[1]);
         const int64_t node = node_index(lo[0] + x, lo[1] + y, lo[2] + z, P.R);
 #pragma unroll
-        for (int f = 0; f < 4; ++f) s_bar[f][t] = g.field_bar[f][node];
+        for (int f = 0; f < 4; ++f) s_bar[f][t] = g_bar.field_bar[f][node];
     }
     __syncthreads();  // uniform: every thread reaches it
     if (!valid) return;
     const M3 F = load_m3(in.F, i, pitch);
     const double vol = (double)cst.volume[i] * (double)det3(F);
     const double cap = cst.capacity[i], T = in.temperature[i], W = in.water[i];
-    double volb = 0.0, Tb = 0.0, Wb = 0.0;
-    const float inv_dx = 1.f / P.dx;
-    float xg[3] = {0.f, 0.f, 0.f};
-#pragma unroll 3
-    for (int j = 0; j < 27; ++j) {
-        int ox, oy, oz;
-        node_offset(j, ox, oy, oz);
-        float dw[3];
-        const double w = (double)weight_and_grad(st, ox, oy, oz, inv_dx, dw);
-        double f0, f1, f2, f3;
-        if (count > 0) {
-            const int t = ((st.b[0] + ox - lo[0]) * ext[1] + (st.b[1] + oy - lo[1])) * ext[2] + (st.b[2] + oz - lo[2]);
-            f0 = s_bar[0][t]; f1 = s_bar[1][t]; f2 = s_bar[2][t]; f3 = s_bar[3][t];
-        } else {
-            const int64_t node = node_index(st.b[0] + ox, st.b[1] + oy, st.b[2] + oz, P.R);
-            f0 = g.field_bar[0][node]; f1 = g.field_bar[1][node]; f2 = g.field_bar[2][node]; f3 = g.field_bar[3][node];
-        }
-        volb += w * f0;
-        Tb += w * cap * f2;
-        Wb += w * f3;
-        const float sv = (float)(vol * f0 + cap * f1 + cap * T * f2 + W * f3);
+    const double* const bar[4] = {g_bar.field_bar[0], g_bar.field_bar[1], g_bar.field_bar[2], g_bar.field_bar[3]};
+    // sums of w f0, w f2 and w f3, and the weight gradients of the cofactor, axis by axis
+    const double capT = cap * T;
+    double v0 = 0.0, v2 = 0.0, v3 = 0.0, g[3] = {0.0, 0.0, 0.0};
+    const int row = count > 0 ? ext[2] : P.R;
+    const int64_t plane = count > 0 ? (int64_t)ext[1] * ext[2] : (int64_t)P.R * P.R;
+    const int64_t corner = count > 0 ? ((int64_t)(st.b[0] - lo[0]) * ext[1] + (st.b[1] - lo[1])) * ext[2] + (st.b[2] - lo[2])
+                                     : node_index(st.b[0], st.b[1], st.b[2], P.R);
+    auto gather = [&](auto field) {
+#pragma unroll 1
+        for (int ox = 0; ox < 3; ++ox) {
+            double x0 = 0.0, x2 = 0.0, x3 = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) xg[c] += dw[c] * sv;
-    }
+            for (int oy = 0; oy < 3; ++oy) {
+                double y0 = 0.0, y2 = 0.0, y3 = 0.0, s0 = 0.0, s1 = 0.0;
+                const int64_t at = corner + ox * plane + oy * row;
+#pragma unroll
+                for (int oz = 0; oz < 3; ++oz) {
+                    const double f0 = field(0, at + oz), f1 = field(1, at + oz), f2 = field(2, at + oz), f3 = field(3, at + oz);
+                    const double w = (double)st.w[2][oz];
+                    const double s = fma(vol, f0, fma(cap, f1, fma(capT, f2, W * f3)));
+                    y0 = fma(w, f0, y0);
+                    y2 = fma(w, f2, y2);
+                    y3 = fma(w, f3, y3);
+                    s0 = fma(w, s, s0);
+                    s1 = fma((double)qweight_grad(st.l[2], oz), s, s1);
+                }
+                const double w = (double)st.w[1][oy];
+                x0 = fma(w, y0, x0);
+                x2 = fma(w, y2, x2);
+                x3 = fma(w, y3, x3);
+                gx = fma(w, s0, gx);
+                gy = fma((double)qweight_grad(st.l[1], oy), s0, gy);
+                gz = fma(w, s1, gz);
+            }
+            const double w = (double)pick3(st.w[0], ox);
+            v0 = fma(w, x0, v0);
+            v2 = fma(w, x2, v2);
+            v3 = fma(w, x3, v3);
+            g[0] = fma((double)qweight_grad(st.l[0], ox), gx, g[0]);
+            g[1] = fma(w, gy, g[1]);
+            g[2] = fma(w, gz, g[2]);
+        }
+    };
+    if (count > 0) gather([&](int f, int64_t t) { return s_bar[f][t]; });
+    else gather([&](int f, int64_t t) { return __ldg(bar[f] + t); });
+    const double volb = v0, Tb = cap * v2, Wb = v3;
+    float xg[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) xg[c] = (float)(g[c] * (double)P.rec_dx);
     a.temperature_in[i] += Tb;
     a.water_in[i] += Wb;
 #pragma unroll
@@ -530,15 +470,31 @@ __global__ void __launch_bounds__(kThreads) k_tadj_scatter(TParams P, BkState in
 
 // ---------------------------------------------------------------- surface
 // Mesh vertex positions of this substep (geometry/mesh_tracking.py:13-38) into surface.vertices,
-// as the forward's transport phase computes them (vertex_block: one block per boundary vertex).
+// as the forward's transport phase computes them: a block of 128 or 256 threads per vertex of a coarse
+// mesh, a warp per vertex of a fine one (kBlock = 32), kVertexWarps to a block.
+constexpr int kVertexWarps = 4;
 template <int kBlock>
-__global__ void __launch_bounds__(kBlock) k_tadj_vertex_positions(TParams P, const float* __restrict__ x,
-                                                               const float* __restrict__ F, BkSurface sf) {
-    const int vid = sf.vertex_ids[blockIdx.x];
-    const float v = vertex_block<kBlock>(sf.binding_offsets, sf.binding_particles, sf.binding_weights,
-                                           sf.reference_offsets, sf.binding_pitch, sf.reference_vertices,
-                                           sf.vertex_pitch, x, F, P.pitch, vid);
-    if (threadIdx.x < 3) sf.vertices[threadIdx.x * sf.vertex_pitch + vid] = v;
+constexpr int vertex_threads() { return kBlock == 32 ? 32 * kVertexWarps : kBlock; }
+
+template <int kBlock>
+__global__ void __launch_bounds__(vertex_threads<kBlock>()) k_tadj_vertex_positions(TParams P, const float* __restrict__ x,
+                                                                                const float* __restrict__ F, BkSurface sf) {
+    pdl_enter();
+    if constexpr (kBlock == 32) {
+        const int64_t k = (int64_t)blockIdx.x * kVertexWarps + (threadIdx.x >> 5);
+        if (k >= sf.vertex_count) return;  // whole warps
+        const int vid = sf.vertex_ids[k];
+        const float v = vertex_warp(sf.binding_offsets, sf.binding_particles, sf.binding_weights, sf.reference_offsets,
+                                    sf.binding_pitch, sf.reference_vertices, sf.vertex_pitch, x, F, P.pitch, vid);
+        const int lane = threadIdx.x & 31;
+        if (lane < 3) sf.vertices[lane * sf.vertex_pitch + vid] = v;
+    } else {
+        const int vid = sf.vertex_ids[blockIdx.x];
+        const float v = vertex_block<kBlock>(sf.binding_offsets, sf.binding_particles, sf.binding_weights,
+                                               sf.reference_offsets, sf.binding_pitch, sf.reference_vertices,
+                                               sf.vertex_pitch, x, F, P.pitch, vid);
+        if (threadIdx.x < 3) sf.vertices[threadIdx.x * sf.vertex_pitch + vid] = v;
+    }
 }
 
 __device__ __forceinline__ void face_vertices(const BkSurface& sf, int f, double q[3][3], int vid[3]) {
@@ -551,14 +507,12 @@ __device__ __forceinline__ void face_vertices(const BkSurface& sf, int f, double
     }
 }
 
-__global__ void k_tadj_owners(TParams P, BkState in, BkConstants cst, BkSurface sf, BkGridFields g,
-                              BkAdjointTransport a, const BkAdjointState adj) {
-    const int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (o >= sf.owner_count) return;
+// Owner o (particle p): its rates' adjoints to the state and to the face vertices; returns the
+// heat-transfer parameter's.
+__device__ __forceinline__ double owner_reverse(const TParams& P, const BkState& in, const BkConstants& cst, const BkSurface& sf,
+                                                const BkGridFields& g, const BkAdjointTransport& a, const BkAdjointState& adj,
+                                                int64_t o, int p, const Stencil& st) {
     const int64_t pitch = P.pitch;
-    const int p = sf.owners[o];
-    Stencil st = make_stencil(load_v3(in.x, p, pitch), P.origin, P.dx, P.R);
-    if (!st.valid) return;
     // recompute the owner's exposed and tray-contact areas
     double exposed = 0.0, contact = 0.0;
     const int f0 = sf.owner_face_offsets[o], f1 = sf.owner_face_offsets[o + 1];
@@ -582,23 +536,39 @@ __global__ void k_tadj_owners(TParams P, BkState in, BkConstants cst, BkSurface 
     const double loss = P.water_enabled ? P.surface_loss * T * sat * exposed : 0.0;
     const double heat = h * exposed * (P.oven - T) + P.tray_transfer * contact * (P.tray - T) - P.latent * loss;
     // gather the heat and loss adjoints from the owner's stencil
-    double heatb = 0.0, lossb = 0.0;
-    const float inv_dx = 1.f / P.dx;
-    float xg[3] = {0.f, 0.f, 0.f};
-#pragma unroll 1
-    for (int j = 0; j < 27; ++j) {
-        int ox, oy, oz;
-        node_offset(j, ox, oy, oz);
-        float dw[3];
-        const double w = (double)weight_and_grad(st, ox, oy, oz, inv_dx, dw);
-        const int64_t node = node_index(st.b[0] + ox, st.b[1] + oy, st.b[2] + oz, P.R);
-        const double fh = g.field_bar[4][node], fl = g.field_bar[5][node];
-        heatb += w * fh;
-        lossb += w * fl;
-        const float s = (float)(heat * fh + loss * fl);
+    double heatb = 0.0, lossb = 0.0, gs[3] = {0.0, 0.0, 0.0};
+    const int64_t R = P.R, corner = node_index(st.b[0], st.b[1], st.b[2], P.R);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) xg[c] += dw[c] * s;
+    for (int ox = 0; ox < 3; ++ox) {
+        double hx = 0.0, lx = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
+#pragma unroll
+        for (int oy = 0; oy < 3; ++oy) {
+            double hy = 0.0, ly = 0.0, s1 = 0.0;
+#pragma unroll
+            for (int oz = 0; oz < 3; ++oz) {
+                const int64_t node = corner + (ox * R + oy) * R + oz;
+                const double fh = __ldg(g.field_bar[4] + node), fl = __ldg(g.field_bar[5] + node);
+                hy = fma((double)st.w[2][oz], fh, hy);
+                ly = fma((double)st.w[2][oz], fl, ly);
+                s1 = fma((double)qweight_grad(st.l[2], oz), heat * fh + loss * fl, s1);
+            }
+            const double w = (double)st.w[1][oy], s0 = heat * hy + loss * ly;
+            hx = fma(w, hy, hx);
+            lx = fma(w, ly, lx);
+            gx = fma(w, s0, gx);
+            gy = fma((double)qweight_grad(st.l[1], oy), s0, gy);
+            gz = fma(w, s1, gz);
+        }
+        const double w = (double)st.w[0][ox];
+        heatb = fma(w, hx, heatb);
+        lossb = fma(w, lx, lossb);
+        gs[0] = fma((double)qweight_grad(st.l[0], ox), gx, gs[0]);
+        gs[1] = fma(w, gy, gs[1]);
+        gs[2] = fma(w, gz, gs[2]);
     }
+    float xg[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) xg[c] = (float)(gs[c] * (double)P.rec_dx);
 #pragma unroll
     for (int c = 0; c < 3; ++c) adj.x[c * pitch + p] += xg[c];
     const double lossb_all = lossb - P.latent * heatb;
@@ -613,7 +583,7 @@ __global__ void k_tadj_owners(TParams P, BkState in, BkConstants cst, BkSurface 
         add_det_grad(adj.F, p, pitch, F, (float)(volb * (double)cst.volume[p]));
     }
     a.temperature_in[p] += Tb;
-    if (a.heat_parameter) atomicAdd(a.heat_parameter, heatb * exposed * (P.oven - T));
+    const double hb = heatb * exposed * (P.oven - T);
     // face areas -> vertex adjoints
     const int64_t vp = sf.vertex_pitch;
     for (int f = f0; f < f1; ++f) {
@@ -640,30 +610,59 @@ __global__ void k_tadj_owners(TParams P, BkState in, BkConstants cst, BkSurface 
             atomicAdd(&a.vertices[c * vp + vid[2]], e2b[c]);
         }
     }
+    return hb;
 }
 
-// One block per surface vertex: its adjoint to the bound particles' x and F, then zeroed.
+__global__ void k_tadj_owners(TParams P, BkState in, BkConstants cst, BkSurface sf, BkGridFields g,
+                              BkAdjointTransport a, const BkAdjointState adj) {
+    pdl_enter();
+    const int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t pitch = P.pitch;
+    const bool mine = o < sf.owner_count;
+    const int p = mine ? sf.owners[o] : 0;
+    double hb = 0.0;
+    Stencil st;
+    st.valid = false;
+    if (mine) st = make_stencil(load_v3(in.x, p, pitch), P.origin, P.dx, P.R, P.rec_dx);
+    if (mine && st.valid) hb = owner_reverse(P, in, cst, sf, g, a, adj, o, p, st);
+    // One shared parameter: a warp's sum in one atomic (an atomic per owner queued tens of thousands of
+    // them on one address: 85 us for a ball of 100k particles, 18 with this and the gather in columns).
+    if (a.heat_parameter) {
+#pragma unroll
+        for (int k = 16; k > 0; k >>= 1) hb += __shfl_xor_sync(0xffffffffu, hb, k);
+        if ((threadIdx.x & 31) == 0 && hb != 0.0) atomicAdd(a.heat_parameter, hb);
+    }
+}
+
+// One block (kBlock = 32: one warp) per surface vertex: its adjoint to the bound particles' x and F,
+// then zeroed.
 template <int kBlock>
-__global__ void __launch_bounds__(kBlock) k_tadj_vertices(TParams P, BkSurface sf, BkAdjointTransport a,
-                                                       const BkAdjointState adj) {
+__global__ void __launch_bounds__(vertex_threads<kBlock>()) k_tadj_vertices(TParams P, BkSurface sf, BkAdjointTransport a,
+                                                                        const BkAdjointState adj) {
+    pdl_enter();
     __shared__ float s_w[kBlock / 32];
-    const int vid = sf.vertex_ids[blockIdx.x];
-    const int t = threadIdx.x;
+    const int64_t k = kBlock == 32 ? (int64_t)blockIdx.x * kVertexWarps + (threadIdx.x >> 5) : (int64_t)blockIdx.x;
+    if (k >= sf.vertex_count) return;  // whole warps, or the whole block
+    const int vid = sf.vertex_ids[k];
+    const int t = threadIdx.x % kBlock;
     const int64_t vp = sf.vertex_pitch, bp = sf.binding_pitch, pitch = P.pitch;
     const double vb[3] = {a.vertices[vid], a.vertices[vp + vid], a.vertices[2 * vp + vid]};
-    __syncthreads();
+    if constexpr (kBlock == 32) __syncwarp();
+    else __syncthreads();
     if (t < 3) a.vertices[t * vp + vid] = 0.0;
     const int b0 = sf.binding_offsets[vid], b1 = sf.binding_offsets[vid + 1];
-    if (b0 == b1 || (vb[0] == 0.0 && vb[1] == 0.0 && vb[2] == 0.0)) return;  // the same for the whole block
+    if (b0 == b1 || (vb[0] == 0.0 && vb[1] == 0.0 && vb[2] == 0.0)) return;  // the same for the whole block or warp
     // v = (1 - sum_b w_b) pred_b0 + sum_b w_b pred_b
     float wsum = 0.f;
     for (int b = b0 + t; b < b1; b += kBlock) wsum += sf.binding_weights[b];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
-    if ((t & 31) == 0) s_w[t >> 5] = wsum;
-    __syncthreads();
-    wsum = 0.f;
-    for (int w = 0; w < kBlock / 32; ++w) wsum += s_w[w];
+    if constexpr (kBlock > 32) {
+        if ((t & 31) == 0) s_w[t >> 5] = wsum;
+        __syncthreads();
+        wsum = 0.f;
+        for (int w = 0; w < kBlock / 32; ++w) wsum += s_w[w];
+    }
     for (int b = b0 + t; b < b1; b += kBlock) {
         const float c = sf.binding_weights[b] + (b == b0 ? 1.f - wsum : 0.f);
         const int p = sf.binding_particles[b];
@@ -673,13 +672,14 @@ __global__ void __launch_bounds__(kBlock) k_tadj_vertices(TParams P, BkSurface s
             const float pb = (float)(c * vb[r]);
             atomicAdd(&adj.x[r * pitch + p], pb);
 #pragma unroll
-            for (int k = 0; k < 3; ++k) atomicAdd(&adj.F[(3 * r + k) * pitch + p], pb * o[k]);
+            for (int k2 = 0; k2 < 3; ++k2) atomicAdd(&adj.F[(3 * r + k2) * pitch + p], pb * o[k2]);
         }
     }
 }
 
 // ------------------------------------------------------------------- clear
 __global__ void k_tadj_clear(TParams P, BkGridFields g, const int32_t* __restrict__ box) {
+    pdl_enter();
     int lo[3], ext[3];
     int64_t count = 1;
 #pragma unroll
@@ -707,7 +707,7 @@ TParams tparams(const BkSubstepParams& p, const BkSurface* sf) {
     TParams t;
     t.n = p.n; t.pitch = p.pitch; t.R = p.resolution;
     for (int k = 0; k < 3; ++k) t.origin[k] = p.origin[k];
-    t.dx = p.spacing; t.dt = p.time_step;
+    t.dx = p.spacing; t.rec_dx = 1.0f / p.spacing; t.dt = p.time_step;
     t.rho_w = p.scalar.water_density;
     t.s0 = p.initial_saturation;
     t.c_water = p.water_stress;
@@ -745,10 +745,10 @@ int bk_transport_adjoint_prepare(const BkSubstepParams* params, const BkState* i
         return fail(BK_ERR_ARGUMENT, "bk_transport_adjoint_prepare: gas mode needs the gas arrays");
     if (p.n == 0) return BK_OK;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    k_tadj_prepare<<<blocks(p.n, 256), 256, 0, s>>>(tparams(p, nullptr), *in, *constants,
-                                                    reinterpret_cast<const double2*>(node_dT_ratio),
-                                                    material_temperature, mass, stress);
-    return check_launch("bk_transport_adjoint_prepare");
+    const cudaError_t e = launch_chained(k_tadj_prepare, blocks(p.n, 256), 256, 0, s, tparams(p, nullptr), *in, *constants,
+                                         reinterpret_cast<const double2*>(node_dT_ratio), material_temperature, mass,
+                                         stress);
+    return check_chained(e, "bk_transport_adjoint_prepare");
 }
 
 int bk_transport_adjoint(const BkSubstepParams* params, const BkState* in, const BkConstants* constants,
@@ -781,39 +781,43 @@ int bk_transport_adjoint(const BkSubstepParams* params, const BkState* in, const
     int device = 0, sms = 148;
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    const unsigned box_blocks = (unsigned)sms * 4;
-    k_tadj_scalar<<<blocks(p.n, kThreads), kThreads, 0, s>>>(P, *in, *constants,
-                                                             reinterpret_cast<const double2*>(grid->node_dT_ratio), a,
-                                                             *mechanics, g.dTr_bar);
-    if (int rc = check_launch("bk_transport_adjoint/scalar")) return rc;
-    k_tadj_diffuse<<<box_blocks, 256, 0, s>>>(P, g, box);
-    if (int rc = check_launch("bk_transport_adjoint/diffuse")) return rc;
-    k_tadj_scatter<<<blocks(p.n, kThreads), kThreads, 0, s>>>(P, *in, *constants, g, a, *mechanics);
-    if (int rc = check_launch("bk_transport_adjoint/scatter")) return rc;
-    if (surface->vertex_count > 0) {
-        const unsigned nv = (unsigned)surface->vertex_count;
-        switch (vertex_block_threads(surface->vertex_count, surface->binding_count)) {
-            case 256: k_tadj_vertex_positions<256><<<nv, 256, 0, s>>>(P, in->x, in->F, *surface); break;
-            case 128: k_tadj_vertex_positions<128><<<nv, 128, 0, s>>>(P, in->x, in->F, *surface); break;
-            default: k_tadj_vertex_positions<32><<<nv, 32, 0, s>>>(P, in->x, in->F, *surface); break;
-        }
-        if (int rc = check_launch("bk_transport_adjoint/vertex_positions")) return rc;
+    // as bk_substep's node-box passes: fewer blocks for small bodies
+    const unsigned box_blocks = p.n / 128 + 1 < (int64_t)sms * 4 ? (unsigned)(p.n / 128 + 1) : (unsigned)sms * 4;
+    cudaError_t e = launch_chained(k_tadj_scalar, blocks(p.n, kThreads), kThreads, 0, s, P, *in, *constants,
+                                   reinterpret_cast<const double2*>(grid->node_dT_ratio), a, *mechanics, g.dTr_bar);
+    if (int rc = check_chained(e, "bk_transport_adjoint/scalar")) return rc;
+    e = launch_chained(k_tadj_diffuse, box_blocks, 256, 0, s, P, g, box);
+    if (int rc = check_chained(e, "bk_transport_adjoint/diffuse")) return rc;
+    e = launch_chained(k_tadj_scatter, blocks(p.n, kThreads), kThreads, 0, s, P, *in, *constants, g, a, *mechanics);
+    if (int rc = check_chained(e, "bk_transport_adjoint/scatter")) return rc;
+    const unsigned nv = (unsigned)surface->vertex_count;
+    const int vertex_block_size = vertex_block_threads(surface->vertex_count, surface->binding_count);
+    if (nv > 0) {
+        if (vertex_block_size == 256)
+            e = launch_chained(k_tadj_vertex_positions<256>, nv, 256, 0, s, P, in->x, in->F, *surface);
+        else if (vertex_block_size == 128)
+            e = launch_chained(k_tadj_vertex_positions<128>, nv, 128, 0, s, P, in->x, in->F, *surface);
+        else
+            e = launch_chained(k_tadj_vertex_positions<32>, blocks(nv, kVertexWarps), 32 * kVertexWarps, 0, s, P, in->x,
+                               in->F, *surface);
+        if (int rc = check_chained(e, "bk_transport_adjoint/vertex_positions")) return rc;
     }
     if (surface->owner_count > 0) {
-        k_tadj_owners<<<blocks(surface->owner_count, 64), 64, 0, s>>>(P, *in, *constants, *surface, g, a, *mechanics);
-        if (int rc = check_launch("bk_transport_adjoint/owners")) return rc;
+        e = launch_chained(k_tadj_owners, blocks(surface->owner_count, 64), 64, 0, s, P, *in, *constants, *surface, g, a,
+                           *mechanics);
+        if (int rc = check_chained(e, "bk_transport_adjoint/owners")) return rc;
     }
-    if (surface->vertex_count > 0) {
-        const unsigned nv = (unsigned)surface->vertex_count;
-        switch (vertex_block_threads(surface->vertex_count, surface->binding_count)) {
-            case 256: k_tadj_vertices<256><<<nv, 256, 0, s>>>(P, *surface, a, *mechanics); break;
-            case 128: k_tadj_vertices<128><<<nv, 128, 0, s>>>(P, *surface, a, *mechanics); break;
-            default: k_tadj_vertices<32><<<nv, 32, 0, s>>>(P, *surface, a, *mechanics); break;
-        }
-        if (int rc = check_launch("bk_transport_adjoint/vertices")) return rc;
+    if (nv > 0) {
+        if (vertex_block_size == 256) e = launch_chained(k_tadj_vertices<256>, nv, 256, 0, s, P, *surface, a, *mechanics);
+        else if (vertex_block_size == 128)
+            e = launch_chained(k_tadj_vertices<128>, nv, 128, 0, s, P, *surface, a, *mechanics);
+        else
+            e = launch_chained(k_tadj_vertices<32>, blocks(nv, kVertexWarps), 32 * kVertexWarps, 0, s, P, *surface, a,
+                               *mechanics);
+        if (int rc = check_chained(e, "bk_transport_adjoint/vertices")) return rc;
     }
-    k_tadj_clear<<<box_blocks, 256, 0, s>>>(P, g, box);
-    return check_launch("bk_transport_adjoint/clear");
+    e = launch_chained(k_tadj_clear, box_blocks, 256, 0, s, P, g, box);
+    return check_chained(e, "bk_transport_adjoint/clear");
 }
 
 }  // extern "C"

@@ -25,6 +25,21 @@ namespace bk {
 
 constexpr unsigned kWarp = 0xffffffffu;
 
+// The 128-byte lines of plane arrays that a warp's 32 particles read, requested into L2 by one
+// instruction per 32 lines (lane c takes plane c) before the values are needed: the loads of a
+// particle kernel fall into phases (position, node gather, state) and each phase otherwise waits for
+// DRAM again.
+BK_DEV void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// Up to 32 planes of three arrays.
+BK_DEV void prefetch_planes(int64_t i, int64_t n, int64_t pitch, const float* a, int na, const float* b, int nb,
+                            const float* c, int nc) {
+    const int lane = threadIdx.x & 31;
+    const int64_t w0 = i - lane;
+    if (w0 >= n || lane >= na + nb + nc) return;
+    prefetch_l2((lane < na ? a + lane * pitch : lane < na + nb ? b + (lane - na) * pitch : c + (lane - na - nb) * pitch) + w0);
+}
+
 // ------------------------------------------------------------- node gathers
 // sum_j w_j v_j and the moments sum_j w_j v_j o_jc over the stencil's nodes, with the offsets o_j in
 // {0, 1, 2} known at compile time: what G2P forms v and C of (C_rc = 4/dx (M_rc - l_c S_r)).
@@ -82,9 +97,14 @@ BK_DEV void gather_scalars(const Stencil& st, const double2* __restrict__ dTr, i
     }
 }
 
+// a[k] for a run-time k in {0, 1, 2} without dynamic register indexing (which would move `a` to local
+// memory): the outer loop of a long gather stays a loop, so that its 27 nodes' loads are not all hoisted
+// and held at once.
+BK_DEV float pick3(const float* a, int k) { return k == 0 ? a[0] : (k == 1 ? a[1] : a[2]); }
+
 // Derivative of the quadratic weight of offset o by l (transfer.py:4-13).
 BK_DEV float qweight_grad(float l, int o) {
-    if (o == 0) return -(1.5f - l);
+    if (o == 0) return l - 1.5f;
     if (o == 1) return -2.f * (l - 1.f);
     return l - 0.5f;
 }

@@ -129,12 +129,6 @@ struct Slot {
 };
 __device__ __forceinline__ Slot grid_slot() { return Slot{(int)blockIdx.x, (int)gridDim.x}; }
 
-// The 128-byte lines of plane arrays that a warp's 32 particles read, requested into L2 by one
-// instruction per 32 lines (lane c takes plane c) before the values are needed: the loads of a
-// particle kernel fall into phases (position, node gather, state) and each phase otherwise waits for
-// DRAM again.
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-
 // How a kernel body takes its parameter structs: by value from a plain launch's parameter space
 // (a reference to a kernel parameter would make the compiler copy it to local memory), by
 // reference to the batched launch's shared-memory entry (a value copy would hold every field in
