@@ -632,12 +632,22 @@ BK_DEV double overstress64(double q, double p, double d, double h, double* warm 
     return r;
 }
 
+// exp(x): the plastic volume strains of a substep are small, and for |x| < 2^-5 ten terms of the series
+// (remainder below 3e-23) take a third of the general function's instructions.
+BK_DEV double exp_small(double x) {
+    if (!(fabs(x) < 0x1p-5)) return exp(x);
+    double s = 1.0 + x * (1.0 / 10.0);
+#pragma unroll
+    for (int k = 9; k >= 1; --k) s = fma(x * (1.0 / k), s, 1.0);
+    return s;
+}
+
 BK_DEV double porosity_prediction(double n, float q, float p, float d, float h, float e, double Vp, float n0,
                                   double* warm = nullptr) {
     double a = pressure_coefficient64(n);
     double r = overstress64((double)q, a * (double)p, (double)d, (double)h * a, warm);
     if (r == 0.0) return Vp - 1.0 + (double)n0;  // no overstress: exp(e (1 - 1/1)) = exp(0) = 1 exactly
-    return Vp * exp((double)e * (1.0 - reciprocal_newton(1.0 + (double)h * a * r))) - 1.0 + (double)n0;
+    return Vp * exp_small((double)e * (1.0 - reciprocal_newton(1.0 + (double)h * a * r))) - 1.0 + (double)n0;
 }
 
 // prediction(n) and its derivative in n. The overstress root r(n) is the reference's 48-step Newton
@@ -656,7 +666,7 @@ BK_DEV double porosity_prediction_slope(double n, float qf, float pf, float df, 
     double r = overstress64(q, a * p, d, h * a, warm);
     const double u = 1.0 + d * r, v = 1.0 + h * a * r;
     const double uv = reciprocal_newton(u * v), iu = v * uv, iv = u * uv;
-    double core = Vp * exp(e * (1.0 - iv));
+    double core = Vp * exp_small(e * (1.0 - iv));
     double dr = 0.0;
     if (q + a * p > 1.0) {
         const double Rr = 1.0 + 2.0 * (d * q * iu * iu * iu + h * a * a * p * iv * iv * iv);
@@ -695,18 +705,20 @@ static __device__ __noinline__ float solve_porosity_bisection(float q, float p, 
 // NULL) reports that certain case; there prediction(float(trial)) has no overstress and equals
 // trial, so the caller can skip that evaluation. Every other case takes the float64 test.
 //
+// `plastic`: the caller has certified q + a(trial) p > 1 (particle_side), so the elastic tests are skipped.
 // A Newton step below 1e-7 n^2 (or 1e-14 n) ends the solve without another evaluation: the error left
 // is of the order of its square over n (a(n) varies with ln n). `consistency` (may be NULL) then returns |float(n) - prediction(float(n))| from the
 // root and the slope there (the terms left out are of the order of ulp^2), or -1 where the caller has
 // to evaluate it.
 BK_DEV float solve_porosity(float q, float p, float d, float h, float e, double Vp, float n0,
-                            double* warm = nullptr, bool* elastic_exit = nullptr, double* consistency = nullptr) {
+                            double* warm = nullptr, bool* elastic_exit = nullptr, double* consistency = nullptr,
+                            bool plastic = false) {
     double r_local = 0.0;
     if (!warm) warm = &r_local;
     if (elastic_exit) *elastic_exit = false;
     if (consistency) *consistency = -1.0;
     double trial = Vp - 1.0 + (double)n0;
-    if (trial > 0.0 && trial < 1.0) {
+    if (!plastic && trial > 0.0 && trial < 1.0) {
         const float nf = (float)trial;
         const float lgf = logf(1.0f / nf);
         const float af = 9.0f / (4.0f * (lgf * lgf) * (3.5f * nf + 1.0f));
@@ -751,7 +763,7 @@ BK_DEV float solve_porosity(float q, float p, float d, float h, float e, double 
 }
 
 // Gas mode's end-state porosity (ding.py:181-197) with its consistency residual and the overstress root
-// it ended with. Out of line: particles that are certainly elastic (certain_elastic) never come here,
+// it ended with. Out of line: particles that are certainly elastic (particle_side) never come here,
 // and the float64 solve would otherwise stand between the instructions that every particle runs (the
 // kernel's top stall was instruction fetch). Scalars by value: a reference to the kernel's parameters
 // would copy them to local memory.
@@ -759,13 +771,13 @@ struct DingPorosity {
     float ret_por, consistency, r;
 };
 static __device__ __noinline__ DingPorosity ding_porosity(float q2, float p2, float df, float ms, float ex, float por,
-                                                          float n0) {
+                                                          float n0, bool plastic) {
     DingPorosity o;
     double r_warm = 0.0;  // overstress root carried from one solve to the next
     const double Vp = 1.0 - (double)n0 + (double)por;
     bool elastic_exit;
     double consistency;
-    o.ret_por = solve_porosity(q2, p2, df, ms, ex, Vp, n0, &r_warm, &elastic_exit, &consistency);
+    o.ret_por = solve_porosity(q2, p2, df, ms, ex, Vp, n0, &r_warm, &elastic_exit, &consistency, plastic);
     if (consistency < 0.0) {
         // Certain elastic exit: prediction(ret_por) has r = 0 and returns Vp - 1 + n0 exactly.
         const double pred = elastic_exit ? Vp - 1.0 + (double)n0
@@ -777,15 +789,16 @@ static __device__ __noinline__ DingPorosity ding_porosity(float q2, float p2, fl
     return o;
 }
 
-// Gas mode: true only where the elastic exit of the porosity solve (q + a(trial) p <= 1) is certain.
-// a(n) from the hardware logarithm is within 1e-5 of its value for n <= 0.9, and q + a p is tested
-// against 1 - 1e-4; other particles take the full branch, which decides exactly.
-BK_DEV bool certain_elastic(float dev2, float mean, float ty, double trial) {
+// Gas mode: on which side of the elastic exit (q + a(trial) p <= 1) a particle certainly lies: -1
+// elastic, 1 plastic, 0 where the exact test has to decide. a(n) from the hardware logarithm is within
+// 1e-5 of its value for n <= 0.9, and q + a p is tested against 1 -+ 1e-4.
+BK_DEV int particle_side(float dev2, float mean, float ty, double trial) {
     const float n = (float)trial;
-    if (!(n >= 1.0e-30f && n <= 0.9f)) return false;
+    if (!(n >= 1.0e-30f && n <= 0.9f)) return 0;
     const float lg = __logf(n);
     const float a = __fdividef(9.0f, 4.0f * (lg * lg) * (3.5f * n + 1.0f));
-    return dev2 + a * mean * mean <= (1.0f - 1.0e-4f) * (ty * ty);
+    const float load = dev2 + a * mean * mean, ty2 = ty * ty;
+    return load <= (1.0f - 1.0e-4f) * ty2 ? -1 : load >= (1.0f + 1.0e-4f) * ty2 ? 1 : 0;
 }
 
 struct DingParticleOut {
@@ -924,7 +937,8 @@ BK_DEV void ding_exact(const DingParamsDev& P, const DingPrelude& d, float por, 
     out.porosity_residual = 0.0f;
     out.yielded = false;
     bool von_mises = false;  // a(n) = 0
-    if (P.coupled_porosity && certain_elastic(dev2, mean, d.ty, trial)) {
+    const int side = P.coupled_porosity ? particle_side(dev2, mean, d.ty, trial) : 0;
+    if (side < 0) {
         ret_por = (float)trial;
         out.porosity_residual = (float)fabs((double)ret_por - trial);
 #pragma unroll
@@ -936,7 +950,8 @@ BK_DEV void ding_exact(const DingParamsDev& P, const DingPrelude& d, float por, 
         float r_warm = 0.0f;
         if (P.coupled_porosity) {
             const float ms = 2.0f / 3.0f * (2.0f * mu + 3.0f * lam) * dt * ty * ty / eta;
-            const DingPorosity o = ding_porosity(q2, mean * mean / ty2, df, ms, 3.0f * mean / (2.0f * mu + 3.0f * lam), por, n0);
+            const DingPorosity o = ding_porosity(q2, mean * mean / ty2, df, ms, 3.0f * mean / (2.0f * mu + 3.0f * lam), por, n0,
+                                                 side > 0);
             ret_por = o.ret_por;
             out.porosity_residual = o.consistency;
             r_warm = o.r;

@@ -901,7 +901,7 @@ __device__ __forceinline__ void ding_store(const Params& P, const BkState& out, 
 // ------------------------------------------------------ return-map surrogate
 struct SurrogateDev {
     const unsigned char* blob;
-    float in_mean[8], in_scale[8], in_low[8], in_high[8], out_scale[4];
+    float in_mean[8], in_scale[8], in_rec[8], in_low[8], in_high[8], out_scale[4];  // in_rec = 1 / in_scale
     float* samples;
     int32_t* sample_count;
     int sample_capacity, sample_stride, sample_offset;
@@ -917,6 +917,7 @@ SurrogateDev surrogate_dev(const BkReturnSurrogate* r) {
     for (int k = 0; k < 8; ++k) {
         d.in_mean[k] = r->norm.in_mean[k];
         d.in_scale[k] = r->norm.in_scale[k] != 0.0f ? r->norm.in_scale[k] : 1.0f;
+        d.in_rec[k] = 1.0f / d.in_scale[k];
         d.in_low[k] = r->in_low[k];
         d.in_high[k] = r->in_high[k];
     }
@@ -953,7 +954,8 @@ __device__ __forceinline__ void surrogate_features(const Params& P, const BkStat
 #pragma unroll
     for (int k = 0; k < 3; ++k) f[k] = sel3(d.e, perm[k]);
     f[3] = d.T_eff;
-    f[4] = P.transport ? (float)(out.water[i] / ((double)P.water_density * (double)cst.volume[i] * (double)J)) : 0.0f;
+    f[4] = P.transport ? (float)(out.water[i] * reciprocal_newton((double)P.water_density * (double)cst.volume[i] * (double)J))
+                       : 0.0f;
     f[5] = P.gas ? (float)out.gas_moles[i] : 0.0f;
     f[6] = logf(1.0f - P.ding.initial_porosity + por);
 }
@@ -968,6 +970,11 @@ __device__ __forceinline__ bool ding_elastic(const DingParamsDev& D, const DingP
     for (int k = 0; k < 3; ++k) ts[k] = 2.0f * D.mu * st[k] + D.lam * tr;
     float mean = (ts[0] + ts[1] + ts[2]) / 3.0f;
     float dev[3] = {ts[0] - mean, ts[1] - mean, ts[2] - mean};
+    if (D.coupled_porosity) {
+        const double trial = 1.0 - (double)D.initial_porosity + (double)por - 1.0 + (double)D.initial_porosity;
+        const int side = particle_side(1.5f * (dev[0] * dev[0] + dev[1] * dev[1] + dev[2] * dev[2]), mean, d.ty, trial);
+        if (side != 0) return side < 0;
+    }
     float ty2 = d.ty * d.ty;
     float q = 1.5f * (dev[0] * dev[0] + dev[1] * dev[1] + dev[2] * dev[2]) / ty2;
     float p = mean * mean / ty2;
@@ -990,11 +997,11 @@ __device__ bool ding_surrogate(const DingParamsDev& D, const DingPrelude& d, flo
     float ret_por = por;
     if (D.coupled_porosity) {
         double dv = (double)d.e[0] + (double)d.e[1] + (double)d.e[2] - ((double)e[0] + e[1] + e[2]);
-        double rp = (1.0 - (double)D.initial_porosity + (double)por) * exp(dv) - 1.0 + (double)D.initial_porosity;
+        double rp = (1.0 - (double)D.initial_porosity + (double)por) * exp_small(dv) - 1.0 + (double)D.initial_porosity;
         if (!(rp > 0.0 && rp < 1.0)) return false;
         ret_por = (float)rp;
     }
-    const float eb = (e[0] + e[1] + e[2]) / 3.0f;
+    const float eb = div_uniform(e[0] + e[1] + e[2], 3.0f, 1.0f / 3.0f);
     float cs[3], ex[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -1172,6 +1179,7 @@ __device__ __forceinline__ void g2p_return_surrogate_body(Arg<Params, kRef> P, A
     uint32_t phase = 0;
     for (int64_t base = (int64_t)sl.block * 128; base < P.n; base += (int64_t)sl.blocks * 128) {
         const int64_t i = base + threadIdx.x;
+        prefetch_planes(i, P.n, pitch, in.F, 9, in.Fe, P.material == 1 ? 9 : 0, in.x, 3);
         M3 Fn, Cn;
         bool ding = false, use_mlp = false;
         DingPrelude d;
@@ -1190,7 +1198,7 @@ __device__ __forceinline__ void g2p_return_surrogate_body(Arg<Params, kRef> P, A
 #pragma unroll
                 for (int k = 0; k < 7; ++k) {
                     use_mlp = use_mlp && f[k] >= sg.in_low[k] && f[k] <= sg.in_high[k];
-                    x[k] = (f[k] - sg.in_mean[k]) / sg.in_scale[k];
+                    x[k] = div_uniform(f[k] - sg.in_mean[k], sg.in_scale[k], sg.in_rec[k]);
                 }
             }
         }
