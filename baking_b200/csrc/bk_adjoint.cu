@@ -386,9 +386,11 @@ template <bool kCoupled, bool kLoaf = false>
 __global__ void __launch_bounds__(kThreads, 4) k_adj_g2p_return(AdjParams P, BkState in, const float4* __restrict__ grid_v,
                                                           const float* __restrict__ eta_param, AdjState out_adj,
                                                           AdjState in_adj, double* __restrict__ params_adj) {
-    pdl_enter();
     if constexpr (kLoaf) fix_loaf_mode(P);
     const int64_t i = blockIdx.x * (int64_t)kThreads + threadIdx.x;
+    prefetch_planes(i, P.n, P.pitch, in.x, 3, in.F, 9, in.Fe, P.material == 1 ? 9 : 0);
+    prefetch_planes(i, P.n, P.pitch, out_adj.C, 9, out_adj.F, 9, out_adj.tau, P.material == 1 ? 9 : 0);
+    pdl_enter();
     float acc_mu = 0.f, acc_lam = 0.f, acc_eta = 0.f;
     if (i < P.n) {
         const int64_t pitch = P.pitch;
@@ -687,11 +689,12 @@ template <bool kLoaf = false>
 __global__ void __launch_bounds__(kThreads, 7) k_adj_g2p_scatter(AdjParams P, BkState in, const float4* __restrict__ grid_v,
                                                             AdjState out_adj, AdjState in_adj,
                                                             float4* __restrict__ grid_v_adj) {
-    pdl_enter();
     if constexpr (kLoaf) fix_loaf_mode(P);
     __shared__ MomentumRecord sm[kThreads / 32];
     const int64_t i = blockIdx.x * (int64_t)kThreads + threadIdx.x;
     const int64_t pitch = P.pitch;
+    prefetch_planes(i, P.n, pitch, in.x, 3, in_adj.C, 9, out_adj.x, 3);
+    pdl_enter();
     Stencil st;
     st.valid = false;
     st.b[0] = st.b[1] = st.b[2] = 0;
@@ -827,9 +830,11 @@ template <bool kLoaf = false>
 __global__ void __launch_bounds__(kThreads, 6) k_adj_p2g(AdjParams P, BkState in, const float* __restrict__ mass,
                                                    const float* __restrict__ volume, const float4* __restrict__ pm_adj,
                                                    AdjState in_adj, double* __restrict__ params_adj) {
-    pdl_enter();
     if constexpr (kLoaf) fix_loaf_mode(P);
     const int64_t i = blockIdx.x * (int64_t)kThreads + threadIdx.x;
+    prefetch_planes(i, P.n, P.pitch, in.x, 3, in.v, 3, in.C, 9);
+    prefetch_planes(i, P.n, P.pitch, in.tau, P.material == 1 ? 9 : 0, in_adj.x, 3, in.F, P.material == 1 ? 0 : 9);
+    pdl_enter();
     float acc_mu = 0.f, acc_lam = 0.f;
     if (i < P.n) {
         const int64_t pitch = P.pitch;

@@ -124,12 +124,12 @@ __global__ void k_tadj_prepare(TParams P, BkState in, BkConstants cst, const dou
 __global__ void __launch_bounds__(kThreads, 8) k_tadj_scalar(TParams P, BkState in, BkConstants cst,
                                                         const double2* __restrict__ dTr, BkAdjointTransport a,
                                                         const BkAdjointState adj, double2* __restrict__ dTr_bar) {
-    pdl_enter();
     __shared__ ScalarRecord<2> sm[kThreads / 32];
     const int tid = threadIdx.x, lane = tid & 31;
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + tid;
     const int64_t pitch = P.pitch;
     prefetch_planes(i, P.n, pitch, in.F, 9, adj.F, 9, adj.x, 3);
+    pdl_enter();
     double rate_b = 0.0;  // dL/d(gas source rate) through this particle
     double Tnb = 0.0, ratiob = 0.0;
     Stencil st;
@@ -363,13 +363,13 @@ constexpr int kScatterTile = 512;
 
 __global__ void __launch_bounds__(kThreads, 7) k_tadj_scatter(TParams P, BkState in, BkConstants cst, BkGridFields g_bar,
                                                          BkAdjointTransport a, const BkAdjointState adj) {
-    pdl_enter();
     __shared__ double s_bar[4][kScatterTile];
     __shared__ int s_box[6];
     const int tid = threadIdx.x, lane = tid & 31;
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + tid;
     const int64_t pitch = P.pitch;
     prefetch_planes(i, P.n, pitch, in.F, 9, adj.F, 9, adj.x, 3);
+    pdl_enter();
     Stencil st;
     st.valid = false;
     st.b[0] = st.b[1] = st.b[2] = 0;

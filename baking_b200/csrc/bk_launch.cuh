@@ -4,6 +4,9 @@
 // the kernel before it in the stream has completed and its memory is visible (which makes the chain
 // transitive), then lets the next kernel launch; its blocks only take SM slots left free by blocks
 // already running. A kernel without a programmatic predecessor returns from the wait at once.
+// Before the wait a kernel may only compute addresses and ask L2 for lines (prefetch_l2: a hint, whatever
+// the kernel before it is still writing): the particle kernels do, so that their first loads find L2
+// warm (elastic body of 41k particles 920 -> 872 us a 40-substep pass, 9k sphere 2106 -> 2049).
 #pragma once
 
 #include <cstdio>
@@ -18,6 +21,7 @@ __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+
 
 // The status of a launch_chained call, as check_launch reports a launch's.
 inline int check_chained(cudaError_t e, const char* name) {

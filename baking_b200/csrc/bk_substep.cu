@@ -400,6 +400,20 @@ __global__ void __launch_bounds__(kOwnerThreads) k_surface_owners(Params P, BkSt
 // with the node box of the substep.
 using ScatterRecord = ScalarRecord<4>;
 
+// Asks L2 for the lines that the warp's particles read in the scatter.
+__device__ __forceinline__ void scatter_prefetch(const Params& P, const BkState& in, const BkConstants& cst, int block) {
+    const int lane = threadIdx.x & 31;
+    const int64_t w0 = block * (int64_t)kOwnerThreads + (threadIdx.x & ~31);
+    if (w0 >= P.n) return;
+    if (lane < 12) prefetch_l2((lane < 3 ? in.x + lane * P.pitch : in.F + (lane - 3) * P.pitch) + w0);
+    else if (lane == 12) prefetch_l2(cst.volume + w0);
+    else if (lane < 19) {
+        const double* a = lane < 15 ? cst.capacity : lane < 17 ? in.temperature : in.water;
+        const int64_t half = w0 + 16 * ((lane - 13) & 1);
+        prefetch_l2(a + (half < P.n ? half : w0));
+    }
+}
+
 template <bool kRef = false>
 __device__ __forceinline__ void transport_scatter_body(Arg<Params, kRef> P, Arg<BkState, kRef> in,
                                                        Arg<BkConstants, kRef> cst, Arg<GridPtrs, kRef> g, int32_t* sim_flags,
@@ -430,6 +444,7 @@ __device__ __forceinline__ void transport_scatter_body(Arg<Params, kRef> P, Arg<
 
 __global__ void __launch_bounds__(kOwnerThreads, 8) k_transport_scatter(Params P, BkState in, BkConstants cst, GridPtrs g,
                                                                int32_t* sim_flags) {
+    scatter_prefetch(P, in, cst, (int)blockIdx.x);
     pdl_enter();
     transport_scatter_body(P, in, cst, g, sim_flags, grid_slot());
 }
@@ -453,8 +468,9 @@ template <int kBlock>
 __global__ void __launch_bounds__(kOwnerThreads, 8) k_vertices_scatter(Params P, BkState in, BkConstants cst, BkSurface sf,
                                                               GridPtrs g, int32_t* sim_flags, int vertex_blocks) {
     static_assert(vertex_launch_threads(kBlock) == kOwnerThreads, "both bodies share the block size");
-    pdl_enter();
     const Mixed m = mixed_block(vertex_blocks);
+    if (!m.is_first) scatter_prefetch(P, in, cst, m.block);
+    pdl_enter();
     if (m.is_first) surface_vertices_body<kBlock>(P, in.x, in.F, sf, Slot{m.block, vertex_blocks});
     else transport_scatter_body(P, in, cst, g, sim_flags, Slot{m.block, (int)gridDim.x - vertex_blocks});
 }
@@ -462,8 +478,9 @@ __global__ void __launch_bounds__(kOwnerThreads, 8) k_vertices_scatter(Params P,
 // The owners of a fine mesh and the transport scatter, after the vertices.
 __global__ void __launch_bounds__(kOwnerThreads, 8) k_owners_scatter(Params P, BkState in, BkConstants cst, BkSurface sf,
                                                             GridPtrs g, int32_t* sim_flags, int owner_blocks) {
-    pdl_enter();
     const Mixed m = mixed_block(owner_blocks);
+    if (!m.is_first) scatter_prefetch(P, in, cst, m.block);
+    pdl_enter();
     if (m.is_first) surface_owners_run_body(P, in, cst, sf, g, sim_flags, Slot{m.block, owner_blocks});
     else transport_scatter_body(P, in, cst, g, sim_flags, Slot{m.block, (int)gridDim.x - owner_blocks});
 }
@@ -710,7 +727,6 @@ __device__ __forceinline__ void p2g_body(Arg<Params, kRef> P, Arg<BkState, kRef>
                                          Arg<BkConstants, kRef> cst, Arg<GridPtrs, kRef> g, Arg<BkFlags, kRef> flags,
                                          float* max_residuals, Slot sl) {
     __shared__ MomentumRecord sm[kP2GThreads / 32];
-    if (sl.block == 0 && threadIdx.x < 2) max_residuals[threadIdx.x] = 0.0f;
     const int64_t i = sl.block * (int64_t)kP2GThreads + threadIdx.x;
     const int64_t pitch = P.pitch;
     {
@@ -730,8 +746,11 @@ __device__ __forceinline__ void p2g_body(Arg<Params, kRef> P, Arg<BkState, kRef>
             if (lane == 8) prefetch_l2(cst.volume + w0);
             if (lane == 9 && P.material == 1 && P.gas) prefetch_l2(in.porosity + w0);
             if (lane == 10 && P.gas && cst.gas_rate_per_particle) prefetch_l2(cst.gas_rate + w0);
+            if (lane >= 11 && lane < 14) prefetch_l2(in.x + (lane - 11) * pitch + w0);
         }
     }
+    if constexpr (!kRef) pdl_enter();
+    if (sl.block == 0 && threadIdx.x < 2) max_residuals[threadIdx.x] = 0.0f;
     bool valid = false;
     Stencil st;
     st.b[0] = st.b[1] = st.b[2] = 0;
@@ -834,7 +853,6 @@ __device__ __forceinline__ void p2g_body(Arg<Params, kRef> P, Arg<BkState, kRef>
 template <bool kLoaf = false>
 __global__ void __launch_bounds__(kP2GThreads, 8) k_p2g(Params P, BkState in, BkState out, BkConstants cst, GridPtrs g,
                                                  BkFlags flags, float* max_residuals) {
-    pdl_enter();
     if constexpr (kLoaf) fix_loaf_mode(P);
     p2g_body(P, in, out, cst, g, flags, max_residuals, grid_slot());
 }
@@ -1102,8 +1120,10 @@ __device__ __forceinline__ void g2p_return_body(Arg<Params, kRef> P, Arg<BkState
                 prefetch_l2((lane < 9 ? in.F + lane * P.pitch : in.Fe + (lane - 9) * P.pitch) + w0);
             if (lane == 18 && P.material == 1) prefetch_l2(in.porosity + w0);
             if (lane == 19 && P.material == 1) prefetch_l2(in.gelled + w0);
+            if (lane >= 20 && lane < 23) prefetch_l2(in.x + (lane - 20) * P.pitch + w0);
         }
     }
+    if constexpr (!kRef) pdl_enter();
     if (sl.block == 0 && threadIdx.x < 6) {
         // This substep's box becomes the box the next substep clears; the active box restarts empty.
         g.bounds[6 + threadIdx.x] = g.bounds[threadIdx.x];
@@ -1144,7 +1164,6 @@ __device__ __forceinline__ void g2p_return_body(Arg<Params, kRef> P, Arg<BkState
 template <bool kLoaf = false, bool kPrescatter = false>
 __global__ void __launch_bounds__(128, 8) k_g2p_return(Params P, BkState in, BkState out, BkConstants cst, GridPtrs g,
                                                    BkDiagnostics diag, BkFlags flags, SurrogateDev sg) {
-    pdl_enter();
     if constexpr (kLoaf) {
         fix_loaf_mode(P);
         P.prescatter_next = kPrescatter;
@@ -1179,7 +1198,8 @@ __device__ __forceinline__ void g2p_return_surrogate_body(Arg<Params, kRef> P, A
     uint32_t phase = 0;
     for (int64_t base = (int64_t)sl.block * 128; base < P.n; base += (int64_t)sl.blocks * 128) {
         const int64_t i = base + threadIdx.x;
-        prefetch_planes(i, P.n, pitch, in.F, 9, in.Fe, P.material == 1 ? 9 : 0, in.x, 3);
+        // the next tile's planes, while this one computes
+        prefetch_planes(i + (int64_t)sl.blocks * 128, P.n, pitch, in.F, 9, in.Fe, P.material == 1 ? 9 : 0, in.x, 3);
         M3 Fn, Cn;
         bool ding = false, use_mlp = false;
         DingPrelude d;
