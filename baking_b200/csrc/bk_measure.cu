@@ -10,6 +10,7 @@
 #include "baking_b200.h"
 #include "bk_common.h"
 #include "bk_device.cuh"
+#include "bk_launch.cuh"
 
 using namespace bk;
 
@@ -194,17 +195,26 @@ __global__ void k_measure_finish(const double* __restrict__ partial, double* __r
 // Step result: the grid mass of the last substep (node masses over its active box, the only
 // nonzero nodes) and the particles' kinetic energy sum 1/2 m |v|^2 with m = dry + W under
 // transport, in two deterministic passes like k_measure.
-__global__ void __launch_bounds__(kThreads) k_step_summary(int64_t n, int64_t pitch, const float* __restrict__ v,
+// Threads per block of the reductions that run inside stepping loops: twice kThreads, so that
+// BK_MEASURE_BLOCKS blocks (two per SM, the scratch's layout) put 32 warps on an SM: they wait for loads.
+// With the launches chained, a step's summary at 1M particles takes 14.3 us instead of 17.7. The check
+// was bound by float64 divisions and roots as well (six and two a particle): 116 -> 72 us at 1M, 411 ->
+// 239 us at 4M yielding particles (DRAM time about 27 and 110).
+constexpr int kWide = 512;
+
+__global__ void __launch_bounds__(kWide, 2) k_step_summary(int64_t n, int64_t pitch, const float* __restrict__ v,
                                                          const float* __restrict__ mass, const double* __restrict__ dry,
                                                          const double* __restrict__ water, const float4* __restrict__ pm,
                                                          const int32_t* __restrict__ box, int R,
                                                          double* __restrict__ partial) {
+    pdl_enter();
     double grid = 0.0, kinetic = 0.0;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const int64_t first = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+#pragma unroll 4
     for (int64_t i = first; i < n; i += stride) {
-        const double m = water ? dry[i] + water[i] : (double)mass[i];
-        const double a = v[i], b = v[pitch + i], c = v[2 * pitch + i];
+        const double m = water ? __ldg(dry + i) + __ldg(water + i) : (double)__ldg(mass + i);
+        const double a = __ldg(v + i), b = __ldg(v + pitch + i), c = __ldg(v + 2 * pitch + i);
         kinetic += 0.5 * m * (a * a + b * b + c * c);
     }
     int lo[3], ext[3];
@@ -222,7 +232,7 @@ __global__ void __launch_bounds__(kThreads) k_step_summary(int64_t n, int64_t pi
         const int x = lo[0] + (int)(t / ((int64_t)ext[2] * ext[1]));
         grid += (double)pm[node_index(x, y, z, R)].w;
     }
-    __shared__ double s_warp[2][kThreads / 32];
+    __shared__ double s_warp[2][kWide / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -236,12 +246,13 @@ __global__ void __launch_bounds__(kThreads) k_step_summary(int64_t n, int64_t pi
     __syncthreads();
     if (threadIdx.x < 2) {
         double b = 0.0;
-        for (int w = 0; w < kThreads / 32; ++w) b += s_warp[threadIdx.x][w];
+        for (int w = 0; w < kWide / 32; ++w) b += s_warp[threadIdx.x][w];
         partial[2 * (int64_t)blockIdx.x + threadIdx.x] = b;
     }
 }
 
 __global__ void k_step_summary_finish(const double* __restrict__ partial, double* __restrict__ out, int blocks) {
+    pdl_enter();
     const int k = blockIdx.x;  // one warp per value
     const double v = warp_slot_reduce(kSum, partial, blocks, 2, k);
     if (threadIdx.x == 0) out[k] = v;
@@ -261,8 +272,12 @@ __host__ __device__ constexpr int check_op(int s) {
 
 __device__ __forceinline__ void check_add(double* acc, int s, double v) { acc[s] = combine(check_op(s), acc[s], v); }
 
-__global__ void __launch_bounds__(kThreads) k_check_state(BkCheckInputs in, double* __restrict__ partial) {
+// Speeds and gas waves are compared as squares, their roots taken once at the end (the square root is
+// monotone; a negative square stays out, as its root, not a number, did); counts are integers.
+__global__ void __launch_bounds__(kWide, 2) k_check_state(BkCheckInputs in, double* __restrict__ partial) {
+    pdl_enter();
     double acc[kCheckSlots];
+    int nonfinite_state = 0, outside_stencil = 0, nonfinite_ding = 0, nonfinite_vertices = 0, inverted_tets = 0;
 #pragma unroll
     for (int s = 0; s < kCheckSlots; ++s) {
         const int op = check_op(s);
@@ -289,7 +304,7 @@ __global__ void __launch_bounds__(kThreads) k_check_state(BkCheckInputs in, doub
             finite = finite && isfinite(f) && isfinite(c);
             F[e] = f;
         }
-        if (!finite) check_add(acc, BK_CHECK_NONFINITE_STATE, 1.0);
+        nonfinite_state += !finite;
         const double J = F[0] * (F[4] * F[8] - F[5] * F[7]) - F[1] * (F[3] * F[8] - F[5] * F[6]) +
                          F[2] * (F[3] * F[7] - F[4] * F[6]);
         check_add(acc, BK_CHECK_J_MIN, J);
@@ -300,25 +315,27 @@ __global__ void __launch_bounds__(kThreads) k_check_state(BkCheckInputs in, doub
             const double g = (x[a] - (double)in.origin[a]) * inv_dx;
             outside = outside || g < 0.5 || g >= hi;
         }
-        if (outside) check_add(acc, BK_CHECK_OUTSIDE_STENCIL, 1.0);
+        outside_stencil += outside;
         const double speed2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
-        check_add(acc, BK_CHECK_SPEED_MAX, sqrt(speed2));
+        check_add(acc, BK_CHECK_SPEED_MAX, speed2);
         const double V0 = (double)in.reference_volume[i];
         check_add(acc, BK_CHECK_PARTICLE_VOLUME, V0 * J);
         const double m = in.water ? in.dry_mass[i] + in.water[i] : (double)in.mass[i];
         check_add(acc, BK_CHECK_TOTAL_MASS, m);
         check_add(acc, BK_CHECK_KINETIC_ENERGY, 0.5 * m * speed2);
-        const double rho = in.water ? m / V0 : (double)in.density;
+        const double inv_rho = in.water ? V0 * reciprocal_newton(m) : 1.0 / (double)in.density;
         if (in.gas_moles) {
-            const double n = (double)in.porosity[i];
+            const double n = (double)in.porosity[i], inv_n = reciprocal_newton(n);
             const float T = in.temperature ? (float)in.temperature[i] : in.material_temperature[i];
-            const double p = gas_pressure(in.gas_moles[i], T, (float)J, (float)n);
-            const double bulk = p * (1.0 + (1.0 - (double)in.initial_porosity + n) / n);
-            check_add(acc, BK_CHECK_GAS_WAVE_MAX, sqrt(((double)in.gas_modulus + bulk) * J / rho));
+            const double Jf = (double)(float)J;
+            const double p = in.gas_moles[i] * kGasConstant * (double)T * (reciprocal_newton(Jf) * inv_n);
+            const double bulk = p * (1.0 + (1.0 - (double)in.initial_porosity + n) * inv_n);
+            const double wave2 = ((double)in.gas_modulus + bulk) * J * inv_rho;
+            if (wave2 >= 0.0) check_add(acc, BK_CHECK_GAS_WAVE_MAX, wave2);
         }
         if (in.water && in.water_enabled) {
-            const double sat = in.water[i] / ((double)in.water_density * V0 * J);
-            check_add(acc, BK_CHECK_WATER_WAVE2_MAX, (double)in.water_stress * sat * J / rho);
+            const double sat = in.water[i] * reciprocal_newton((double)in.water_density * V0 * J);
+            check_add(acc, BK_CHECK_WATER_WAVE2_MAX, (double)in.water_stress * sat * J * inv_rho);
         }
         if (in.Fe) {
             M3 Fe, Ff;
@@ -334,7 +351,7 @@ __global__ void __launch_bounds__(kThreads) k_check_state(BkCheckInputs in, doub
 #pragma unroll
                 for (int e = 0; e < 9; ++e) ok = ok && isfinite(Fp.m[e]);
             }
-            if (!ok) check_add(acc, BK_CHECK_NONFINITE_DING, 1.0);
+            nonfinite_ding += !ok;
             if (in.return_residuals) check_add(acc, BK_CHECK_RESIDUAL_MAX, (double)in.return_residuals[i]);
         }
     }
@@ -359,7 +376,7 @@ __global__ void __launch_bounds__(kThreads) k_check_state(BkCheckInputs in, doub
     const int64_t vp = in.vertex_pitch;
     for (int64_t q = first; q < in.vertex_count; q += stride) {
         const float a = in.vertices[q], b = in.vertices[vp + q], c = in.vertices[2 * vp + q];
-        if (!(isfinite(a) && isfinite(b) && isfinite(c))) check_add(acc, BK_CHECK_NONFINITE_VERTICES, 1.0);
+        nonfinite_vertices += !(isfinite(a) && isfinite(b) && isfinite(c));
     }
     for (int64_t t = first; t < in.tet_count; t += stride) {
         double c[4][3];
@@ -382,9 +399,16 @@ __global__ void __launch_bounds__(kThreads) k_check_state(BkCheckInputs in, doub
         const double vol = e[0][0] * (e[1][1] * e[2][2] - e[1][2] * e[2][1]) -
                            e[0][1] * (e[1][0] * e[2][2] - e[1][2] * e[2][0]) +
                            e[0][2] * (e[1][0] * e[2][1] - e[1][1] * e[2][0]);
-        if (!inside || vol <= 0.0) check_add(acc, BK_CHECK_INVERTED_TETS, 1.0);
+        inverted_tets += !inside || vol <= 0.0;
     }
-    __shared__ double s_warp[kThreads / 32];
+    acc[BK_CHECK_NONFINITE_STATE] = nonfinite_state;
+    acc[BK_CHECK_OUTSIDE_STENCIL] = outside_stencil;
+    acc[BK_CHECK_NONFINITE_DING] = nonfinite_ding;
+    acc[BK_CHECK_NONFINITE_VERTICES] = nonfinite_vertices;
+    acc[BK_CHECK_INVERTED_TETS] = inverted_tets;
+    if (acc[BK_CHECK_SPEED_MAX] >= 0.0) acc[BK_CHECK_SPEED_MAX] = sqrt(acc[BK_CHECK_SPEED_MAX]);
+    if (acc[BK_CHECK_GAS_WAVE_MAX] >= 0.0) acc[BK_CHECK_GAS_WAVE_MAX] = sqrt(acc[BK_CHECK_GAS_WAVE_MAX]);
+    __shared__ double s_warp[kWide / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int s = 0; s < kCheckSlots; ++s) {
@@ -396,7 +420,7 @@ __global__ void __launch_bounds__(kThreads) k_check_state(BkCheckInputs in, doub
         __syncthreads();
         if (threadIdx.x == 0) {
             double b = s_warp[0];
-            for (int w = 1; w < kThreads / 32; ++w) b = combine(op, b, s_warp[w]);
+            for (int w = 1; w < kWide / 32; ++w) b = combine(op, b, s_warp[w]);
             partial[(int64_t)blockIdx.x * kCheckSlots + s] = b;
         }
         __syncthreads();
@@ -405,6 +429,7 @@ __global__ void __launch_bounds__(kThreads) k_check_state(BkCheckInputs in, doub
 
 __global__ void k_check_finish(const double* __restrict__ partial, double* __restrict__ out, int blocks,
                                BkCheckInputs in) {
+    pdl_enter();
     const int s = blockIdx.x;  // one warp per slot
     const int op = check_op(s);
     double v = warp_slot_reduce(op, partial, blocks, kCheckSlots, s);
@@ -437,13 +462,13 @@ extern "C" int bk_step_summary(const BkSubstepParams* params, const BkState* sta
                                                                       : !constants->mass))
         return fail(BK_ERR_ARGUMENT, "bk_step_summary: missing arrays");
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    k_step_summary<<<BK_MEASURE_BLOCKS, kThreads, 0, s>>>(p.n, p.pitch, state->v, constants->mass, constants->dry_mass,
-                                                          p.transport ? state->water : nullptr,
-                                                          reinterpret_cast<const float4*>(grid->node_pm),
-                                                          grid->bounds + 6, p.resolution, scratch);
-    if (int rc = check_launch("bk_step_summary")) return rc;
-    k_step_summary_finish<<<2, 32, 0, s>>>(scratch, out, BK_MEASURE_BLOCKS);
-    return check_launch("bk_step_summary/finish");
+    cudaError_t e = launch_chained(k_step_summary, BK_MEASURE_BLOCKS, kWide, 0, s, p.n, p.pitch, state->v, constants->mass,
+                                   constants->dry_mass, p.transport ? (const double*)state->water : nullptr,
+                                   reinterpret_cast<const float4*>(grid->node_pm), grid->bounds + 6, p.resolution,
+                                   scratch);
+    if (int rc = check_chained(e, "bk_step_summary")) return rc;
+    e = launch_chained(k_step_summary_finish, 2, 32, 0, s, scratch, out, BK_MEASURE_BLOCKS);
+    return check_chained(e, "bk_step_summary/finish");
 }
 
 extern "C" int bk_measure_state(const BkMeasureInputs* in, double* out, double* scratch, void* stream) {
@@ -485,8 +510,8 @@ extern "C" int bk_check_state(const BkCheckInputs* in, double* out, double* scra
         return fail(BK_ERR_ARGUMENT, "bk_check_state: bad vertex array");
     if (c.tet_count > 0 && (!c.tets || c.vertex_count == 0)) return fail(BK_ERR_ARGUMENT, "bk_check_state: bad tets");
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    k_check_state<<<BK_MEASURE_BLOCKS, kThreads, 0, s>>>(c, scratch);
-    if (int rc = check_launch("bk_check_state")) return rc;
-    k_check_finish<<<kCheckSlots, 32, 0, s>>>(scratch, out, BK_MEASURE_BLOCKS, c);
-    return check_launch("bk_check_state/finish");
+    cudaError_t e = launch_chained(k_check_state, BK_MEASURE_BLOCKS, kWide, 0, s, c, scratch);
+    if (int rc = check_chained(e, "bk_check_state")) return rc;
+    e = launch_chained(k_check_finish, kCheckSlots, 32, 0, s, scratch, out, BK_MEASURE_BLOCKS, c);
+    return check_chained(e, "bk_check_state/finish");
 }
