@@ -7,7 +7,7 @@
 //                    v', C', F', Fe', tau', porosity' back to F, Fe, porosity, temperature and the
 //                    material parameters, and form the v-bar, C-bar the G2P gather receives.
 //   adj_g2p_scatter  per particle: the weight-gradient terms of x; v-bar, C-bar scattered to the
-//                    grid-velocity adjoint through shared-memory tiles (the forward P2G's scheme).
+//                    grid-velocity adjoint by warp runs (the forward P2G's scheme, bk_scatter.cuh).
 //   adj_grid         per node: velocity adjoint -> momentum and mass adjoints (walls clamp to zero).
 //   adj_p2g          per particle: gather the momentum/mass adjoints -> v, C, tau (and, for the
 //                    neo-Hookean model, F and mu, lambda) and the weight-gradient terms of x.
@@ -714,7 +714,11 @@ __global__ void __launch_bounds__(kThreads, 7) k_adj_g2p_scatter(AdjParams P, Bk
 #pragma unroll
         for (int r = 0; r < 3; ++r)
             q[r] = vb[r] - (A[3 * r] * st.l[0] + A[3 * r + 1] * st.l[1] + A[3 * r + 2] * st.l[2]);
-        float dw[3][3];
+        // the gather counts offsets from the middle node: |l - 1| <= 1/2, so its differences lose less
+        float qc[3], dw[3][3];
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+            qc[r] = vb[r] - (A[3 * r] * (st.l[0] - 1.f) + A[3 * r + 1] * (st.l[1] - 1.f) + A[3 * r + 2] * (st.l[2] - 1.f));
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll
@@ -729,7 +733,7 @@ __global__ void __launch_bounds__(kThreads, 7) k_adj_g2p_scatter(AdjParams P, Bk
             for (int oy = 0; oy < 3; ++oy) {
                 float Q[3], Sy[3] = {0.f, 0.f, 0.f}, s0 = 0.f, s1 = 0.f;
 #pragma unroll
-                for (int r = 0; r < 3; ++r) Q[r] = q[r] + ((float)ox * A[3 * r] + (float)oy * A[3 * r + 1]);
+                for (int r = 0; r < 3; ++r) Q[r] = qc[r] + ((float)(ox - 1) * A[3 * r] + (float)(oy - 1) * A[3 * r + 1]) - A[3 * r + 2];
 #pragma unroll
                 for (int oz = 0; oz < 3; ++oz) {
                     const float4 u = __ldg(nodes + (ox * R + oy) * R + oz);
@@ -864,7 +868,8 @@ __global__ void __launch_bounds__(kThreads, 6) k_adj_p2g(AdjParams P, BkState in
             float A[9];
 #pragma unroll
             for (int e = 0; e < 9; ++e) A[e] = m * Cm.m[e] - scale * tau.m[e];
-            // Node mass w m and momentum w Q_j, Q_j = q + A dx o_j with q = m v - A l dx: with the node
+            // Node mass w m and momentum w Q_j, Q_j = q + A dx o_j with q = m v - A (l - 1) dx and o_j counted
+            // from the middle node (M below loses l S, which is three times as large from the first): with the node
             // adjoints pb_j (momentum) and g_j (mass), everything follows from S = sum w pb, G = sum w g,
             // M_c = sum w pb o_c and the weight gradients of the cofactor g_j m + pb_j . Q_j, summed axis by
             // axis (about 20 operations a node; the plain sums took 100: 126 us at 1M particles, now 73, at six blocks per SM).
@@ -874,7 +879,8 @@ __global__ void __launch_bounds__(kThreads, 6) k_adj_p2g(AdjParams P, BkState in
             for (int e = 0; e < 9; ++e) Ad[e] = A[e] * P.dx;
 #pragma unroll
             for (int r = 0; r < 3; ++r)
-                q[r] = m * vel.v[r] - (Ad[3 * r] * st.l[0] + Ad[3 * r + 1] * st.l[1] + Ad[3 * r + 2] * st.l[2]);
+                q[r] = m * vel.v[r] -
+                       (Ad[3 * r] * (st.l[0] - 1.f) + Ad[3 * r + 1] * (st.l[1] - 1.f) + Ad[3 * r + 2] * (st.l[2] - 1.f));
 #pragma unroll
             for (int a = 0; a < 3; ++a)
 #pragma unroll
@@ -889,7 +895,7 @@ __global__ void __launch_bounds__(kThreads, 6) k_adj_p2g(AdjParams P, BkState in
                 for (int oy = 0; oy < 3; ++oy) {
                     float Q[3], Sy[4] = {0.f, 0.f, 0.f, 0.f}, Zy[3] = {0.f, 0.f, 0.f}, s0 = 0.f, s1 = 0.f;
 #pragma unroll
-                    for (int r = 0; r < 3; ++r) Q[r] = q[r] + ((float)ox * Ad[3 * r] + (float)oy * Ad[3 * r + 1]);
+                    for (int r = 0; r < 3; ++r) Q[r] = q[r] + ((float)(ox - 1) * Ad[3 * r] + (float)(oy - 1) * Ad[3 * r + 1]) - Ad[3 * r + 2];
 #pragma unroll
                     for (int oz = 0; oz < 3; ++oz) {
                         const float4 n = __ldg(nodes + (ox * R + oy) * R + oz);
@@ -900,9 +906,9 @@ __global__ void __launch_bounds__(kThreads, 6) k_adj_p2g(AdjParams P, BkState in
                         const float p[4] = {n.x, n.y, n.z, n.w};
 #pragma unroll
                         for (int r = 0; r < 4; ++r) Sy[r] += w * p[r];
-                        if (oz)
+                        if (oz != 1)
 #pragma unroll
-                            for (int r = 0; r < 3; ++r) Zy[r] += ((float)oz * w) * p[r];
+                            for (int r = 0; r < 3; ++r) Zy[r] += ((float)(oz - 1) * w) * p[r];
 #pragma unroll
                         for (int r = 0; r < 3; ++r) Q[r] += Ad[3 * r + 2];
                     }
@@ -914,7 +920,7 @@ __global__ void __launch_bounds__(kThreads, 6) k_adj_p2g(AdjParams P, BkState in
                     for (int r = 0; r < 4; ++r) Sx[r] += w * Sy[r];
 #pragma unroll
                     for (int r = 0; r < 3; ++r) {
-                        if (oy) My[r] += ((float)oy * w) * Sy[r];
+                        if (oy != 1) My[r] += ((float)(oy - 1) * w) * Sy[r];
                         Mz[r] += w * Zy[r];
                     }
                 }
@@ -926,7 +932,7 @@ __global__ void __launch_bounds__(kThreads, 6) k_adj_p2g(AdjParams P, BkState in
                 for (int r = 0; r < 4; ++r) S[r] += w * Sx[r];
 #pragma unroll
                 for (int r = 0; r < 3; ++r) {
-                    M[3 * r] += ((float)ox * w) * Sx[r];
+                    M[3 * r] += ((float)(ox - 1) * w) * Sx[r];
                     M[3 * r + 1] += w * My[r];
                     M[3 * r + 2] += w * Mz[r];
                 }
@@ -938,7 +944,7 @@ __global__ void __launch_bounds__(kThreads, 6) k_adj_p2g(AdjParams P, BkState in
                 vb[r] = m * S[r];
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
-                    Ab[3 * r + c] = P.dx * (M[3 * r + c] - st.l[c] * S[r]);
+                    Ab[3 * r + c] = P.dx * (M[3 * r + c] - (st.l[c] - 1.f) * S[r]);
                     mb += Cm.m[3 * r + c] * Ab[3 * r + c];
                 }
             }
