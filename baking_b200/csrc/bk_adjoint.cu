@@ -766,7 +766,7 @@ __global__ void __launch_bounds__(kThreads, 7) k_adj_g2p_scatter(AdjParams P, Bk
 #pragma unroll
         for (int c = 0; c < 3; ++c) in_adj.x[c * pitch + i] = 0.f;
     }
-    scatter_momentum(sm[threadIdx.x >> 5], valid, st, 0.f, q, A, grid_v_adj, P.R, group_lanes(P.n, P.R));
+    scatter_momentum(sm, valid, st, 0.f, q, A, grid_v_adj, P.R, group_lanes(P.n, P.R), false);
 }
 
 // ------------------------------------------------------------- grid update

@@ -5,7 +5,7 @@
 // its 27 node weights (w_x w_y) w_z, as the reference rounds them, and its values in the warp's
 // record in shared memory; the run is then summed over its particles and every node receives one
 // atomic per run (one 16-byte vector atomic for momentum and mass). Nothing is shared between
-// warps, so a block has no barrier.
+// warps, so a block has no barrier (large bodies: merge_runs, below).
 //
 // What bounds it, and why there is no block tile: a shared-memory tile over the block's node box
 // (summing the block's runs before one global atomic per node) needs three block barriers, the
@@ -135,6 +135,17 @@ constexpr int64_t kGroupParticles = 256;
 
 BK_DEV bool group_lanes(int64_t n, int R) { return n >= kGroupParticles && R <= 1024; }
 
+// Bodies of this many particles (same grids) merge the momentum runs of a block before they reach the
+// grid. A particle that has just crossed into another cell gives that cell's far nodes weights of 1e-6
+// and less; sent alone, such a sum is below half a unit of a node's last place and lost: 20 substeps
+// after a 1M loaf's particles were ordered its grid mass lacks 1.0e-8 of itself, with blocks of 128
+// merged 0.45e-8, of 256 (the earlier node tile) 0.33e-8. It costs 12 of 88 us of P2G at 1M particles and 2.5 of 19
+// at 200k. Below 65536 particles the share lost hides under the random error of so few node sums, and the
+// merge's two barriers would cost 7 us of a substep that takes 50 (9k particles).
+constexpr int64_t kMergeParticles = 65536;
+
+BK_DEV bool merge_blocks(int64_t n, int R) { return n >= kMergeParticles && R <= 1024; }
+
 BK_DEV Runs find_runs(bool valid, const int* b, bool group) {
     const int lane = threadIdx.x & 31;
     const int p0 = __shfl_up_sync(kWarp, b[0], 1), p1 = __shfl_up_sync(kWarp, b[1], 1),
@@ -215,30 +226,102 @@ struct MomentumRecord {
     int64_t corner[32];  // the stencil's first node (a run reads its start's: one broadcast, no shuffles)
     float a8[32];
     float w[27][33];
+    unsigned key[32];              // the stencil base, 10 bits an axis
+    unsigned base[kGroupRuns];     // of the runs kept for the block
+    int kept;
 };
 
-// (The adjoint of G2P has the same form with m = 0.)
-BK_DEV void scatter_momentum(MomentumRecord& rec, bool valid, const Stencil& st, float m, const float* q,
-                             const float* A, float4* __restrict__ nodes, int R, bool group) {
+BK_DEV unsigned pack_base(int x, int y, int z) { return (unsigned)(x << 20 | y << 10 | z); }
+
+// The block's kept runs, summed in a tile over their node box and sent to L2 as one atomic per node. Warp
+// c sums component c, run by run in the order of the block's particles, in the space of its particles'
+// values (no shared atomics: no two warps touch a word).
+constexpr int kMergeNodes = 384;
+
+BK_DEV void merge_runs(MomentumRecord* sm, float4* __restrict__ nodes, int R) {
+    static_assert(sizeof(MomentumRecord::val) >= kMergeNodes * sizeof(float) && kGroupRuns == 8, "tile and slots");
+    const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
+    __syncthreads();
+    const int from = lane >> 3, slot = lane & 7;
+    const bool kept = slot < sm[from].kept;
+    const unsigned mask = __ballot_sync(kWarp, kept);
+    if (!mask) return;  // the same for every warp
+    const unsigned b = kept ? sm[from].base[slot] : 0u;
+    int lo[3], ext[3], at[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        at[a] = (int)(b >> (20 - 10 * a)) & 1023;
+        lo[a] = __reduce_min_sync(kWarp, kept ? at[a] : 1024);
+        ext[a] = __reduce_max_sync(kWarp, kept ? at[a] : 0) + 3 - lo[a];
+    }
+    const int count = ext[0] * ext[1] * ext[2];
+    int ox, oy, oz;
+    node_offset(lane < 27 ? lane : 0, ox, oy, oz);
+    if (count <= kMergeNodes) {
+        float* const tile = reinterpret_cast<float*>(sm[c].val);
+        for (int t = lane; t < count; t += 32) tile[t] = 0.f;
+        const int corner = ((at[0] - lo[0]) * ext[1] + at[1] - lo[1]) * ext[2] + at[2] - lo[2];
+        float* const mine = tile + (ox * ext[1] + oy) * ext[2] + oz;
+        const int row = 33 * (lane < 27 ? lane : 0) + c;
+        __syncwarp();
+        for (unsigned left = mask; left; left &= left - 1) {
+            const int l = __ffs(left) - 1;
+            const int first = __shfl_sync(kWarp, corner, l);
+            if (lane < 27) mine[first] += (&sm[l >> 3].w[0][0])[row + 4 * (l & 7)];
+            __syncwarp();
+        }
+        __syncthreads();
+        // (exact quotients: t * ext < 2^16, since both other extents are at least 3)
+        const unsigned by_z = (unsigned)__fdividef(65536.f, (float)ext[2]) + 1u, by_y = (unsigned)__fdividef(65536.f, (float)ext[1]) + 1u;
+        for (int t = threadIdx.x; t < count; t += 128) {
+            const float4 sum = make_float4(reinterpret_cast<const float*>(sm[0].val)[t], reinterpret_cast<const float*>(sm[1].val)[t],
+                                           reinterpret_cast<const float*>(sm[2].val)[t], reinterpret_cast<const float*>(sm[3].val)[t]);
+            if (sum.x == 0.f && sum.y == 0.f && sum.z == 0.f && sum.w == 0.f) continue;
+            const int yx = (int)((unsigned)t * by_z >> 16), x = (int)((unsigned)yx * by_y >> 16);
+            const int y = yx - x * ext[1], z = t - yx * ext[2];
+            atomicAdd(nodes + node_index(lo[0] + x, lo[1] + y, lo[2] + z, R), sum);
+        }
+    } else if (lane < 27) {  // far apart: each warp its own runs
+        const MomentumRecord& rec = sm[c];
+        for (int k = 0; k < rec.kept; ++k) {
+            const unsigned a = rec.base[k];
+            const float* v = rec.w[lane] + 4 * k;
+            atomicAdd(nodes + node_index((int)(a >> 20) + ox, (int)(a >> 10 & 1023) + oy, (int)(a & 1023) + oz, R),
+                      make_float4(v[0], v[1], v[2], v[3]));
+        }
+    }
+}
+
+// (The adjoint of G2P has the same form with m = 0.) With `merge` every warp of a block of 128
+// threads calls it; `group` and
+// `merge` are the same for all of them.
+BK_DEV void scatter_momentum(MomentumRecord* sm, bool valid, const Stencil& st, float m, const float* q,
+                             const float* A, float4* __restrict__ nodes, int R, bool group, bool merge) {
     const int lane = threadIdx.x & 31;
+    MomentumRecord& rec = sm[threadIdx.x >> 5];
     const Runs runs = find_runs(valid, st.b, group);
+    const bool keep = merge && __popc(runs.starts) < kGroupRuns;
+    int kept = 0;
     put_weights(rec.w, runs.column, valid, st);
     rec.val[runs.column][0] = make_float4(m, q[0], q[1], q[2]);
     rec.val[runs.column][1] = make_float4(A[0], A[1], A[2], A[3]);
     rec.val[runs.column][2] = make_float4(A[4], A[5], A[6], A[7]);
     rec.a8[runs.column] = A[8];
     rec.corner[runs.column] = node_index(st.b[0], st.b[1], st.b[2], R);
+    if (merge) rec.key[runs.column] = pack_base(st.b[0], st.b[1], st.b[2]);
     __syncwarp();
     int ox, oy, oz;
     node_offset(lane < 27 ? lane : 0, ox, oy, oz);
     const float fo[3] = {(float)ox, (float)oy, (float)oz};
-    const float* wj = rec.w[lane < 27 ? lane : 0];
+    float* const wj = rec.w[lane < 27 ? lane : 0];
     float4* const mine = nodes + ((int64_t)ox * R + oy) * R + oz;
     unsigned starts = runs.starts;
     while (starts) {
         const int s = __ffs(starts) - 1;
         starts &= starts - 1;
         const int e = run_end(starts);
+        // A kept run's sums take the weights' place: row j is read by lane j only, columns below e no more.
+        const bool here = keep && 4 * (kept + 1) <= e;
         if (lane < 27) {
             float2 mq0 = {0.f, 0.f}, q12 = {0.f, 0.f}, A01 = {0.f, 0.f}, A23 = {0.f, 0.f};
             float2 A45 = {0.f, 0.f}, A67 = {0.f, 0.f};
@@ -262,8 +345,23 @@ BK_DEV void scatter_momentum(MomentumRecord& rec, bool valid, const Stencil& st,
 #pragma unroll
             for (int r = 0; r < 3; ++r)
                 ap[r] = aq[r] + (aA[3 * r] * fo[0] + aA[3 * r + 1] * fo[1] + aA[3 * r + 2] * fo[2]);
-            atomicAdd(mine + rec.corner[s], make_float4(ap[0], ap[1], ap[2], mq0.x));
+            if (here) {
+                wj[4 * kept] = ap[0];
+                wj[4 * kept + 1] = ap[1];
+                wj[4 * kept + 2] = ap[2];
+                wj[4 * kept + 3] = mq0.x;
+            } else {
+                atomicAdd(mine + rec.corner[s], make_float4(ap[0], ap[1], ap[2], mq0.x));
+            }
         }
+        if (here) {
+            if (lane == 0) rec.base[kept] = rec.key[s];
+            ++kept;
+        }
+    }
+    if (merge) {
+        if (lane == 0) rec.kept = kept;
+        merge_runs(sm, nodes, R);
     }
 }
 

@@ -2,14 +2,16 @@
 //
 // The reference runs ~16 Warp launches per substep (physics/mpm.py:163-225,
 // physics/thermal_water.py:296-367) with three host synchronisations and fresh
-// dense-grid allocations. Here one substep is eight launches, clear_previous (which zeroes the last
-// substep's momentum box) and these seven:
+// dense-grid allocations. Here one substep is seven bodies in six launches (four without transport):
 //
 //   surface_vertices   rebuild only the boundary-face vertices (a block of 32-256 threads per
 //                      vertex, sized by its mean particle bindings)
 //   surface_owners     face areas -> boundary heat/loss/exchange of face-owning particles, scattered
-//   transport_scatter  scalar P2G (volume, capacity, energy, water), warp-cooperative per stencil base
-//   diffuse            7-point finite-volume heat/water flux over the active node box only
+//   transport_scatter  scalar P2G (volume, capacity, energy, water), warp-cooperative per stencil base;
+//                      its blocks are spread among those of the vertices of a coarse mesh, or of the
+//                      owners of a fine one (launch_substep)
+//   diffuse            7-point finite-volume heat/water flux over the active node box only; its blocks
+//                      also zero the last substep's momentum box (a launch of its own without transport)
 //   p2g                scalar G2P + gas source + gas/water stress + momentum P2G, fused per particle
 //   grid_update        momentum -> velocity with walls over the active box; zeroes the scatter fields
 //   g2p_return         G2P (v, C, x, F) fused with the Ding return map (float64 SVD in registers)
@@ -847,7 +849,7 @@ __device__ __forceinline__ void p2g_body(Arg<Params, kRef> P, Arg<BkState, kRef>
 #pragma unroll
         for (int e = 0; e < 9; ++e) A[e] *= P.dx;
     }
-    scatter_momentum(sm[threadIdx.x >> 5], valid, st, mass, q, A, g.pm, P.R, group_lanes(P.n, P.R));
+    scatter_momentum(sm, valid, st, mass, q, A, g.pm, P.R, group_lanes(P.n, P.R), merge_blocks(P.n, P.R));
 }
 
 template <bool kLoaf = false>
