@@ -139,8 +139,8 @@ BK_DEV bool group_lanes(int64_t n, int R) { return n >= kGroupParticles && R <= 
 // grid. A particle that has just crossed into another cell gives that cell's far nodes weights of 1e-6
 // and less; sent alone, such a sum is below half a unit of a node's last place and lost: 20 substeps
 // after a 1M loaf's particles were ordered its grid mass lacks 1.0e-8 of itself, with blocks of 128
-// merged 0.45e-8, of 256 (the earlier node tile) 0.33e-8. It costs 12 of 88 us of P2G at 1M particles and 2.5 of 19
-// at 200k. Below 65536 particles the share lost hides under the random error of so few node sums, and the
+// merged 0.45e-8, of 256 (the earlier node tile) 0.33e-8. It costs 13.5 us of a substep of 1M particles (P2G 76 to 90)
+// and 5 at 200k. Below 65536 particles the share lost hides under the random error of so few node sums, and the
 // merge's two barriers would cost 7 us of a substep that takes 50 (9k particles).
 constexpr int64_t kMergeParticles = 65536;
 
@@ -235,7 +235,7 @@ BK_DEV unsigned pack_base(int x, int y, int z) { return (unsigned)(x << 20 | y <
 
 // The block's kept runs, summed in a tile over their node box and sent to L2 as one atomic per node. Warp
 // c sums component c, run by run in the order of the block's particles, in the space of its particles'
-// values (no shared atomics: no two warps touch a word).
+// values (no shared atomics: no two warps touch a word; with a thread per node looping over the runs 18 us).
 constexpr int kMergeNodes = 384;
 
 BK_DEV void merge_runs(MomentumRecord* sm, float4* __restrict__ nodes, int R) {

@@ -720,8 +720,8 @@ __global__ void k_grid_update(Params P, GridPtrs g) {
 // (69% of its peak at 1M particles: the run loop's broadcasts and the node gather) and by the loads'
 // latency behind it. Loads are plain: staging the block's planes by bulk copies (33 KB and two
 // barriers a block) took 87.0 us where this form, with its L2 prefetch and no barrier, takes 82.
-// Blocks of 128 against 256: 81.8 and 84.2 us at 1M particles (no barrier spans a block, so the size
-// only sets how early a finished block's slot is refilled).
+// Blocks of 128 against 256: 81.8 and 84.2 us at 1M particles (a finished block's slot is refilled
+// earlier). The merge of large bodies' runs (merge_runs) and its barriers come on top.
 constexpr int kP2GThreads = 128;
 
 template <bool kRef = false>
