@@ -61,6 +61,7 @@ struct Params {
     float ambient, density, elastic_modulus, cfl, peak, width;
     int keep_fields;
     int prescattered, prescatter_next, prescatter_stale;
+    int box_widened;  // the launches before P2G in this call widen the node box over the same positions
     int32_t* status;
 };
 
@@ -84,6 +85,7 @@ Params to_params(const BkSubstepParams& p) {
     k.prescattered = p.transport_prescattered;
     k.prescatter_next = p.transport_prescatter_next;
     k.prescatter_stale = p.transport_prescatter_stale;
+    k.box_widened = 0;
     k.status = p.status;
     return k;
 }
@@ -761,8 +763,7 @@ __device__ __forceinline__ void p2g_body(Arg<Params, kRef> P, Arg<BkState, kRef>
         valid = st.valid;
         if (!valid) set_flag(flags.simulation, 1);
     }
-    // The transport scatter of this substep has widened the box over the same positions already.
-    if (!P.transport || P.prescattered) widen_box(g.bounds, valid, st.b);
+    if (!P.box_widened) widen_box(g.bounds, valid, st.b);
     float mass = 0.f, q[3] = {0.f, 0.f, 0.f}, A[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (valid) {
         M3 F = load_m3(in.F, i, pitch);
@@ -1374,8 +1375,8 @@ int check_substep_args(const BkSubstepParams* params, const BkState* in, const B
 }
 
 
-// The launches of one substep (or of its phases); P carries this substep's prescatter flags.
-int launch_substep(const BkSubstepParams& p, const Params& P, const GridPtrs& g, const BkState& in, const BkState& out,
+// The launches of one substep (or of its phases); `with_flags` carries this substep's prescatter flags.
+int launch_substep(const BkSubstepParams& p, const Params& with_flags, const GridPtrs& g, const BkState& in, const BkState& out,
                    const BkConstants& constants, const BkSurface* surface, const BkDiagnostics& diagnostics,
                    const BkFlags& flags, int32_t phases, int sms, cudaStream_t s) {
     const bool loaf = loaf_mode(p, diagnostics);
@@ -1384,6 +1385,10 @@ int launch_substep(const BkSubstepParams& p, const Params& P, const GridPtrs& g,
     // first SMs to drain: P2G of a 9k-particle sphere took 16 us after 592 diffusion blocks.
     const unsigned box_blocks = (unsigned)std::min<int64_t>((int64_t)sms * 4, (p.n + 127) / 128);
     const bool transport = (phases & BK_PHASE_TRANSPORT) && p.transport;
+    // P2G leaves the node box to the transport scatter only where this call launches it: a mechanics phase
+    // by itself, or one on fields scattered ahead (their box is another), finds the box empty.
+    Params P = with_flags;
+    P.box_widened = transport && !P.prescattered;
     cudaError_t e = cudaSuccess;
     if (transport) {
         const unsigned scatter_blocks = P.prescattered ? 0u : blocks_for(p.n, kOwnerThreads);
@@ -1614,6 +1619,7 @@ struct BatchArgs {
     const int32_t* owner;       // the instance of every block of every stage, stage by stage
     uint32_t owner_offset[kBatchStages];  // where each stage's blocks start in `owner`
     int count, parity, prescattered, prescatter_next;
+    int scatters;  // the call has a transport phase
 };
 
 // The instance that owns this block in `stage` (one load from the block map) and the block's slot
@@ -1638,6 +1644,7 @@ __device__ __forceinline__ Slot batch_load(const BatchArgs& b, int stage, BatchE
         e.P.prescattered = b.prescattered && e.prescatter_ok;
         e.P.prescatter_next = b.prescatter_next && e.prescatter_ok;
         e.P.prescatter_stale = 0;
+        e.P.box_widened = b.scatters && e.P.transport && !e.P.prescattered;
     }
     __syncthreads();
     return sl;
@@ -1845,6 +1852,7 @@ int bk_batch_substep(BkBatch* batch, int32_t parity, int32_t phases, int32_t pre
     a.parity = parity;
     a.prescattered = prescattered ? 1 : 0;
     a.prescatter_next = prescatter_next ? 1 : 0;
+    a.scatters = phases & BK_PHASE_TRANSPORT ? 1 : 0;
     const uint32_t* T = B.total;
     cudaStream_t s = S(stream);
     if ((phases & BK_PHASE_TRANSPORT) && B.any_transport) {

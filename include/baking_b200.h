@@ -317,7 +317,9 @@ typedef struct BkSubstepParams {
 #define BK_PHASE_TRANSPORT 1       /* surface terms, scalar P2G, diffusion */
 #define BK_PHASE_MECHANICS 2       /* scalar G2P + gas/water stress + P2G, grid update, G2P + return map */
 
-/* The fused substep of physics/mpm.py:163-225: reads `in`, writes `out`, uses `grid` as scratch. */
+/* The fused substep of physics/mpm.py:163-225: reads `in`, writes `out`, uses `grid` as scratch. The
+   phases may come from separate calls, with nothing changed in between; a mechanics phase with
+   transport on reads whatever node_dT_ratio holds, whether or not a transport phase went before it. */
 BK_API int bk_substep(const BkSubstepParams *params, const BkState *in, BkState *out, const BkConstants *constants,
                       BkGrid *grid, BkSurface *surface, BkDiagnostics *diagnostics, BkFlags *flags,
                       int32_t phases, void *stream);
