@@ -725,13 +725,18 @@ __global__ void k_grid_update(Params P, GridPtrs g) {
 // Blocks of 128 against 256: 81.8 and 84.2 us at 1M particles (a finished block's slot is refilled
 // earlier). The merge of large bodies' runs (merge_runs) and its barriers come on top.
 constexpr int kP2GThreads = 128;
+// Bodies of at most this many particles are one block, whose warps send their sums in step after a
+// barrier: the atomics of a node leave one SM in the same order each time, and a run repeats bit for bit
+// (160 runs of a 192-particle body; with two blocks of 128, or without the barrier, 1 in 8 differed, and
+// finite differences of such a body carried that noise). The time is the same (17 us).
+constexpr int kP2GSmall = 256;
 
-template <bool kRef = false>
+template <bool kRef = false, int kBlock = kP2GThreads>
 __device__ __forceinline__ void p2g_body(Arg<Params, kRef> P, Arg<BkState, kRef> in, Arg<BkState, kRef> out,
                                          Arg<BkConstants, kRef> cst, Arg<GridPtrs, kRef> g, Arg<BkFlags, kRef> flags,
                                          float* max_residuals, Slot sl) {
-    __shared__ MomentumRecord sm[kP2GThreads / 32];
-    const int64_t i = sl.block * (int64_t)kP2GThreads + threadIdx.x;
+    __shared__ MomentumRecord sm[kBlock / 32];
+    const int64_t i = sl.block * (int64_t)kBlock + threadIdx.x;
     const int64_t pitch = P.pitch;
     {
         // v, C, F and tau planes by lane, then the scalars' lines (two per float64 array)
@@ -850,14 +855,15 @@ __device__ __forceinline__ void p2g_body(Arg<Params, kRef> P, Arg<BkState, kRef>
 #pragma unroll
         for (int e = 0; e < 9; ++e) A[e] *= P.dx;
     }
+    if constexpr (kBlock == kP2GSmall) __syncthreads();  // the warps send their sums in step (kP2GSmall)
     scatter_momentum(sm, valid, st, mass, q, A, g.pm, P.R, group_lanes(P.n, P.R), merge_blocks(P.n, P.R));
 }
 
-template <bool kLoaf = false>
-__global__ void __launch_bounds__(kP2GThreads, 8) k_p2g(Params P, BkState in, BkState out, BkConstants cst, GridPtrs g,
+template <bool kLoaf = false, int kBlock = kP2GThreads>
+__global__ void __launch_bounds__(kBlock, 1024 / kBlock) k_p2g(Params P, BkState in, BkState out, BkConstants cst, GridPtrs g,
                                                  BkFlags flags, float* max_residuals) {
     if constexpr (kLoaf) fix_loaf_mode(P);
-    p2g_body(P, in, out, cst, g, flags, max_residuals, grid_slot());
+    p2g_body<false, kBlock>(P, in, out, cst, g, flags, max_residuals, grid_slot());
 }
 
 // ------------------------------------------------------ fused G2P + return
@@ -1461,8 +1467,11 @@ int launch_substep(const BkSubstepParams& p, const Params& with_flags, const Gri
         }
         {
             const int rec = profile_begin("p2g", s);
-            e = launch_chained(loaf ? k_p2g<true> : k_p2g<false>, blocks_for(p.n, kP2GThreads), kP2GThreads, 0, s, P, in,
-                               out, constants, g, flags, diagnostics.max_residuals);
+            const int threads = p.n <= kP2GSmall ? kP2GSmall : kP2GThreads;
+            auto* kernel = p.n <= kP2GSmall ? (loaf ? k_p2g<true, kP2GSmall> : k_p2g<false, kP2GSmall>)
+                                            : (loaf ? k_p2g<true> : k_p2g<false>);
+            e = launch_chained(kernel, blocks_for(p.n, threads), threads, 0, s, P, in, out, constants, g, flags,
+                               diagnostics.max_residuals);
             profile_end(rec, s);
             if (int rc = check_chained(e, "bk_substep/p2g")) return rc;
         }
