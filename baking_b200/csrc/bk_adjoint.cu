@@ -1073,9 +1073,7 @@ int bk_substep_adjoint(const BkSubstepParams* params, const BkState* in, const B
         int device = 0, sms = 148;
         cudaGetDevice(&device);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        // as bk_substep's node-box passes: fewer blocks for small bodies
-        const int64_t box_blocks = p.n / 128 + 1 < (int64_t)sms * 4 ? p.n / 128 + 1 : (int64_t)sms * 4;
-        e = launch_chained(k_adj_grid_box, (unsigned)box_blocks, 256, 0, s, a, node_box,
+        e = launch_chained(k_adj_grid_box, node_box_blocks(p.n, p.resolution, sms), 256, 0, s, a, node_box,
                            reinterpret_cast<const float4*>(node_pm), reinterpret_cast<float4*>(node_v_adjoint),
                            reinterpret_cast<float4*>(node_pm_adjoint));
     } else {

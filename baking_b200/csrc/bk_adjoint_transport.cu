@@ -781,8 +781,7 @@ int bk_transport_adjoint(const BkSubstepParams* params, const BkState* in, const
     int device = 0, sms = 148;
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    // as bk_substep's node-box passes: fewer blocks for small bodies
-    const unsigned box_blocks = p.n / 128 + 1 < (int64_t)sms * 4 ? (unsigned)(p.n / 128 + 1) : (unsigned)sms * 4;
+    const unsigned box_blocks = node_box_blocks(p.n, p.resolution, sms);
     cudaError_t e = launch_chained(k_tadj_scalar, blocks(p.n, kThreads), kThreads, 0, s, P, *in, *constants,
                                    reinterpret_cast<const double2*>(grid->node_dT_ratio), a, *mechanics, g.dTr_bar);
     if (int rc = check_chained(e, "bk_transport_adjoint/scalar")) return rc;

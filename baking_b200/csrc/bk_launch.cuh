@@ -9,6 +9,8 @@
 // warm (elastic body of 41k particles 920 -> 872 us a 40-substep pass, 9k sphere 2106 -> 2049).
 #pragma once
 
+#include <algorithm>
+#include <cstdint>
 #include <cstdio>
 #include <utility>
 
@@ -22,6 +24,17 @@ __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Blocks of a pass over the node box, whose size only the device knows: up to four per SM. A compact body
+// is best served by one per 128 particles (9k sphere, 69 blocks: 46.9 us a substep, 49.6 with three per SM,
+// 51.2 with four; 41k cube, 324 blocks: 22.3, with three per SM 24.3: the next kernel's blocks find emptier
+// SMs), but a box may hold far more nodes than particles, up to the whole grid. So small bodies take three
+// per SM where the grid has that many tiles of 256 nodes: two clumps of 324 particles across a 128^3 grid
+// take 101 us a substep (two per SM: 112, four: 99; a block per 128 particles: 2000).
+inline unsigned node_box_blocks(int64_t n, int resolution, int sms) {
+    const int64_t grid = ((int64_t)resolution * resolution * resolution + 255) / 256;
+    const int64_t few = std::max<int64_t>(std::min<int64_t>(grid, (int64_t)sms * 3), (n + 127) / 128);
+    return (unsigned)std::min<int64_t>((int64_t)sms * 4, few);
+}
 
 // The status of a launch_chained call, as check_launch reports a launch's.
 inline int check_chained(cudaError_t e, const char* name) {

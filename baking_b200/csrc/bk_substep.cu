@@ -1386,10 +1386,7 @@ int launch_substep(const BkSubstepParams& p, const Params& with_flags, const Gri
                    const BkConstants& constants, const BkSurface* surface, const BkDiagnostics& diagnostics,
                    const BkFlags& flags, int32_t phases, int sms, cudaStream_t s) {
     const bool loaf = loaf_mode(p, diagnostics);
-    // Node-box passes: four blocks per SM, or for small bodies a block per 128 particles. A full grid of
-    // them leaves no registers free for the next kernel's few blocks, which then start packed on the
-    // first SMs to drain: P2G of a 9k-particle sphere took 16 us after 592 diffusion blocks.
-    const unsigned box_blocks = (unsigned)std::min<int64_t>((int64_t)sms * 4, (p.n + 127) / 128);
+    const unsigned box_blocks = node_box_blocks(p.n, p.resolution, sms);
     const bool transport = (phases & BK_PHASE_TRANSPORT) && p.transport;
     // P2G leaves the node box to the transport scatter only where this call launches it: a mechanics phase
     // by itself, or one on fields scattered ahead (their box is another), finds the box empty.

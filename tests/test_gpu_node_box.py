@@ -86,3 +86,32 @@ def test_mechanics_alone_on_a_fresh_grid(table):
         b.Step()
     a._stale = True
     compare(a, b)
+
+
+@pytest.mark.parametrize("subdivisions", [1, 3])
+def test_passes_over_a_sparse_box(subdivisions):
+    """Two halves of a small cube in far corners: the node box holds thousands of nodes for every
+    particle, and its passes are shared by enough blocks that a substep stays within 8 times that
+    of the compact cube (the box passes move some 100 MB: two substeps' time; with blocks counted by
+    particles it took 30 times)."""
+    import torch
+    times = []
+    for apart in (0.0, 0.25):
+        sim, _ = baking_cube("cuda", subdivisions=subdivisions, gravity=(0., 0., 0.), dt=1e-6)
+        sim = type(sim)(sim.tet_mesh, sim.particle_samples, replace(sim.simulation_config, grid_resolution=128,
+                                                                    grid_spacing=1.0 / 128),
+                        sim.material.material_config, ding_config=sim.material.ding_config,
+                        transport_config=sim.transport.config, diagnostics="lean")
+        x, half = sim.current_state.particle_positions, sim.particle_data.particle_count // 2
+        x[:half] += apart
+        x[half:] -= apart
+        best = float("inf")
+        for _ in range(4):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            sim.AdvanceUnchecked(20)
+            end.record()
+            torch.cuda.synchronize()
+            best = min(best, start.elapsed_time(end))
+        times.append(best)
+    assert times[1] <= 8.0 * times[0], times
