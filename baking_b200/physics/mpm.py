@@ -16,6 +16,7 @@ first substep whose flags were set.
 from __future__ import annotations
 
 import math
+import operator
 from dataclasses import fields, replace
 from pathlib import Path
 
@@ -510,6 +511,7 @@ class MpmSimulator:
         return messages
 
     def Advance(self, step_count):
+        step_count = operator.index(step_count)  # a whole number, as range() takes it
         if step_count < 1:
             raise ValueError("step_count must be positive")
         start = self.step_count
@@ -542,7 +544,7 @@ class MpmSimulator:
         With ``scatter_ahead`` set, each substep's G2P within the call scatters the next substep's
         transport fields ahead."""
         ahead = self.scatter_ahead and self._engine.prescatter_allowed()
-        self._unchecked_substeps(step_count, ahead)
+        self._unchecked_substeps(operator.index(step_count), ahead)
 
     def StepSummary(self, out=None):
         """Device tensor (grid mass of the last substep, particle kinetic energy of the current
