@@ -1499,6 +1499,8 @@ int launch_substep(const BkSubstepParams& p, const Params& with_flags, const Gri
     return BK_OK;
 }
 
+thread_local int32_t substeps_launched = 0;  // by this thread's last bk_substeps call
+
 int sm_count() {
     int device = 0, sms = 148;
     cudaGetDevice(&device);
@@ -1523,6 +1525,7 @@ int bk_substeps(const BkSubstepParams* params, const BkState* states, double* co
                 double* const* heat_exchanges, const BkConstants* constants, BkGrid* grid, const BkSurface* surface,
                 const BkDiagnostics* diagnostics, BkFlags* flags, int32_t count, int32_t scatter_ahead, void* stream) {
     const int32_t phases = BK_PHASE_TRANSPORT | BK_PHASE_MECHANICS;
+    substeps_launched = 0;
     BK_REQUIRE(states && diagnostics && count >= 0, "bk_substeps: null argument or negative count");
     BK_REQUIRE(params && !params->transport_prescattered && !params->transport_prescatter_next,
                "bk_substeps: the call sets the prescatter flags itself");
@@ -1554,9 +1557,12 @@ int bk_substeps(const BkSubstepParams* params, const BkState* states, double* co
         if (int rc = launch_substep(p, P, g, states[from], states[to], *constants, &sf, diagnostics[to], *flags, phases, sms,
                                     S(stream)))
             return rc;
+        ++substeps_launched;
     }
     return BK_OK;
 }
+
+int bk_substeps_launched(void) { return substeps_launched; }
 
 int bk_surface_accumulate(const BkSurface* surface, float time_step, double* water_losses, double* heat_exchanges,
                           void* stream) {

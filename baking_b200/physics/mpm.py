@@ -465,28 +465,39 @@ class MpmSimulator:
         if self.sort_interval and self.step_count % self.sort_interval == 0:
             self.SortParticles()
 
+    # Most substeps launched from one library call: between calls an interrupt is served, and the state
+    # is a substep's.
+    _SUBSTEPS_PER_CALL = 64
+
     def _unchecked_substeps(self, count, ahead=False):
         """``count`` unchecked substeps. Past settling, and unless a state history or a recorder wants
-        to see each of them, the library launches them from one call (the host's work per substep was
+        to see each of them, the library launches them from few calls (the host's work per substep was
         more than a small body's substep takes on the device), in pieces that end where the particles
-        are re-sorted. ``ahead``: each substep scatters the next one's transport fields, to the last."""
+        are re-sorted. ``ahead``: each substep of a piece scatters the next one's transport fields, to
+        the last. A launch that fails leaves the last complete substep as the current state."""
         if self.IsSettling or self.retain_history or getattr(self, "result_recorder", None) is not None:
             for k in range(count):
                 self._substep(check=False, prescattered=ahead and k > 0, prescatter_next=ahead and k + 1 < count)
             return
         full = self.diagnostics == "full"
         while count > 0:
-            piece = count
+            piece = min(count, self._SUBSTEPS_PER_CALL)
             if self.sort_interval:
-                piece = min(count, self.sort_interval - self.step_count % self.sort_interval)
-            self._engine.run_many(self._current, self.next_state, piece, full, ahead)
-            if piece % 2:
+                piece = min(piece, self.sort_interval - self.step_count % self.sort_interval)
+            done, error = piece, None
+            try:
+                self._engine.run_many(self._current, self.next_state, piece, full, ahead)
+            except RuntimeError as failure:
+                done, error = getattr(failure, "launched", 0), failure
+            if done % 2:
                 self._current, self.next_state = self.next_state, self._current
-            self._stale = True
+            self._stale = self._stale or done > 0
+            self.step_count += done
+            if error is not None:
+                raise error
             if full:
                 self._engine.materialize(self._current, plastic=False)
                 self._stale = False
-            self.step_count += piece
             count -= piece
             if self.sort_interval and self.step_count % self.sort_interval == 0:
                 self.SortParticles()

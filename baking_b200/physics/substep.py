@@ -105,6 +105,7 @@ _SIGS = {
     "bk_check_state": [P, P, P, P],
     "bk_substep": [P] * 8 + [C.c_int32, P],
     "bk_substeps": [P] * 9 + [C.c_int32, C.c_int32, P],
+    "bk_substeps_launched": [],
     "bk_materialize": [P] * 11 + [P],
     "bk_surface_accumulate": [P, C.c_float, P, P, P],
     "bk_batch_create": [P, C.c_int32, P],
@@ -349,7 +350,8 @@ class SubstepEngine:
 
     def run_many(self, state, other, count, full_diagnostics, scatter_ahead=False):
         """``count`` unchecked substeps past settling, state -> other -> state ..., in one library call
-        (bk_substeps): what ``count`` runs with ``accumulate`` of the state written would launch."""
+        (bk_substeps): what ``count`` runs with ``accumulate`` of the state written would launch. An
+        error's ``launched`` says how many of them were launched before it."""
         p, cst = self.prepare(False)
         p.status = _p(self.status)
         p.transport_prescatter_stale = int(self.transport and self.prescatter_pending)
@@ -366,7 +368,9 @@ class SubstepEngine:
                                   C.byref(self.surface), diags, C.byref(self.flags), int(count), int(scatter_ahead),
                                   _lib.stream_handle())
         if rc != 0:
-            raise RuntimeError(f"bk_substeps failed ({rc}): {self.lib.bk_last_error().decode(errors='replace')}")
+            error = RuntimeError(f"bk_substeps failed ({rc}): {self.lib.bk_last_error().decode(errors='replace')}")
+            error.launched = int(self.lib.bk_substeps_launched())
+            raise error
 
     def run(self, state_in, state_out, settling, phases, full_diagnostics, grid=None, keep_fields=False,
             prescattered=False, prescatter_next=False, accumulate=None, prepared=None):

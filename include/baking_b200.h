@@ -335,6 +335,9 @@ BK_API int bk_substeps(const BkSubstepParams *params, const BkState *states, dou
                        double *const *heat_exchanges, const BkConstants *constants, BkGrid *grid,
                        const BkSurface *surface, const BkDiagnostics *diagnostics, BkFlags *flags, int32_t count,
                        int32_t scatter_ahead, void *stream);
+/* How many substeps the calling thread's last bk_substeps call launched completely: its count, or where
+   it failed, the substeps before the one that did (their result is in states[launched & 1]). */
+BK_API int bk_substeps_launched(void);
 
 /* bk_substep's mechanics phase with the grid held in a fixed array inside this library, for
    callers that must not allocate device memory (code inside an allocator hook, a real-time or

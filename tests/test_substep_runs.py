@@ -42,8 +42,18 @@ def test_pieces(count, sort_interval):
     sim = simulator(sort_interval)
     sim.AdvanceUnchecked(np.int64(count))
     assert sim.step_count == sim._current["steps"] == sum(sim._engine.calls) == count
+    assert max(sim._engine.calls, default=0) <= 64  # an interrupt waits for no more than that
     assert sim._stale == (count > 0)
     assert sim.sorts == [k for k in range(1, count + 1) if sort_interval and k % sort_interval == 0]
+
+
+@pytest.mark.parametrize("fail_at", [0, 1, 2, 63, 64, 67, 128])
+def test_a_failing_launch_leaves_the_last_complete_substep(fail_at):
+    sim = simulator(fail_at=fail_at)
+    with pytest.raises(RuntimeError, match="launch failed"):
+        sim.AdvanceUnchecked(130)
+    assert sim.step_count == sim._current["steps"] == fail_at
+    assert sim._stale == (fail_at > 0)
 
 
 @pytest.mark.parametrize("count", [2.5, 2.0, "2", None, np.float32(3)])
