@@ -383,7 +383,7 @@ __device__ void block_accumulate(double* target, float value) {
 // kCoupled: gas mode's coupled porosity (a separate instance, so the other modes keep their registers).
 // kLoaf: the loaf configuration (Ding with temperature, transport) as compile-time constants.
 template <bool kCoupled, bool kLoaf = false>
-__global__ void __launch_bounds__(kThreads, 4) k_adj_g2p_return(AdjParams P, BkState in, const float4* __restrict__ grid_v,
+__global__ void __launch_bounds__(kThreads, 4) k_adj_g2p_return(AdjParams P, BkState in, const float4* grid_v,
                                                           const float* __restrict__ eta_param, AdjState out_adj,
                                                           AdjState in_adj, double* __restrict__ params_adj) {
     if constexpr (kLoaf) fix_loaf_mode(P);
@@ -686,7 +686,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_adj_g2p_return(AdjParams P, BkS
 // operations a node where the plain double sum took 45; with the scatter by warp runs 128 -> 102 us at
 // 1M particles.
 template <bool kLoaf = false>
-__global__ void __launch_bounds__(kThreads, 7) k_adj_g2p_scatter(AdjParams P, BkState in, const float4* __restrict__ grid_v,
+__global__ void __launch_bounds__(kThreads, 7) k_adj_g2p_scatter(AdjParams P, BkState in, const float4* grid_v,
                                                             AdjState out_adj, AdjState in_adj,
                                                             float4* __restrict__ grid_v_adj) {
     if constexpr (kLoaf) fix_loaf_mode(P);
@@ -736,7 +736,7 @@ __global__ void __launch_bounds__(kThreads, 7) k_adj_g2p_scatter(AdjParams P, Bk
                 for (int r = 0; r < 3; ++r) Q[r] = qc[r] + ((float)(ox - 1) * A[3 * r] + (float)(oy - 1) * A[3 * r + 1]) - A[3 * r + 2];
 #pragma unroll
                 for (int oz = 0; oz < 3; ++oz) {
-                    const float4 u = __ldg(nodes + (ox * R + oy) * R + oz);
+                    const float4 u = nodes[(ox * R + oy) * R + oz];
                     const float s = u.x * Q[0] + u.y * Q[1] + u.z * Q[2];
                     s0 += st.w[2][oz] * s;
                     s1 += dw[2][oz] * s;
@@ -770,7 +770,7 @@ __global__ void __launch_bounds__(kThreads, 7) k_adj_g2p_scatter(AdjParams P, Bk
 }
 
 // ------------------------------------------------------------- grid update
-__device__ __forceinline__ void adj_grid_node(const AdjParams& P, const float4* __restrict__ pm,
+__device__ __forceinline__ void adj_grid_node(const AdjParams& P, const float4* pm,
                                               float4* __restrict__ grid_v_adj, float4* __restrict__ pm_adj,
                                               int64_t i, int c0, int c1, int c2, bool clear) {
     float4 a = grid_v_adj[i];
@@ -796,7 +796,7 @@ __device__ __forceinline__ void adj_grid_node(const AdjParams& P, const float4* 
 }
 
 // Every node of the grid (velocity adjoint zeroed beforehand by the caller of the substep).
-__global__ void k_adj_grid(AdjParams P, const float4* __restrict__ pm, float4* __restrict__ grid_v_adj,
+__global__ void k_adj_grid(AdjParams P, const float4* pm, float4* __restrict__ grid_v_adj,
                            float4* __restrict__ pm_adj, int64_t nodes) {
     pdl_enter();
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -807,7 +807,7 @@ __global__ void k_adj_grid(AdjParams P, const float4* __restrict__ pm, float4* _
 
 // The nodes of the forward substep's active box (inclusive lo[3], hi[3] on the device), which holds
 // every stencil node; the velocity adjoint is zeroed behind, so the next call finds it zero.
-__global__ void k_adj_grid_box(AdjParams P, const int32_t* __restrict__ box, const float4* __restrict__ pm,
+__global__ void k_adj_grid_box(AdjParams P, const int32_t* box, const float4* pm,
                                float4* __restrict__ grid_v_adj, float4* __restrict__ pm_adj) {
     pdl_enter();
     int lo[3], ext[3];
@@ -831,8 +831,8 @@ __global__ void k_adj_grid_box(AdjParams P, const int32_t* __restrict__ box, con
 // ---------------------------------------------------------------- P2G
 // tau is the Ding state stress, or the neo-Hookean stress of F.
 template <bool kLoaf = false>
-__global__ void __launch_bounds__(kThreads, 6) k_adj_p2g(AdjParams P, BkState in, const float* __restrict__ mass,
-                                                   const float* __restrict__ volume, const float4* __restrict__ pm_adj,
+__global__ void __launch_bounds__(kThreads, 6) k_adj_p2g(AdjParams P, BkState in, const float* mass,
+                                                   const float* __restrict__ volume, const float4* pm_adj,
                                                    AdjState in_adj, double* __restrict__ params_adj) {
     if constexpr (kLoaf) fix_loaf_mode(P);
     const int64_t i = blockIdx.x * (int64_t)kThreads + threadIdx.x;
@@ -898,7 +898,7 @@ __global__ void __launch_bounds__(kThreads, 6) k_adj_p2g(AdjParams P, BkState in
                     for (int r = 0; r < 3; ++r) Q[r] = q[r] + ((float)(ox - 1) * Ad[3 * r] + (float)(oy - 1) * Ad[3 * r + 1]) - Ad[3 * r + 2];
 #pragma unroll
                     for (int oz = 0; oz < 3; ++oz) {
-                        const float4 n = __ldg(nodes + (ox * R + oy) * R + oz);
+                        const float4 n = nodes[(ox * R + oy) * R + oz];
                         const float w = st.w[2][oz];
                         const float s = n.w * m + (n.x * Q[0] + n.y * Q[1] + n.z * Q[2]);
                         s0 += w * s;

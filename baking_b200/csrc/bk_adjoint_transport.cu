@@ -82,7 +82,7 @@ __device__ __forceinline__ double source_moles(const TParams& P, const BkState& 
 }
 
 // ------------------------------------------------------------------ prepare
-__global__ void k_tadj_prepare(TParams P, BkState in, BkConstants cst, const double2* __restrict__ dTr,
+__global__ void k_tadj_prepare(TParams P, BkState in, BkConstants cst, const double2* dTr,
                                float* __restrict__ T_mat, float* __restrict__ mass, float* __restrict__ tau_eff) {
     pdl_enter();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -122,7 +122,7 @@ __global__ void k_tadj_prepare(TParams P, BkState in, BkConstants cst, const dou
 // its gradients and a block tile per node and particle, now 133; it waits for memory (long_scoreboard 12
 // of 17 cycles an issue at 4 blocks per SM), so eight blocks per SM with a few spilled registers are faster.
 __global__ void __launch_bounds__(kThreads, 8) k_tadj_scalar(TParams P, BkState in, BkConstants cst,
-                                                        const double2* __restrict__ dTr, BkAdjointTransport a,
+                                                        const double2* dTr, BkAdjointTransport a,
                                                         const BkAdjointState adj, double2* __restrict__ dTr_bar) {
     __shared__ ScalarRecord<2> sm[kThreads / 32];
     const int tid = threadIdx.x, lane = tid & 31;
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(kThreads, 8) k_tadj_scalar(TParams P, BkState 
 #pragma unroll
                 for (int oz = 0; oz < 3; ++oz) {
                     const double wz = (double)st.w[2][oz], gz = (double)qweight_grad(st.l[2], oz);
-                    const double2 d = __ldg(nodes + (ox * R + oy) * R + oz);
+                    const double2 d = nodes[(ox * R + oy) * R + oz];
                     ty = fma(wz, d.x, ty);
                     ry = fma(wz, d.y, ry);
                     tg = fma(gz, d.x, tg);
@@ -271,7 +271,7 @@ __device__ __forceinline__ NodeVals node_vals(const TParams& P, double* const* f
     return n;
 }
 
-__global__ void k_tadj_diffuse(TParams P, BkGridFields g, const int32_t* __restrict__ box) {
+__global__ void k_tadj_diffuse(TParams P, BkGridFields g, const int32_t* box) {
     pdl_enter();
     int lo[3], ext[3];
     int64_t count = 1;
@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(kThreads, 7) k_tadj_scatter(TParams P, BkState
         }
     };
     if (count > 0) gather([&](int f, int64_t t) { return s_bar[f][t]; });
-    else gather([&](int f, int64_t t) { return __ldg(bar[f] + t); });
+    else gather([&](int f, int64_t t) { return bar[f][t]; });
     const double volb = v0, Tb = cap * v2, Wb = v3;
     float xg[3];
 #pragma unroll
@@ -477,8 +477,8 @@ template <int kBlock>
 constexpr int vertex_threads() { return kBlock == 32 ? 32 * kVertexWarps : kBlock; }
 
 template <int kBlock>
-__global__ void __launch_bounds__(vertex_threads<kBlock>()) k_tadj_vertex_positions(TParams P, const float* __restrict__ x,
-                                                                                const float* __restrict__ F, BkSurface sf) {
+__global__ void __launch_bounds__(vertex_threads<kBlock>()) k_tadj_vertex_positions(TParams P, const float* x,
+                                                                                const float* F, BkSurface sf) {
     pdl_enter();
     if constexpr (kBlock == 32) {
         const int64_t k = (int64_t)blockIdx.x * kVertexWarps + (threadIdx.x >> 5);
@@ -547,7 +547,7 @@ __device__ __forceinline__ double owner_reverse(const TParams& P, const BkState&
 #pragma unroll
             for (int oz = 0; oz < 3; ++oz) {
                 const int64_t node = corner + (ox * R + oy) * R + oz;
-                const double fh = __ldg(g.field_bar[4] + node), fl = __ldg(g.field_bar[5] + node);
+                const double fh = g.field_bar[4][node], fl = g.field_bar[5][node];
                 hy = fma((double)st.w[2][oz], fh, hy);
                 ly = fma((double)st.w[2][oz], fl, ly);
                 s1 = fma((double)qweight_grad(st.l[2], oz), heat * fh + loss * fl, s1);
@@ -678,7 +678,7 @@ __global__ void __launch_bounds__(vertex_threads<kBlock>()) k_tadj_vertices(TPar
 }
 
 // ------------------------------------------------------------------- clear
-__global__ void k_tadj_clear(TParams P, BkGridFields g, const int32_t* __restrict__ box) {
+__global__ void k_tadj_clear(TParams P, BkGridFields g, const int32_t* box) {
     pdl_enter();
     int lo[3], ext[3];
     int64_t count = 1;

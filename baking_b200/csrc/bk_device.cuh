@@ -61,20 +61,23 @@ BK_DEV double reciprocal_newton(double x) {
 }
 
 // ------------------------------------------------------------- SoA access
-BK_DEV V3 load_v3(const float* __restrict__ p, int64_t i, int64_t pitch) {
+// Plain loads, here and wherever a chained kernel (bk_launch.cuh) reads what the kernels before it write:
+// it starts while they still run, and the read-only path (__ldg, or a const __restrict__ kernel
+// parameter) asks for data that nothing writes while the kernel lives. Only constants take that path.
+BK_DEV V3 load_v3(const float* p, int64_t i, int64_t pitch) {
     V3 r;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) r.v[c] = __ldg(p + c * pitch + i);
+    for (int c = 0; c < 3; ++c) r.v[c] = p[c * pitch + i];
     return r;
 }
 BK_DEV void store_v3(float* __restrict__ p, int64_t i, int64_t pitch, const V3& a) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) p[c * pitch + i] = a.v[c];
 }
-BK_DEV M3 load_m3(const float* __restrict__ p, int64_t i, int64_t pitch) {
+BK_DEV M3 load_m3(const float* p, int64_t i, int64_t pitch) {
     M3 r;
 #pragma unroll
-    for (int c = 0; c < 9; ++c) r.m[c] = __ldg(p + c * pitch + i);
+    for (int c = 0; c < 9; ++c) r.m[c] = p[c * pitch + i];
     return r;
 }
 BK_DEV void store_m3(float* __restrict__ p, int64_t i, int64_t pitch, const M3& a) {
@@ -1036,8 +1039,8 @@ inline int vertex_block_threads(int64_t vertices, int64_t bindings) {
 template <int kBlock>
 BK_DEV float vertex_block(const int* __restrict__ offsets, const int* __restrict__ particles,
                           const float* __restrict__ weights, const float* __restrict__ ref_offsets, int64_t bp,
-                          const float* __restrict__ ref_vertices, int64_t vp, const float* __restrict__ x,
-                          const float* __restrict__ F, int64_t pitch, int vid) {
+                          const float* __restrict__ ref_vertices, int64_t vp, const float* x,
+                          const float* F, int64_t pitch, int vid) {
     __shared__ float s_part[3][kBlock / 32];
     const int b0 = offsets[vid], b1 = offsets[vid + 1];
     const int t = threadIdx.x;
@@ -1085,8 +1088,8 @@ BK_DEV float vertex_block(const int* __restrict__ offsets, const int* __restrict
 // with one warp, so both give the same bits.
 BK_DEV float vertex_warp(const int* __restrict__ offsets, const int* __restrict__ particles,
                          const float* __restrict__ weights, const float* __restrict__ ref_offsets, int64_t bp,
-                         const float* __restrict__ ref_vertices, int64_t vp, const float* __restrict__ x,
-                         const float* __restrict__ F, int64_t pitch, int vid) {
+                         const float* __restrict__ ref_vertices, int64_t vp, const float* x,
+                         const float* F, int64_t pitch, int vid) {
     const int b0 = offsets[vid], b1 = offsets[vid + 1];
     const int lane = threadIdx.x & 31;
     if (b0 == b1) return lane < 3 ? ref_vertices[lane * vp + vid] : 0.0f;  // the same branch for the warp

@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kThreads) k_measure(BkMeasureInputs in, double
 
 // One slot's block partials reduced by one warp: lane l combines partials l, l + 32, ... in that
 // order, then a fixed butterfly combines the lanes (a deterministic order, whatever the schedule).
-__device__ __forceinline__ double warp_slot_reduce(int op, const double* __restrict__ partial, int blocks, int stride,
+__device__ __forceinline__ double warp_slot_reduce(int op, const double* partial, int blocks, int stride,
                                                    int slot) {
     const int lane = threadIdx.x & 31;
     double v = op == kMin ? INFINITY : (op == kMax ? -INFINITY : 0.0);
@@ -202,10 +202,10 @@ __global__ void k_measure_finish(const double* __restrict__ partial, double* __r
 // 239 us at 4M yielding particles (DRAM time about 27 and 110).
 constexpr int kWide = 512;
 
-__global__ void __launch_bounds__(kWide, 2) k_step_summary(int64_t n, int64_t pitch, const float* __restrict__ v,
+__global__ void __launch_bounds__(kWide, 2) k_step_summary(int64_t n, int64_t pitch, const float* v,
                                                          const float* __restrict__ mass, const double* __restrict__ dry,
-                                                         const double* __restrict__ water, const float4* __restrict__ pm,
-                                                         const int32_t* __restrict__ box, int R,
+                                                         const double* water, const float4* pm,
+                                                         const int32_t* box, int R,
                                                          double* __restrict__ partial) {
     pdl_enter();
     double grid = 0.0, kinetic = 0.0;
@@ -213,8 +213,8 @@ __global__ void __launch_bounds__(kWide, 2) k_step_summary(int64_t n, int64_t pi
     const int64_t first = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
 #pragma unroll 4
     for (int64_t i = first; i < n; i += stride) {
-        const double m = water ? __ldg(dry + i) + __ldg(water + i) : (double)__ldg(mass + i);
-        const double a = __ldg(v + i), b = __ldg(v + pitch + i), c = __ldg(v + 2 * pitch + i);
+        const double m = water ? __ldg(dry + i) + water[i] : (double)__ldg(mass + i);
+        const double a = v[i], b = v[pitch + i], c = v[2 * pitch + i];
         kinetic += 0.5 * m * (a * a + b * b + c * c);
     }
     int lo[3], ext[3];
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(kWide, 2) k_step_summary(int64_t n, int64_t pi
     }
 }
 
-__global__ void k_step_summary_finish(const double* __restrict__ partial, double* __restrict__ out, int blocks) {
+__global__ void k_step_summary_finish(const double* partial, double* __restrict__ out, int blocks) {
     pdl_enter();
     const int k = blockIdx.x;  // one warp per value
     const double v = warp_slot_reduce(kSum, partial, blocks, 2, k);
@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(kWide, 2) k_check_state(BkCheckInputs in, doub
     }
 }
 
-__global__ void k_check_finish(const double* __restrict__ partial, double* __restrict__ out, int blocks,
+__global__ void k_check_finish(const double* partial, double* __restrict__ out, int blocks,
                                BkCheckInputs in) {
     pdl_enter();
     const int s = blockIdx.x;  // one warp per slot

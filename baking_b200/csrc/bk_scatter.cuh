@@ -43,7 +43,7 @@ BK_DEV void prefetch_planes(int64_t i, int64_t n, int64_t pitch, const float* a,
 // ------------------------------------------------------------- node gathers
 // sum_j w_j v_j and the moments sum_j w_j v_j o_jc over the stencil's nodes, with the offsets o_j in
 // {0, 1, 2} known at compile time: what G2P forms v and C of (C_rc = 4/dx (M_rc - l_c S_r)).
-BK_DEV void gather_velocity(const Stencil& st, const float4* __restrict__ node_v, int R32, float* nv, float* mo) {
+BK_DEV void gather_velocity(const Stencil& st, const float4* node_v, int R32, float* nv, float* mo) {
 #pragma unroll
     for (int r = 0; r < 3; ++r) nv[r] = 0.f;
 #pragma unroll
@@ -58,7 +58,7 @@ BK_DEV void gather_velocity(const Stencil& st, const float4* __restrict__ node_v
 #pragma unroll
             for (int oz = 0; oz < 3; ++oz) {
                 float w = wxy * st.w[2][oz];
-                float4 u = __ldg(vbase + (ox * R + oy) * R + oz);
+                float4 u = vbase[(ox * R + oy) * R + oz];
                 float wu[3] = {w * u.x, w * u.y, w * u.z};
 #pragma unroll
                 for (int r = 0; r < 3; ++r) {
@@ -73,7 +73,7 @@ BK_DEV void gather_velocity(const Stencil& st, const float4* __restrict__ node_v
 
 // sum_j w_j (dT, dW/W)_j of the diffused node fields in float64, axis by axis (two multiply-adds a
 // node instead of a weight product, its conversion and two multiply-adds).
-BK_DEV void gather_scalars(const Stencil& st, const double2* __restrict__ dTr, int R32, double& dT, double& ratio) {
+BK_DEV void gather_scalars(const Stencil& st, const double2* dTr, int R32, double& dT, double& ratio) {
     const double2* nodes = dTr + node_index(st.b[0], st.b[1], st.b[2], R32);
     const int64_t R = R32;
     dT = ratio = 0.0;
@@ -85,7 +85,7 @@ BK_DEV void gather_scalars(const Stencil& st, const double2* __restrict__ dTr, i
             double ty = 0.0, ry = 0.0;
 #pragma unroll
             for (int oz = 0; oz < 3; ++oz) {
-                const double2 d = __ldg(nodes + (ox * R + oy) * R + oz);
+                const double2 d = nodes[(ox * R + oy) * R + oz];
                 ty = fma((double)st.w[2][oz], d.x, ty);
                 ry = fma((double)st.w[2][oz], d.y, ry);
             }

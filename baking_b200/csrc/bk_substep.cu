@@ -154,8 +154,8 @@ inline unsigned vertex_launch_blocks(int64_t vertices, int threads) {
 constexpr int vertex_launch_threads(int threads) { return threads == 32 ? 32 * kVertexWarps : threads; }
 
 template <int kBlock, bool kRef = false>
-__device__ __forceinline__ void surface_vertices_body(Arg<Params, kRef> P, const float* __restrict__ x,
-                                                      const float* __restrict__ F, Arg<BkSurface, kRef> sf, Slot sl) {
+__device__ __forceinline__ void surface_vertices_body(Arg<Params, kRef> P, const float* x,
+                                                      const float* F, Arg<BkSurface, kRef> sf, Slot sl) {
     if constexpr (kBlock == 32) {
         const int64_t k = (int64_t)sl.block * kVertexWarps + (threadIdx.x >> 5);
         if (k >= sf.vertex_count) return;  // whole warps
@@ -175,8 +175,8 @@ __device__ __forceinline__ void surface_vertices_body(Arg<Params, kRef> P, const
 }
 
 template <int kBlock>
-__global__ void __launch_bounds__(kBlock == 32 ? 32 * kVertexWarps : kBlock) k_surface_vertices(Params P, const float* __restrict__ x,
-                                                          const float* __restrict__ F, BkSurface sf) {
+__global__ void __launch_bounds__(kBlock == 32 ? 32 * kVertexWarps : kBlock) k_surface_vertices(Params P, const float* x,
+                                                          const float* F, BkSurface sf) {
     pdl_enter();
     surface_vertices_body<kBlock>(P, x, F, sf, grid_slot());
 }
@@ -274,7 +274,7 @@ struct OwnerState {
 };
 template <class PP, class ST, class CS>
 __device__ __forceinline__ OwnerState owner_state(const PP& P, const ST& in, const CS& cst, int p) {
-    return OwnerState{load_v3(in.x, p, P.pitch), load_m3(in.F, p, P.pitch), __ldg(in.temperature + p), __ldg(in.water + p),
+    return OwnerState{load_v3(in.x, p, P.pitch), load_m3(in.F, p, P.pitch), in.temperature[p], in.water[p],
                       __ldg(cst.volume + p)};
 }
 
@@ -776,7 +776,7 @@ __device__ __forceinline__ void p2g_body(Arg<Params, kRef> P, Arg<BkState, kRef>
         M3 tau;
         float T_mat = 0.f;
         float rho_ref = P.density;
-        double sat = 0.0, N = 0.0;
+        double sat = 0.0, N = 0.0, T_new = 0.0, W_new = 0.0;
         if (P.transport) {
             // The scalar G2P of the diffused node fields (thermal_water.py:206-215).
             double dTp, ratio;
@@ -786,8 +786,8 @@ __device__ __forceinline__ void p2g_body(Arg<Params, kRef> P, Arg<BkState, kRef>
             double Wn = in.water[i] * (1.0 + ratio);
             double dry = cst.dry_mass[i];
             float V0 = cst.volume[i];
-            out.temperature[i] = Tn;
-            out.water[i] = Wn;
+            T_new = Tn;
+            W_new = Wn;
             mass = (float)(dry + Wn);
             rho_ref = (float)((dry + Wn) / (double)V0);
             sat = Wn / ((double)P.water_density * (double)V0 * (double)J);
@@ -799,7 +799,6 @@ __device__ __forceinline__ void p2g_body(Arg<Params, kRef> P, Arg<BkState, kRef>
                     double z = (Tm - (double)P.peak) / (double)P.width;
                     N += (double)(P.dt * P.density) * (double)cst.gas_rate[cst.gas_rate_per_particle ? i : 0] * exp(-(z * z));
                 }
-                out.gas_moles[i] = N;
             }
         } else {
             mass = cst.mass[i];
@@ -846,6 +845,11 @@ __device__ __forceinline__ void p2g_body(Arg<Params, kRef> P, Arg<BkState, kRef>
         float scale = P.dt * cst.volume[i] * 4.0f / (P.dx * P.dx);
         M3 Cm = load_m3(in.C, i, pitch);
         V3 vel = load_v3(in.v, i, pitch);
+        if (P.transport) {  // after the loads, which the compiler may not move over a store
+            out.temperature[i] = T_new;
+            out.water[i] = W_new;
+            if (P.gas) out.gas_moles[i] = N;
+        }
 #pragma unroll
         for (int e = 0; e < 9; ++e) A[e] = mass * Cm.m[e] - scale * tau.m[e];
         // w (m v + A (o - l) dx) = w (q + A dx o) with q = m v - A l dx.
