@@ -685,12 +685,14 @@ __global__ void __launch_bounds__(kThreads, 4) k_adj_g2p_return(AdjParams P, BkS
 // three additions, the cofactor, its sums with w_z and w_z', and w_z u), the gather takes about 14
 // operations a node where the plain double sum took 45; with the scatter by warp runs 128 -> 102 us at
 // 1M particles.
-template <bool kLoaf = false>
-__global__ void __launch_bounds__(kThreads, 7) k_adj_g2p_scatter(AdjParams P, BkState in, const float4* grid_v,
+template <Sums kSums, bool kLoaf = false>
+__global__ void __launch_bounds__(kThreads, kSums == Sums::kTiles ? 4 : 7) k_adj_g2p_scatter(AdjParams P, BkState in, const float4* grid_v,
                                                             AdjState out_adj, AdjState in_adj,
                                                             float4* __restrict__ grid_v_adj) {
     if constexpr (kLoaf) fix_loaf_mode(P);
     __shared__ MomentumRecord sm[kThreads / 32];
+    WarpTiles* tiles = nullptr;
+    if constexpr (kSums == Sums::kTiles) tiles = warp_tiles();
     const int64_t i = blockIdx.x * (int64_t)kThreads + threadIdx.x;
     const int64_t pitch = P.pitch;
     prefetch_planes(i, P.n, pitch, in.x, 3, in_adj.C, 9, out_adj.x, 3);
@@ -766,7 +768,7 @@ __global__ void __launch_bounds__(kThreads, 7) k_adj_g2p_scatter(AdjParams P, Bk
 #pragma unroll
         for (int c = 0; c < 3; ++c) in_adj.x[c * pitch + i] = 0.f;
     }
-    scatter_momentum(sm, valid, st, 0.f, q, A, grid_v_adj, P.R, group_lanes(P.n, P.R), false);
+    scatter_momentum<kSums>(sm, tiles, valid, st, 0.f, q, A, grid_v_adj, P.R, group_lanes(P.n, P.R), P.R <= 1024);
 }
 
 // ------------------------------------------------------------- grid update
@@ -1065,7 +1067,8 @@ int bk_substep_adjoint(const BkSubstepParams* params, const BkState* in, const B
                                    constants->viscosity_parameter, adj_state(*out_adjoint), adj_state(*in_adjoint),
                                    parameter_adjoint);
     if (int rc = bk::check_chained(e, "bk_substep_adjoint/g2p_return")) return rc;
-    e = launch_chained(loaf ? k_adj_g2p_scatter<true> : k_adj_g2p_scatter<false>, blocks, kThreads, 0, s, a, *in,
+    auto* scatter = loaf ? k_adj_g2p_scatter<Sums::kAlone, true> : k_adj_g2p_scatter<Sums::kAlone>;
+    e = launch_chained(scatter, blocks, kThreads, 0, s, a, *in,
                        reinterpret_cast<const float4*>(node_v), adj_state(*out_adjoint), adj_state(*in_adjoint),
                        reinterpret_cast<float4*>(node_v_adjoint));
     if (int rc = bk::check_chained(e, "bk_substep_adjoint/g2p_scatter")) return rc;

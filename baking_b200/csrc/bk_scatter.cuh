@@ -4,13 +4,13 @@
 // A warp splits its 32 particles into runs of equal stencil base. Each particle's own thread stores
 // its 27 node weights (w_x w_y) w_z, as the reference rounds them, and its values in the warp's
 // record in shared memory; the run is then summed over its particles and every node receives one
-// atomic per run (one 16-byte vector atomic for momentum and mass). Nothing is shared between
-// warps, so a block has no barrier (large bodies: merge_runs, below).
+// atomic per run (one 16-byte vector atomic for momentum and mass). The transport fields, float64, go to the
+// grid that way; the float32 momentum is summed over the block first (below).
 //
-// What bounds it, and why there is no block tile: a shared-memory tile over the block's node box
-// (summing the block's runs before one global atomic per node) needs three block barriers, the
-// zeroing and flushing of the tile, and shared float atomics, which are compare-and-swap loops with
-// bank conflicts; it held the LSU data pipe at 73% (momentum) and 71% (transport) of its peak. A run
+// What bounds it, and why no warps share a tile: a shared-memory tile over the block's node box that every
+// warp adds to needs three block barriers, the zeroing and flushing of the tile, and shared float atomics,
+// which are compare-and-swap loops with bank conflicts; it held the LSU data pipe at 73% (momentum)
+// and 71% (transport) of its peak. A run
 // of ~18 particles already divides the atomics by 18, and L2 takes the rest without waiting. 1M
 // particles, 128^3 grid, 40 particles a cell, fused P2G kernel: 102 us with the tile, 87 us with the
 // same kernel writing straight to L2; transport scatter 68.5 against 62.1 us, 55 with the float64
@@ -128,23 +128,25 @@ struct Runs {
 // (8 a cell) runs a warp and gain nothing; particles in another order, as sampled tet by tet (up to 32
 // runs a warp, about 10 bases), get a third of the atomics, and node sums of fewer and larger parts.
 // P2G in tet order: 41k particles 16 -> 8.6 us, 5k 9.7 -> 8.3. Smaller bodies keep the order of their
-// samples (192 particles: 9.4 us, grouped 8.6): their float32 sums, and with them every rounding of a
-// position, stay those that finite differences over a few hundred particles were resolved with.
+// samples although grouping is faster there too (192 particles: 9.4 us, grouped 8.6): the finite differences
+// that check the gradients over such bodies are differences of float32 roundings, and were resolved with
+// the sums in that order (grouped, two of them miss their tolerance, by 9% and 74%).
 constexpr int kGroupRuns = 8;
 constexpr int64_t kGroupParticles = 256;
 
 BK_DEV bool group_lanes(int64_t n, int R) { return n >= kGroupParticles && R <= 1024; }
 
-// Bodies of this many particles (same grids) merge the momentum runs of a block before they reach the
-// grid. A particle that has just crossed into another cell gives that cell's far nodes weights of 1e-6
-// and less; sent alone, such a sum is below half a unit of a node's last place and lost: 20 substeps
-// after a 1M loaf's particles were ordered its grid mass lacks 1.0e-8 of itself, with blocks of 128
-// merged 0.45e-8, of 256 (the earlier node tile) 0.33e-8. It costs 13.5 us of a substep of 1M particles (P2G 76 to 90)
-// and 5 at 200k. Below 65536 particles the share lost hides under the random error of so few node sums, and the
-// merge's two barriers would cost 7 us of a substep that takes 50 (9k particles).
-constexpr int64_t kMergeParticles = 65536;
-
-BK_DEV bool merge_blocks(int64_t n, int R) { return n >= kMergeParticles && R <= 1024; }
+// Momentum sums of a block's warps are merged before they reach the grid. A particle that has just crossed
+// into another cell gives that cell's far nodes weights of 1e-6 and less; sent alone, such a sum is
+// below half a unit of a node's last place and lost. Error against 64 bits of warps' sums sent
+// alone over that of a node tile shared by 256 particles: grid mass of a strained 39k cube in sample order
+// 2.5 +- 0.4, velocities of a pre-stressed 60k loaf 1.009 +- 0.001, its temperature gradient 1.05 (where
+// the reverse scatter is not merged either); merged 0.94 +- 0.2, 1.000 and 1.003. Two forms:
+// * bodies below kKeptParticles: every warp sums into a tile of its own (WarpTiles), which costs the fewest
+//   steps and 24 KB a block: four blocks on an SM, where such a body has no more than that.
+// * larger bodies, which need eight blocks on an SM: the warps keep their sums in their records and
+//   add them up in the space of the values (merge_runs).
+constexpr int64_t kKeptParticles = 65536;
 
 BK_DEV Runs find_runs(bool valid, const int* b, bool group) {
     const int lane = threadIdx.x & 31;
@@ -159,14 +161,19 @@ BK_DEV Runs find_runs(bool valid, const int* b, bool group) {
         const unsigned key = valid ? (unsigned)(b[0] << 20 | b[1] << 10 | b[2]) : 0x80000000u | (unsigned)lane;
         const unsigned peers = __match_any_sync(kWarp, key);
         const int rank = __popc(peers & ((1u << lane) - 1u)), first = __ffs(peers) - 1;
-        const int size = rank == 0 ? __popc(peers) : 0;
-        int sum = size;  // columns up to and including this lane's group, groups in the order of their first lanes
+        // Groups of four or more first (each leaves room for a kept sum, merge_runs), then the others, in the
+        // order of their first lanes: two prefix sums of the sizes in one word.
+        const int peer_count = __popc(peers);
+        const bool large = peer_count >= 4;
+        int sum = rank == 0 ? (large ? peer_count : peer_count << 16) : 0;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const int v = __shfl_up_sync(kWarp, sum, o);
             if (lane >= o) sum += v;
         }
-        r.column = __shfl_sync(kWarp, sum - size, first) + rank;
+        const int all_large = __shfl_sync(kWarp, sum, 31) & 0xffff;
+        const int start = (large ? sum & 0xffff : all_large + (sum >> 16)) - peer_count;  // of a first lane's group
+        r.column = __shfl_sync(kWarp, start, first) + rank;
         r.starts = __reduce_or_sync(kWarp, valid && rank == 0 ? 1u << r.column : 0u);
     }
     return r;
@@ -233,11 +240,32 @@ struct MomentumRecord {
 
 BK_DEV unsigned pack_base(int x, int y, int z) { return (unsigned)(x << 20 | y << 10 | z); }
 
+// Nodes of a block's box that fit a tile. A block of 128 covers up to 300 in the sample order of a 41k cube, 85 to
+// 95% of the blocks of a ball or sphere at 8 particles a cell have 384 or fewer; the others' sums go
+// to the grid one by one.
+constexpr int kMergeNodes = 384;
+
+// Node t of a box with the extents ext (t < 384, so t * ext < 2^16: exact quotients).
+BK_DEV int64_t box_node(int t, const int* lo, const int* ext, int R) {
+    const unsigned by_z = (unsigned)__fdividef(65536.f, (float)ext[2]) + 1u, by_y = (unsigned)__fdividef(65536.f, (float)ext[1]) + 1u;
+    const int yx = (int)((unsigned)t * by_z >> 16), x = (int)((unsigned)yx * by_y >> 16);
+    return node_index(lo[0] + x, lo[1] + yx - x * ext[1], lo[2] + t - yx * ext[2], R);
+}
+
+// A tile over the block's node box for each of its four warps.
+struct WarpTiles {
+    float4 node[4][kMergeNodes];
+    int low[4][3], high[4][3];  // each warp's bases
+};
+// (Declared in an inlined function, as warp_records of the substep's scatter.)
+BK_DEV WarpTiles* warp_tiles() {
+    __shared__ WarpTiles tiles;
+    return &tiles;
+}
+
 // The block's kept runs, summed in a tile over their node box and sent to L2 as one atomic per node. Warp
 // c sums component c, run by run in the order of the block's particles, in the space of its particles'
 // values (no shared atomics: no two warps touch a word; with a thread per node looping over the runs 18 us).
-constexpr int kMergeNodes = 384;
-
 BK_DEV void merge_runs(MomentumRecord* sm, float4* __restrict__ nodes, int R) {
     static_assert(sizeof(MomentumRecord::val) >= kMergeNodes * sizeof(float) && kGroupRuns == 8, "tile and slots");
     const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
@@ -271,15 +299,11 @@ BK_DEV void merge_runs(MomentumRecord* sm, float4* __restrict__ nodes, int R) {
             __syncwarp();
         }
         __syncthreads();
-        // (exact quotients: t * ext < 2^16, since both other extents are at least 3)
-        const unsigned by_z = (unsigned)__fdividef(65536.f, (float)ext[2]) + 1u, by_y = (unsigned)__fdividef(65536.f, (float)ext[1]) + 1u;
         for (int t = threadIdx.x; t < count; t += 128) {
             const float4 sum = make_float4(reinterpret_cast<const float*>(sm[0].val)[t], reinterpret_cast<const float*>(sm[1].val)[t],
                                            reinterpret_cast<const float*>(sm[2].val)[t], reinterpret_cast<const float*>(sm[3].val)[t]);
             if (sum.x == 0.f && sum.y == 0.f && sum.z == 0.f && sum.w == 0.f) continue;
-            const int yx = (int)((unsigned)t * by_z >> 16), x = (int)((unsigned)yx * by_y >> 16);
-            const int y = yx - x * ext[1], z = t - yx * ext[2];
-            atomicAdd(nodes + node_index(lo[0] + x, lo[1] + y, lo[2] + z, R), sum);
+            atomicAdd(nodes + box_node(t, lo, ext, R), sum);
         }
     } else if (lane < 27) {  // far apart: each warp its own runs
         const MomentumRecord& rec = sm[c];
@@ -292,74 +316,126 @@ BK_DEV void merge_runs(MomentumRecord* sm, float4* __restrict__ nodes, int R) {
     }
 }
 
-// (The adjoint of G2P has the same form with m = 0.) With `merge` every warp of a block of 128
-// threads calls it; `group` and
-// `merge` are the same for all of them.
-BK_DEV void scatter_momentum(MomentumRecord* sm, bool valid, const Stencil& st, float m, const float* q,
-                             const float* A, float4* __restrict__ nodes, int R, bool group, bool merge) {
-    const int lane = threadIdx.x & 31;
-    MomentumRecord& rec = sm[threadIdx.x >> 5];
+// Sum of one run's particles, columns s to e - 1, at this lane's node (j < 27): momentum and mass.
+BK_DEV float4 run_sum(const MomentumRecord& rec, const float* wj, const float* fo, int s, int e) {
+    float2 mq0 = {0.f, 0.f}, q12 = {0.f, 0.f}, A01 = {0.f, 0.f}, A23 = {0.f, 0.f};
+    float2 A45 = {0.f, 0.f}, A67 = {0.f, 0.f};
+    float A8 = 0.f;
+#pragma unroll 2
+    for (int k = s; k < e; ++k) {
+        const float w = wj[k];
+        const float2 ww = make_float2(w, w);
+        const float4 v0 = rec.val[k][0], v1 = rec.val[k][1], v2 = rec.val[k][2];
+        mq0 = ffma2(ww, make_float2(v0.x, v0.y), mq0);
+        q12 = ffma2(ww, make_float2(v0.z, v0.w), q12);
+        A01 = ffma2(ww, make_float2(v1.x, v1.y), A01);
+        A23 = ffma2(ww, make_float2(v1.z, v1.w), A23);
+        A45 = ffma2(ww, make_float2(v2.x, v2.y), A45);
+        A67 = ffma2(ww, make_float2(v2.z, v2.w), A67);
+        A8 = fmaf(w, rec.a8[k], A8);
+    }
+    const float aq[3] = {mq0.y, q12.x, q12.y};
+    const float aA[9] = {A01.x, A01.y, A23.x, A23.y, A45.x, A45.y, A67.x, A67.y, A8};
+    float ap[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+        ap[r] = aq[r] + (aA[3 * r] * fo[0] + aA[3 * r + 1] * fo[1] + aA[3 * r + 2] * fo[2]);
+    return make_float4(ap[0], ap[1], ap[2], mq0.x);
+}
+
+// How a block's sums reach the grid.
+enum class Sums { kAlone, kTiles, kKept };
+
+// (The adjoint of G2P has the same form with m = 0.) kTiles and kKept: every warp of a block of 128 threads
+// calls it; `tiles` is used by kTiles only. kKept keys bases by 10 bits an axis: on larger grids
+// (`keyed` false) it sends the sums one by one. `group` and `keyed` are the same for all threads.
+template <Sums kSums>
+BK_DEV void scatter_momentum(MomentumRecord* sm, WarpTiles* tiles, bool valid, const Stencil& st, float m, const float* q,
+                             const float* A, float4* __restrict__ nodes, int R, bool group, bool keyed = true) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    MomentumRecord& rec = sm[warp];
     const Runs runs = find_runs(valid, st.b, group);
-    const bool keep = merge && __popc(runs.starts) < kGroupRuns;
-    int kept = 0;
+    const bool keep = kSums == Sums::kKept && keyed;
     put_weights(rec.w, runs.column, valid, st);
     rec.val[runs.column][0] = make_float4(m, q[0], q[1], q[2]);
     rec.val[runs.column][1] = make_float4(A[0], A[1], A[2], A[3]);
     rec.val[runs.column][2] = make_float4(A[4], A[5], A[6], A[7]);
     rec.a8[runs.column] = A[8];
     rec.corner[runs.column] = node_index(st.b[0], st.b[1], st.b[2], R);
-    if (merge) rec.key[runs.column] = pack_base(st.b[0], st.b[1], st.b[2]);
+    if (keep) rec.key[runs.column] = pack_base(st.b[0], st.b[1], st.b[2]);
+    int lo[3], ext[3], count = 0;  // the block's box (kTiles), count its nodes where they fit
+    float4* tile = nullptr;
+    if constexpr (kSums == Sums::kTiles) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const int low = __reduce_min_sync(kWarp, valid ? st.b[a] : INT_MAX);
+            const int high = __reduce_max_sync(kWarp, valid ? st.b[a] : INT_MIN);
+            if (lane == 0) {
+                tiles->low[warp][a] = low;
+                tiles->high[warp][a] = high;
+            }
+        }
+        __syncthreads();
+        int64_t all = 1;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = min(min(tiles->low[0][a], tiles->low[1][a]), min(tiles->low[2][a], tiles->low[3][a]));
+            const int high = max(max(tiles->high[0][a], tiles->high[1][a]), max(tiles->high[2][a], tiles->high[3][a]));
+            if (lo[a] > high) return;  // no valid particle in the block (lo = INT_MAX): the same for all threads
+            ext[a] = high + 3 - lo[a];
+            all *= ext[a];
+        }
+        if (all <= kMergeNodes) count = (int)all;
+        tile = tiles->node[warp];
+        for (int t = lane; t < count; t += 32) tile[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (valid) rec.key[runs.column] = ((st.b[0] - lo[0]) * ext[1] + st.b[1] - lo[1]) * ext[2] + st.b[2] - lo[2];
+    }
     __syncwarp();
     int ox, oy, oz;
     node_offset(lane < 27 ? lane : 0, ox, oy, oz);
     const float fo[3] = {(float)ox, (float)oy, (float)oz};
     float* const wj = rec.w[lane < 27 ? lane : 0];
     float4* const mine = nodes + ((int64_t)ox * R + oy) * R + oz;
+    if constexpr (kSums == Sums::kTiles) tile += (ox * ext[1] + oy) * ext[2] + oz;
+    int kept = 0;
     unsigned starts = runs.starts;
     while (starts) {
         const int s = __ffs(starts) - 1;
         starts &= starts - 1;
         const int e = run_end(starts);
         // A kept run's sums take the weights' place: row j is read by lane j only, columns below e no more.
-        const bool here = keep && 4 * (kept + 1) <= e;
+        const bool here = keep && kept < kGroupRuns && 4 * (kept + 1) <= e;
         if (lane < 27) {
-            float2 mq0 = {0.f, 0.f}, q12 = {0.f, 0.f}, A01 = {0.f, 0.f}, A23 = {0.f, 0.f};
-            float2 A45 = {0.f, 0.f}, A67 = {0.f, 0.f};
-            float A8 = 0.f;
-#pragma unroll 2
-            for (int k = s; k < e; ++k) {
-                const float w = wj[k];
-                const float2 ww = make_float2(w, w);
-                const float4 v0 = rec.val[k][0], v1 = rec.val[k][1], v2 = rec.val[k][2];
-                mq0 = ffma2(ww, make_float2(v0.x, v0.y), mq0);
-                q12 = ffma2(ww, make_float2(v0.z, v0.w), q12);
-                A01 = ffma2(ww, make_float2(v1.x, v1.y), A01);
-                A23 = ffma2(ww, make_float2(v1.z, v1.w), A23);
-                A45 = ffma2(ww, make_float2(v2.x, v2.y), A45);
-                A67 = ffma2(ww, make_float2(v2.z, v2.w), A67);
-                A8 = fmaf(w, rec.a8[k], A8);
-            }
-            const float aq[3] = {mq0.y, q12.x, q12.y};
-            const float aA[9] = {A01.x, A01.y, A23.x, A23.y, A45.x, A45.y, A67.x, A67.y, A8};
-            float ap[3];
-#pragma unroll
-            for (int r = 0; r < 3; ++r)
-                ap[r] = aq[r] + (aA[3 * r] * fo[0] + aA[3 * r + 1] * fo[1] + aA[3 * r + 2] * fo[2]);
+            const float4 sum = run_sum(rec, wj, fo, s, e);
             if (here) {
-                wj[4 * kept] = ap[0];
-                wj[4 * kept + 1] = ap[1];
-                wj[4 * kept + 2] = ap[2];
-                wj[4 * kept + 3] = mq0.x;
+                wj[4 * kept] = sum.x;
+                wj[4 * kept + 1] = sum.y;
+                wj[4 * kept + 2] = sum.z;
+                wj[4 * kept + 3] = sum.w;
+            } else if (kSums == Sums::kTiles && count > 0) {
+                float4& node = tile[rec.key[s]];
+                const float4 old = node;
+                node = make_float4(old.x + sum.x, old.y + sum.y, old.z + sum.z, old.w + sum.w);
             } else {
-                atomicAdd(mine + rec.corner[s], make_float4(ap[0], ap[1], ap[2], mq0.x));
+                atomicAdd(mine + rec.corner[s], sum);
             }
         }
+        if (kSums == Sums::kTiles) __syncwarp();  // the next run's lanes meet these nodes
         if (here) {
             if (lane == 0) rec.base[kept] = rec.key[s];
             ++kept;
         }
     }
-    if (merge) {
+    if constexpr (kSums == Sums::kTiles) {
+        __syncthreads();
+        for (int t = threadIdx.x; t < count; t += 128) {
+            const float4 a = tiles->node[0][t], b = tiles->node[1][t], c = tiles->node[2][t], d = tiles->node[3][t];
+            const float4 sum = make_float4((a.x + b.x) + (c.x + d.x), (a.y + b.y) + (c.y + d.y), (a.z + b.z) + (c.z + d.z),
+                                           (a.w + b.w) + (c.w + d.w));
+            if (sum.x == 0.f && sum.y == 0.f && sum.z == 0.f && sum.w == 0.f) continue;
+            atomicAdd(nodes + box_node(t, lo, ext, R), sum);
+        }
+    } else if (keep) {
         if (lane == 0) rec.kept = kept;
         merge_runs(sm, nodes, R);
     }

@@ -723,7 +723,7 @@ __global__ void k_grid_update(Params P, GridPtrs g) {
 // latency behind it. Loads are plain: staging the block's planes by bulk copies (33 KB and two
 // barriers a block) took 87.0 us where this form, with its L2 prefetch and no barrier, takes 82.
 // Blocks of 128 against 256: 81.8 and 84.2 us at 1M particles (a finished block's slot is refilled
-// earlier). The merge of large bodies' runs (merge_runs) and its barriers come on top.
+// earlier). The merge of a block's sums (bk_scatter.cuh) and its barriers come on top.
 constexpr int kP2GThreads = 128;
 // Bodies of at most this many particles are one block, whose warps send their sums in step after a
 // barrier: the atomics of a node leave one SM in the same order each time, and a run repeats bit for bit
@@ -731,11 +731,17 @@ constexpr int kP2GThreads = 128;
 // finite differences of such a body carried that noise). The time is the same (17 us).
 constexpr int kP2GSmall = 256;
 
-template <bool kRef = false, int kBlock = kP2GThreads>
+constexpr int p2g_threads(Sums sums) { return sums == Sums::kAlone ? kP2GSmall : kP2GThreads; }
+inline Sums p2g_sums(int64_t n) { return n <= kP2GSmall ? Sums::kAlone : n < kKeptParticles ? Sums::kTiles : Sums::kKept; }
+
+template <Sums kSums, bool kRef = false>
 __device__ __forceinline__ void p2g_body(Arg<Params, kRef> P, Arg<BkState, kRef> in, Arg<BkState, kRef> out,
                                          Arg<BkConstants, kRef> cst, Arg<GridPtrs, kRef> g, Arg<BkFlags, kRef> flags,
                                          float* max_residuals, Slot sl) {
+    constexpr int kBlock = p2g_threads(kSums);
     __shared__ MomentumRecord sm[kBlock / 32];
+    WarpTiles* tiles = nullptr;
+    if constexpr (kSums == Sums::kTiles) tiles = warp_tiles();
     const int64_t i = sl.block * (int64_t)kBlock + threadIdx.x;
     const int64_t pitch = P.pitch;
     {
@@ -859,15 +865,15 @@ __device__ __forceinline__ void p2g_body(Arg<Params, kRef> P, Arg<BkState, kRef>
 #pragma unroll
         for (int e = 0; e < 9; ++e) A[e] *= P.dx;
     }
-    if constexpr (kBlock == kP2GSmall) __syncthreads();  // the warps send their sums in step (kP2GSmall)
-    scatter_momentum(sm, valid, st, mass, q, A, g.pm, P.R, group_lanes(P.n, P.R), merge_blocks(P.n, P.R));
+    if constexpr (kSums == Sums::kAlone) __syncthreads();  // the warps send their sums in step (kP2GSmall)
+    scatter_momentum<kSums>(sm, tiles, valid, st, mass, q, A, g.pm, P.R, group_lanes(P.n, P.R), P.R <= 1024);
 }
 
-template <bool kLoaf = false, int kBlock = kP2GThreads>
-__global__ void __launch_bounds__(kBlock, 1024 / kBlock) k_p2g(Params P, BkState in, BkState out, BkConstants cst, GridPtrs g,
+template <Sums kSums, bool kLoaf = false>
+__global__ void __launch_bounds__(p2g_threads(kSums), kSums == Sums::kKept ? 8 : 4) k_p2g(Params P, BkState in, BkState out, BkConstants cst, GridPtrs g,
                                                  BkFlags flags, float* max_residuals) {
     if constexpr (kLoaf) fix_loaf_mode(P);
-    p2g_body<false, kBlock>(P, in, out, cst, g, flags, max_residuals, grid_slot());
+    p2g_body<kSums>(P, in, out, cst, g, flags, max_residuals, grid_slot());
 }
 
 // ------------------------------------------------------ fused G2P + return
@@ -1468,9 +1474,11 @@ int launch_substep(const BkSubstepParams& p, const Params& with_flags, const Gri
         }
         {
             const int rec = profile_begin("p2g", s);
-            const int threads = p.n <= kP2GSmall ? kP2GSmall : kP2GThreads;
-            auto* kernel = p.n <= kP2GSmall ? (loaf ? k_p2g<true, kP2GSmall> : k_p2g<false, kP2GSmall>)
-                                            : (loaf ? k_p2g<true> : k_p2g<false>);
+            const Sums sums = p2g_sums(p.n);
+            const int threads = p2g_threads(sums);
+            auto* kernel = sums == Sums::kAlone   ? (loaf ? k_p2g<Sums::kAlone, true> : k_p2g<Sums::kAlone>)
+                           : sums == Sums::kTiles ? (loaf ? k_p2g<Sums::kTiles, true> : k_p2g<Sums::kTiles>)
+                                                  : (loaf ? k_p2g<Sums::kKept, true> : k_p2g<Sums::kKept>);
             e = launch_chained(kernel, blocks_for(p.n, threads), threads, 0, s, P, in, out, constants, g, flags,
                                diagnostics.max_residuals);
             profile_end(rec, s);
@@ -1700,10 +1708,11 @@ __global__ void __launch_bounds__(kThreads) kb_clear_previous(BatchArgs b) {
     clear_previous_body<true>(e.P, e.g, sl);
 }
 
-__global__ void __launch_bounds__(kP2GThreads, 8) kb_p2g(BatchArgs b) {
+template <Sums kSums>
+__global__ void __launch_bounds__(kP2GThreads, kSums == Sums::kKept ? 8 : 4) kb_p2g(BatchArgs b) {
     __shared__ BatchEntry e;
     const Slot sl = batch_load(b, kStP2G, e);
-    p2g_body<true>(e.P, e.in, e.out, e.cst, e.g, e.flags, e.diag.max_residuals, sl);
+    p2g_body<kSums, true>(e.P, e.in, e.out, e.cst, e.g, e.flags, e.diag.max_residuals, sl);
 }
 
 __global__ void __launch_bounds__(kThreads) kb_grid_update(BatchArgs b) {
@@ -1736,6 +1745,7 @@ struct BkBatch {
     int vertex_block = 32;
     bool all_prescatter = true;     // every transport instance takes part in the prescatter
     bool any_transport = false;
+    bool tiles = true;              // every instance is small enough for P2G's tiles
 };
 
 extern "C" {
@@ -1791,6 +1801,7 @@ int bk_batch_create(const BkBatchInstance* instances, int32_t count, BkBatch** b
             e.owners_in_runs = owners_in_runs(in.surface.owner_count, p.n);
         }
         host.any_transport = host.any_transport || p.transport;
+        host.tiles = host.tiles && p.n < kKeptParticles;
         if (p.transport && (p.keep_transport_fields || surrogate)) host.all_prescatter = false;
         uint32_t blocks[kBatchStages] = {};
         const int64_t n = p.n;
@@ -1910,7 +1921,8 @@ int bk_batch_substep(BkBatch* batch, int32_t parity, int32_t phases, int32_t pre
         }
         if (T[kStP2G]) {
             int rec = profile_begin("batch_p2g", s);
-            kb_p2g<<<T[kStP2G], kP2GThreads, 0, s>>>(a);
+            if (B.tiles) kb_p2g<Sums::kTiles><<<T[kStP2G], kP2GThreads, 0, s>>>(a);
+            else kb_p2g<Sums::kKept><<<T[kStP2G], kP2GThreads, 0, s>>>(a);
             profile_end(rec, s);
             if (int rc = check_launch("bk_batch_substep/p2g")) return rc;
         }
