@@ -1067,7 +1067,8 @@ int bk_substep_adjoint(const BkSubstepParams* params, const BkState* in, const B
                                    constants->viscosity_parameter, adj_state(*out_adjoint), adj_state(*in_adjoint),
                                    parameter_adjoint);
     if (int rc = bk::check_chained(e, "bk_substep_adjoint/g2p_return")) return rc;
-    auto* scatter = loaf ? k_adj_g2p_scatter<Sums::kAlone, true> : k_adj_g2p_scatter<Sums::kAlone>;
+    auto* scatter = p.n < kKeptParticles ? (loaf ? k_adj_g2p_scatter<Sums::kTiles, true> : k_adj_g2p_scatter<Sums::kTiles>)
+                                         : (loaf ? k_adj_g2p_scatter<Sums::kKept, true> : k_adj_g2p_scatter<Sums::kKept>);
     e = launch_chained(scatter, blocks, kThreads, 0, s, a, *in,
                        reinterpret_cast<const float4*>(node_v), adj_state(*out_adjoint), adj_state(*in_adjoint),
                        reinterpret_cast<float4*>(node_v_adjoint));

@@ -38,3 +38,23 @@ def test_grid_mass():
             sim.AdvanceUnchecked(10)
             losses.append(float(sim.grid_state.node_masses.double().sum()) / total - 1.0)
     assert abs(np.mean(losses)) <= 3.5e-9
+
+
+@pytest.mark.parametrize("voxels,bound", [(11, 1.6e-7), (14, 1.9e-7)])
+def test_gradient_of_the_momentum(voxels, bound):
+    """Internal forces conserve momentum, so d(sum m c . v') / dv = m c whatever the body does in between.
+    Relative error of that gradient after 8 substeps with the shared tile and with sums sent alone:
+    1.33e-7 and 1.88e-7 (39,930 particles), 1.51e-7 and 2.35e-7 (82,320), each +- 0.05e-7 over 8 seeds."""
+    import torch
+    from baking_b200.physics.adjoint import Rollout
+    c = torch.tensor([0.7, -1.1, 0.9], dtype=torch.float64, device="cuda")
+    errors = []
+    for seed in range(8):
+        sim = cube(voxels, seed)
+        sim.AdvanceUnchecked(10)
+        v = sim.current_state.particle_velocities.clone().requires_grad_(True)
+        m = sim.particle_data.particle_masses.double()[:, None]
+        out = Rollout(sim, 8, checkpoint_every=4, velocities=v)["velocities"]
+        (m * c * out.double()).sum().backward()
+        errors.append(float((v.grad.double() - m * c).norm() / (m * c).norm()))
+    assert np.mean(errors) <= bound
