@@ -709,17 +709,16 @@ static __device__ __noinline__ float solve_porosity_bisection(float q, float p, 
 // trial, so the caller can skip that evaluation. Every other case takes the float64 test.
 //
 // `plastic`: the caller has certified q + a(trial) p > 1 (particle_side), so the elastic tests are skipped.
-// A Newton step below 1e-7 n^2 (or 1e-14 n) ends the solve without another evaluation: the error left
-// is of the order of its square over n (a(n) varies with ln n). `consistency` (may be NULL) then returns |float(n) - prediction(float(n))| from the
-// root and the slope there (the terms left out are of the order of ulp^2), or -1 where the caller has
-// to evaluate it.
+// A Newton step below 1e-7 n^2 (1 - n) (or 1e-14 n) ends the solve without another evaluation: a(n) varies
+// with ln n and, towards n = 1, with ln (1 - n), so the error left is of the order of the step's square
+// over n (1 - n), below 1e-14 n. Against 80-bit roots of 3,000 plastic states with porosities from 0.001 to 0.9 the
+// root is as near as with a last step of 1e-14 n: 1.9e-13, 2.5e-15, 5.4e-16 by decade of n with that, 1.0e-13,
+// 2.5e-15, 5.3e-16 so, in 2.5 evaluations instead of 3.2.
 BK_DEV float solve_porosity(float q, float p, float d, float h, float e, double Vp, float n0,
-                            double* warm = nullptr, bool* elastic_exit = nullptr, double* consistency = nullptr,
-                            bool plastic = false) {
+                            double* warm = nullptr, bool* elastic_exit = nullptr, bool plastic = false) {
     double r_local = 0.0;
     if (!warm) warm = &r_local;
     if (elastic_exit) *elastic_exit = false;
-    if (consistency) *consistency = -1.0;
     double trial = Vp - 1.0 + (double)n0;
     if (!plastic && trial > 0.0 && trial < 1.0) {
         const float nf = (float)trial;
@@ -742,10 +741,7 @@ BK_DEV float solve_porosity(float q, float p, float d, float h, float e, double 
         double slope;
         double pred = porosity_prediction_slope(n, q, p, d, h, e, Vp, n0, slope, warm);
         double g = n - pred;
-        if (g == 0.0) {  // n is the root
-            if (consistency) *consistency = fabs(((double)(float)n - n) * (1.0 - slope));
-            break;
-        }
+        if (g == 0.0) break;  // n is the root
         if (n < pred) lo = n; else hi = n;
         double dg = 1.0 - slope;
         double next = n - g * reciprocal_newton(dg);
@@ -753,9 +749,8 @@ BK_DEV float solve_porosity(float q, float p, float d, float h, float e, double 
         // the end of the bracket that n just became (g at the float64 rounding level, as when the
         // mean stress vanishes), the step falls on that end, and treating it as a bracket escape
         // would bisect all the way back to it.
-        if (fabs(next - n) <= fmax(1e-14 * fabs(n), 1e-7 * n * n)) {
+        if (fabs(next - n) <= fmax(1e-14 * fabs(n), 1e-7 * n * n * (1.0 - n))) {
             if (next > lo && next < hi) n = next;
-            if (consistency) *consistency = fabs(((double)(float)n - n) * dg);
             break;
         }
         if (!(next > lo && next < hi)) next = 0.5 * (lo + hi);
@@ -779,15 +774,12 @@ static __device__ __noinline__ DingPorosity ding_porosity(float q2, float p2, fl
     double r_warm = 0.0;  // overstress root carried from one solve to the next
     const double Vp = 1.0 - (double)n0 + (double)por;
     bool elastic_exit;
-    double consistency;
-    o.ret_por = solve_porosity(q2, p2, df, ms, ex, Vp, n0, &r_warm, &elastic_exit, &consistency, plastic);
-    if (consistency < 0.0) {
-        // Certain elastic exit: prediction(ret_por) has r = 0 and returns Vp - 1 + n0 exactly.
-        const double pred = elastic_exit ? Vp - 1.0 + (double)n0
-                                         : porosity_prediction((double)o.ret_por, q2, p2, df, ms, ex, Vp, n0, &r_warm);
-        consistency = fabs((double)o.ret_por - pred);
-    }
-    o.consistency = (float)consistency;
+    o.ret_por = solve_porosity(q2, p2, df, ms, ex, Vp, n0, &r_warm, &elastic_exit, plastic);
+    // Evaluated anew: it has to tell a root that the solve got wrong. Certain elastic exit:
+    // prediction(ret_por) has r = 0 and returns Vp - 1 + n0 exactly.
+    const double pred = elastic_exit ? Vp - 1.0 + (double)n0
+                                     : porosity_prediction((double)o.ret_por, q2, p2, df, ms, ex, Vp, n0, &r_warm);
+    o.consistency = (float)fabs((double)o.ret_por - pred);
     o.r = (float)r_warm;
     return o;
 }
