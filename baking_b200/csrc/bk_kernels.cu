@@ -507,6 +507,20 @@ __global__ void k_solve_porosity(int64_t n, const float* __restrict__ q, const f
     pred[i] = porosity_prediction((double)r, q[i], p[i], d[i], h[i], e[i], Vp[i], n0);
 }
 
+// The arithmetic helpers of bk_device.cuh on arrays.
+__global__ void k_arithmetic(int op, int64_t n, const double* __restrict__ a, const double* __restrict__ b,
+                             double* __restrict__ out) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double x = a[i], y = b[i];
+    switch (op) {
+        case BK_OP_DIV_UNIFORM: out[i] = (double)div_uniform((float)x, (float)y, 1.0f / (float)y); break;
+        case BK_OP_RECIPROCAL: out[i] = reciprocal_newton(x); break;
+        case BK_OP_RSQRT: out[i] = rsqrt_newton(x); break;
+        default: out[i] = exp_small(x); break;
+    }
+}
+
 __global__ void k_porosity_coefficient(int64_t n, const float* __restrict__ por, float* __restrict__ out) {
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -794,6 +808,14 @@ int bk_solve_porosity(int64_t n, const float* q, const float* p, const float* de
                                                                plastic_volume, initial_porosity, porosity,
                                                                prediction);
     return check_launch("bk_solve_porosity");
+}
+
+int bk_arithmetic(int32_t op, int64_t n, const double* a, const double* b, double* out, void* stream) {
+    BK_REQUIRE(n >= 0 && op >= BK_OP_DIV_UNIFORM && op <= BK_OP_EXP_SMALL, "bk_arithmetic: bad count or operation");
+    BK_EMPTY_OK(n);
+    BK_REQUIRE(a && b && out, "bk_arithmetic: null pointer");
+    k_arithmetic<<<blocks_for(n), kBlock, 0, S(stream)>>>(op, n, a, b, out);
+    return check_launch("bk_arithmetic");
 }
 
 int bk_porosity_coefficient(int64_t n, const float* porosity, float* coefficient, void* stream) {

@@ -178,6 +178,15 @@ BK_API int bk_solve_porosity(int64_t n, const float *q, const float *p, const fl
 /* Device evaluation of porosity_coefficient (physics/materials/ding.py:68-74) per entry. */
 BK_API int bk_porosity_coefficient(int64_t n, const float *porosity, float *coefficient, void *stream);
 
+/* Device evaluation of the kernels' arithmetic helpers per entry (a, b and out float64):
+   DIV_UNIFORM a / b in float32 from the rounded reciprocal, RECIPROCAL 1 / a, RSQRT 1 / sqrt(a),
+   EXP_SMALL exp(a); b is read by DIV_UNIFORM only. */
+#define BK_OP_DIV_UNIFORM 0
+#define BK_OP_RECIPROCAL 1
+#define BK_OP_RSQRT 2
+#define BK_OP_EXP_SMALL 3
+BK_API int bk_arithmetic(int32_t op, int64_t n, const double *a, const double *b, double *out, void *stream);
+
 /* ---- fused substep (the simulator's hot path) ----------------------------- */
 
 /* One particle state (ping-pong buffer). Planes share BkSubstepParams.pitch. */
