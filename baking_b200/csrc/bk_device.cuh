@@ -1031,13 +1031,15 @@ inline int vertex_block_threads(int64_t vertices, int64_t bindings) {
 // anchor) over its bindings b0..b1, pred_b = x_p + F_p o_b (o_b: the binding's reference offset,
 // 3 planes of `bp`), the anchor being the first binding's prediction; a vertex without bindings
 // keeps its reference position. Every thread of the block must call it (it synchronises the block);
-// threads 0, 1, 2 get components x, y, z.
-template <int kBlock>
+// threads 0, 1, 2 get components x, y, z. With kParts = 2 a thread keeps the sums of two, t and t + kBlock:
+// the terms, their order and so the bits of a block of twice as many.
+template <int kBlock, int kParts = 1>
 BK_DEV float vertex_block(const int* __restrict__ offsets, const int* __restrict__ particles,
                           const float* __restrict__ weights, const float* __restrict__ ref_offsets, int64_t bp,
                           const float* __restrict__ ref_vertices, int64_t vp, const float* x,
                           const float* F, int64_t pitch, int vid) {
-    __shared__ float s_part[3][kBlock / 32];
+    constexpr int kWarps = kBlock / 32;
+    __shared__ float s_part[3][kParts * kWarps];
     const int b0 = offsets[vid], b1 = offsets[vid + 1];
     const int t = threadIdx.x;
     if (b0 == b1) return t < 3 ? ref_vertices[t * vp + vid] : 0.0f;  // the same branch for the whole block
@@ -1051,28 +1053,40 @@ BK_DEV float vertex_block(const int* __restrict__ offsets, const int* __restrict
     };
     float anchor[3];
     predict(b0, anchor);
-    float disp[3] = {0.f, 0.f, 0.f};
-#pragma unroll 4
-    for (int b = b0 + t; b < b1; b += kBlock) {  // unrolled: several bindings' gathers in flight
-        float pr[3];
-        predict(b, pr);
-        const float w = weights[b];
+    float disp[kParts][3];
 #pragma unroll
-        for (int a = 0; a < 3; ++a) disp[a] += w * (pr[a] - anchor[a]);
+    for (int part = 0; part < kParts; ++part)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) disp[part][a] = 0.f;
+#pragma unroll (4 / kParts)
+    for (int first = b0 + t; first < b1; first += kParts * kBlock) {  // unrolled: several bindings' gathers in flight
+#pragma unroll
+        for (int part = 0; part < kParts; ++part) {
+            const int b = first + part * kBlock;
+            if (part > 0 && b >= b1) break;
+            float pr[3];
+            predict(b, pr);
+            const float w = weights[b];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) disp[part][a] += w * (pr[a] - anchor[a]);
+        }
     }
 #pragma unroll
-    for (int a = 0; a < 3; ++a)
+    for (int part = 0; part < kParts; ++part) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) disp[a] += __shfl_xor_sync(0xffffffffu, disp[a], o);
-    if ((t & 31) == 0) {
+        for (int a = 0; a < 3; ++a)
 #pragma unroll
-        for (int a = 0; a < 3; ++a) s_part[a][t >> 5] = disp[a];
+            for (int o = 16; o > 0; o >>= 1) disp[part][a] += __shfl_xor_sync(0xffffffffu, disp[part][a], o);
+        if ((t & 31) == 0) {
+#pragma unroll
+            for (int a = 0; a < 3; ++a) s_part[a][part * kWarps + (t >> 5)] = disp[part][a];
+        }
     }
     __syncthreads();
     float out = 0.0f;
     if (t < 3) {
         float sum = 0.0f;
-        for (int w = 0; w < kBlock / 32; ++w) sum += s_part[t][w];
+        for (int w = 0; w < kParts * kWarps; ++w) sum += s_part[t][w];
         out = anchor[t] + sum;
     }
     return out;

@@ -153,7 +153,7 @@ inline unsigned vertex_launch_blocks(int64_t vertices, int threads) {
 }
 constexpr int vertex_launch_threads(int threads) { return threads == 32 ? 32 * kVertexWarps : threads; }
 
-template <int kBlock, bool kRef = false>
+template <int kBlock, bool kRef = false, int kParts = 1>
 __device__ __forceinline__ void surface_vertices_body(Arg<Params, kRef> P, const float* x,
                                                       const float* F, Arg<BkSurface, kRef> sf, Slot sl) {
     if constexpr (kBlock == 32) {
@@ -167,7 +167,7 @@ __device__ __forceinline__ void surface_vertices_body(Arg<Params, kRef> P, const
         if (lane < 3) sf.vertices[lane * sf.vertex_pitch + vid] = v;
     } else {
         const int vid = sf.vertex_ids[sl.block];
-        const float v = vertex_block<kBlock>(sf.binding_offsets, sf.binding_particles, sf.binding_weights,
+        const float v = vertex_block<kBlock, kParts>(sf.binding_offsets, sf.binding_particles, sf.binding_weights,
                                                sf.reference_offsets, sf.binding_pitch, sf.reference_vertices,
                                                sf.vertex_pitch, x, F, P.pitch, vid);
         if (threadIdx.x < 3) sf.vertices[threadIdx.x * sf.vertex_pitch + vid] = v;
@@ -467,15 +467,17 @@ __device__ __forceinline__ Mixed mixed_block(int first) {
 }
 
 // The surface vertices and the transport scatter of one substep: both read only the state. The
-// vertices' blocks are chains of dependent gathers that leave the SMs' issue slots free.
+// vertices' blocks are chains of dependent gathers that leave the SMs' issue slots free. kBlock is the block
+// of k_surface_vertices that sums the same bits; that of 256 threads is taken by half as many.
 template <int kBlock>
 __global__ void __launch_bounds__(kOwnerThreads, 8) k_vertices_scatter(Params P, BkState in, BkConstants cst, BkSurface sf,
                                                               GridPtrs g, int32_t* sim_flags, int vertex_blocks) {
-    static_assert(vertex_launch_threads(kBlock) == kOwnerThreads, "both bodies share the block size");
+    constexpr int kParts = kBlock / kOwnerThreads > 1 ? kBlock / kOwnerThreads : 1;
+    static_assert(vertex_launch_threads(kBlock / kParts) == kOwnerThreads, "both bodies share the block size");
     const Mixed m = mixed_block(vertex_blocks);
     if (!m.is_first) scatter_prefetch(P, in, cst, m.block);
     pdl_enter();
-    if (m.is_first) surface_vertices_body<kBlock>(P, in.x, in.F, sf, Slot{m.block, vertex_blocks});
+    if (m.is_first) surface_vertices_body<kBlock / kParts, false, kParts>(P, in.x, in.F, sf, Slot{m.block, vertex_blocks});
     else transport_scatter_body(P, in, cst, g, sim_flags, Slot{m.block, (int)gridDim.x - vertex_blocks});
 }
 
@@ -1419,8 +1421,10 @@ int launch_substep(const BkSubstepParams& p, const Params& with_flags, const Gri
         if (with_vertices) {
             const int rec = profile_begin("transport_scatter", s);
             const unsigned vb = vertex_threads == 32 ? vertex_launch_blocks(nv, 32) : nv;
-            e = launch_chained(vertex_threads == 32 ? k_vertices_scatter<32> : k_vertices_scatter<128>, vb + scatter_blocks,
-                               kOwnerThreads, 0, s, P, in, constants, *surface, g, flags.simulation, (int)vb);
+            auto* kernel = vertex_threads == 32    ? k_vertices_scatter<32>
+                           : vertex_threads == 128 ? k_vertices_scatter<128>
+                                                   : k_vertices_scatter<256>;
+            e = launch_chained(kernel, vb + scatter_blocks, kOwnerThreads, 0, s, P, in, constants, *surface, g, flags.simulation, (int)vb);
             profile_end(rec, s);
             if (int rc = check_chained(e, "bk_substep/vertices_scatter")) return rc;
         } else if (nv > 0) {
