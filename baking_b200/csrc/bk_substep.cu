@@ -972,10 +972,6 @@ SurrogateDev surrogate_dev(const BkReturnSurrogate* r) {
     return d;
 }
 
-// a[k] for a runtime k in {0, 1, 2} without dynamic register indexing (which would move `a` to
-// local memory).
-__device__ __forceinline__ float sel3(const float* a, int k) { return k == 0 ? a[0] : (k == 1 ? a[1] : a[2]); }
-
 // Singular-value order (descending) the network sees, from the values or their logs.
 __device__ __forceinline__ void order3(const float* s, int* perm) {
     int a = 0, b = 1, c = 2, t;
@@ -991,7 +987,7 @@ __device__ __forceinline__ void surrogate_features(const Params& P, const BkStat
                                                    int64_t i, const DingPrelude& d, float por, float J,
                                                    const int* perm, float* f) {
 #pragma unroll
-    for (int k = 0; k < 3; ++k) f[k] = sel3(d.e, perm[k]);
+    for (int k = 0; k < 3; ++k) f[k] = pick3(d.e, perm[k]);
     f[3] = d.T_eff;
     f[4] = P.transport ? (float)(out.water[i] * reciprocal_newton((double)P.water_density * (double)cst.volume[i] * (double)J))
                        : 0.0f;
@@ -1115,7 +1111,7 @@ __device__ __forceinline__ void g2p_return_particle(const Params& P, const BkSta
 #pragma unroll
             for (int k = 0; k < 7; ++k) row[k] = f[k];
 #pragma unroll
-            for (int k = 0; k < 3; ++k) row[7 + k] = sel3(o.e, perm[k]) - f[k];
+            for (int k = 0; k < 3; ++k) row[7 + k] = pick3(o.e, perm[k]) - f[k];
             row[10] = 0.0f;
             row[11] = 0.0f;
         }
@@ -1258,7 +1254,7 @@ __device__ __forceinline__ void g2p_return_surrogate_body(Arg<Params, kRef> P, A
 #pragma unroll
                 for (int j = 0; j < 3; ++j) {
                     const int r = perm[0] == j ? 0 : (perm[1] == j ? 1 : 2);
-                    e[j] = d.e[j] + sel3(y, r) * sel3(sg.out_scale, r);
+                    e[j] = d.e[j] + pick3(y, r) * pick3(sg.out_scale, r);
                 }
                 done = ding_surrogate(P.ding, d, por, Fn, e, flags.ding, o, diag.plastic_gradients != nullptr);
                 // Judged in whole warps, so that the exact map's cost falls on 1 warp in judge_stride.

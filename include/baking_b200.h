@@ -369,7 +369,7 @@ BK_API int bk_substep_static_grid(const BkSubstepParams *params, const BkState *
    of bk_substep instead of one per stage and simulator: each block of a batched launch finds its
    instance in a device table and runs the plain kernel's body on it. An instance gets the blocks
    its own launch would use (particles, surface vertices, face owners) and, for the node-box passes,
-   about one block per 2048 particles. Each instance holds its two ping-pong states: parity 0 steps
+   a block per 256 particles (diffusion) or 1024 (clears, grid update), up to four per SM. Each instance holds its two ping-pong states: parity 0 steps
    states[0] -> states[1], parity 1 steps states[1] -> states[0]. Instances with transport need
    18-int grid bounds (the transport prescatter) and the surface accumulators of both states, which
    bk_batch_substep advances in its surface kernel (the instances' own accumulate_* fields are
