@@ -71,30 +71,27 @@ BK_DEV void gather_velocity(const Stencil& st, const float4* node_v, int R32, fl
         }
 }
 
-// sum_j w_j (dT, dW/W)_j of the diffused node fields in float64, axis by axis (two multiply-adds a
-// node instead of a weight product, its conversion and two multiply-adds).
+// sum_j w_j (dT, dW/W)_j of the diffused node fields in float64, with the weights as the scatter rounds them
+// (put_weights): the heat and water that leave one particle then arrive at others to the last float64 place.
+// Summed axis by axis from unrounded weights (a conversion and a product less a node) the energy of an
+// insulated 40k cube drifted by 5.6e-11 of the heat moved in 100 substeps, with these by 2e-14.
 BK_DEV void gather_scalars(const Stencil& st, const double2* dTr, int R32, double& dT, double& ratio) {
     const double2* nodes = dTr + node_index(st.b[0], st.b[1], st.b[2], R32);
     const int64_t R = R32;
     dT = ratio = 0.0;
 #pragma unroll
-    for (int ox = 0; ox < 3; ++ox) {
-        double tx = 0.0, rx = 0.0;
+    for (int ox = 0; ox < 3; ++ox)
 #pragma unroll
         for (int oy = 0; oy < 3; ++oy) {
-            double ty = 0.0, ry = 0.0;
+            const float wxy = st.w[0][ox] * st.w[1][oy];
 #pragma unroll
             for (int oz = 0; oz < 3; ++oz) {
                 const double2 d = nodes[(ox * R + oy) * R + oz];
-                ty = fma((double)st.w[2][oz], d.x, ty);
-                ry = fma((double)st.w[2][oz], d.y, ry);
+                const double w = (double)(wxy * st.w[2][oz]);
+                dT = fma(w, d.x, dT);
+                ratio = fma(w, d.y, ratio);
             }
-            tx = fma((double)st.w[1][oy], ty, tx);
-            rx = fma((double)st.w[1][oy], ry, rx);
         }
-        dT = fma((double)st.w[0][ox], tx, dT);
-        ratio = fma((double)st.w[0][ox], rx, ratio);
-    }
 }
 
 // a[k] for a run-time k in {0, 1, 2} without dynamic register indexing (which would move `a` to local
