@@ -721,7 +721,7 @@ __global__ void k_grid_update(Params P, GridPtrs g) {
 // Scalar G2P (thermal_water.py:206-229), local gas source (:238-245), gas stress (gas.py:16-35),
 // water stress (thermal_water.py:248-253) and momentum P2G (transfer.py:47-70) for one particle
 // per thread, then the momentum scatter by warp runs (bk_scatter.cuh). Bound by the LSU data pipe
-// (69% of its peak at 1M particles: the run loop's broadcasts and the node gather) and by the loads'
+// (70% of its peak at 1M particles: the run loop's broadcasts and the node gather) and by the loads'
 // latency behind it. Loads are plain: staging the block's planes by bulk copies (33 KB and two
 // barriers a block) took 87.0 us where this form, with its L2 prefetch and no barrier, takes 82.
 // Blocks of 128 against 256: 81.8 and 84.2 us at 1M particles (a finished block's slot is refilled
